@@ -1,0 +1,228 @@
+// FP64 work on the integer pipes.  GB300 starts one FP64 instruction of a
+// warp every 16 cycles per SM (measured: DFMA, conversions and compares
+// alike), an integer one every half cycle, so whatever a plain-form kernel
+// can evaluate exactly, or to more than 53 bits, in 64-bit integers is
+// cheaper there, and runs beside the FP64 pipe.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <math.h>
+#include <stdint.h>
+
+namespace phk {
+
+typedef unsigned long long u64;
+
+// The significand of a normal double, left-aligned in 64 bits: with its
+// biased exponent e, |v| = mant64 * 2^(e - 1086).
+__device__ __forceinline__ u64 mant64(int hi, int lo) {
+    const unsigned h = __funnelshift_l((unsigned)lo, (unsigned)hi, 11) | 0x80000000u;
+    return ((u64)h << 32) | ((unsigned)lo << 11);
+}
+__device__ __forceinline__ int biased_exp(int hi) { return (hi >> 20) & 0x7ff; }
+
+// v >> r for any r >= 0 (0 from 64 on; the PTX shift clamps its amount)
+__device__ __forceinline__ u64 shr_clamp(u64 v, int r) {
+    u64 o;
+    asm("shr.u64 %0, %1, %2;" : "=l"(o) : "l"(v), "r"(r));
+    return o;
+}
+
+// -------------------------------------------------------------------
+// FixHist64: per-slice sums of FP64 coordinates as 64-bit fixed-point
+// integers, the FP64 counterpart of FixHist (phk_track.cuh).
+//
+// Every thread-block cluster agrees on one unit per coordinate: of the
+// largest finite |u| of every warp's first values, the smallest (a single
+// stray value cannot coarsen the unit) maps to [2^56, 2^57).  A value
+// becomes the integer v = u / unit truncated toward zero (exact for |u|
+// down to 2^-3 of that typical value, off by at most 2^-56 of it otherwise:
+// below the rounding of the FP64 additions it replaces) and is split into
+// three unsigned 16-bit digits and the signed rest, added to 32-bit
+// shared-memory counters; 2^16 values per counter stay in range (a CTA
+// carries its counters into the cluster's column at least that often).
+// NaN, +-inf and |v| >= 2^62 (32 times the typical value) mark the slice
+// instead; the cluster then sums that slice's values again in FP64 at the
+// end of the pass, so any input gets the sum a floating-point loop would
+// give it.  Unmarked slices are integer sums, converted once: they are the
+// same bits on every launch.
+//
+// What it replaces: warp-private FP64 histograms, whose lanes were
+// serialised by bids in shared memory, two FP64 additions for each round
+// whatever the number of lanes left (19 cycles of the FP64 pipe each, 2 to
+// 5 rounds at 500 to 50 slices).
+// -------------------------------------------------------------------
+constexpr int kFix64Words = 9;   // per slice: count, 4 digits of x, 4 of y
+
+struct FixHist64 {
+    int* w;               // [S][kFix64Words]
+    unsigned* flag;       // [(S + 3) / 4]: one byte per slice, bit q: marked
+    int* any;             // a slice of this CTA is marked
+    int k[2];             // v = mant64 >> (k[q] - e)
+
+    __device__ __forceinline__ void add_q(int q, int s, double u) const {
+        const int hi = __double2hiint(u), lo = __double2loint(u);
+        const int r = k[q] - biased_exp(hi);
+        if (r < 2) {
+            atomicOr(flag + (s >> 2), 1u << (8 * (s & 3) + q));
+            *any = 1;
+            return;
+        }
+        u64 v = shr_clamp(mant64(hi, lo), r);
+        if (hi < 0) v = 0ull - v;
+        const unsigned vl = (unsigned)v;
+        const int vh = (int)(v >> 32);
+        int* d = w + s * kFix64Words + 1 + 4 * q;
+        atomicAdd(d, (int)(vl & 0xffffu));
+        atomicAdd(d + 1, (int)(vl >> 16));
+        atomicAdd(d + 2, vh & 0xffff);
+        atomicAdd(d + 3, vh >> 16);
+    }
+    __device__ __forceinline__ void add(int s, double x, double y) const {
+        atomicAdd(w + s * kFix64Words, 1);
+        add_q(0, s, x);
+        add_q(1, s, y);
+    }
+    __device__ __forceinline__ bool marked(int s, int q) const {
+        return (flag[s >> 2] >> (8 * (s & 3) + q)) & 1u;
+    }
+};
+
+// k of a coordinate from its typical magnitude (the high word of the
+// double, sign cleared; ~0 when every first value is zero: values below 4
+// are then in range).  Clamped so that add_q marks NaN and infinity
+// (exponent 2047) and shifts zeros and subnormals (exponent 0) out.
+__device__ __forceinline__ int fix64_k(unsigned mhi) {
+    int e = mhi != ~0u ? (int)(mhi >> 20) : 1019;
+    e = e < 100 ? 100 : (e > 2000 ? 2000 : e);
+    return e + 7;
+}
+
+// the FP64 value of a slice's integer sum: L1 = sum of d0 + d1 2^16,
+// d2 and d3 the sums of the third and fourth digits (d3 with the carries)
+__device__ __forceinline__ double fix64_value(long long L1, long long d2,
+                                              long long d3, int k) {
+    const double v = fma((double)(d3 * 65536 + d2), 4294967296.0, (double)L1);
+    // unit 2^(k - 1086) (see FixHist64::k)
+    return scalbn(v, k - 1086);
+}
+
+// -------------------------------------------------------------------
+// Sine and cosine of 2 pi F 2^-64, F an unsigned 64-bit fraction of a turn
+// (the integer turns drop out by themselves), in units of 2^-62.
+//
+// The quarter wave is tabulated at 1025 points (shared memory, 8 KB); the
+// remainder theta < 2 pi / 4096 enters through angle addition,
+//   S cos(theta) + C sin(theta) = S + C sin(theta) - S (1 - cos(theta)),
+// with the Maclaurin series sin(theta) = theta - theta^3/6 + theta^5/120 and
+// 1 - cos(theta) = theta^2/2 - theta^4/24 (next terms 4e-24 and 2e-20).
+// Fixed point throughout: the absolute error is below 2^-61 (4e-19), the
+// table's rounding and one truncation per product; a double near 1 resolves
+// 1.1e-16.  About 65 integer instructions, no FP64 one, against 21 FP64
+// multiply-adds (336 cycles of the FP64 pipe) for the library's sin.
+// -------------------------------------------------------------------
+constexpr int kSineEntries = 1025;
+__device__ static const u64 kSineQuarter[kSineEntries] = {
+#include "phk_sine_table.inc"
+};
+
+// copies the table to shared memory (all threads; a barrier must follow)
+__device__ __forceinline__ void stage_sine(u64* tab, int tid, int nthreads) {
+    for (int i = tid; i < kSineEntries; i += nthreads) tab[i] = kSineQuarter[i];
+}
+
+struct SineParts {
+    u64 s, c;       // table values of the quarter wave at j and 1024 - j
+    u64 th;         // sin(theta), units of 2^-73
+    u64 q;          // 1 - cos(theta), units of 2^-82
+};
+
+// u: a quarter turn or less, units of 2^-64 turn
+__device__ __forceinline__ SineParts sine_parts(const u64* tab, u64 u) {
+    SineParts p;
+    const int j = (int)(u >> 52);
+    p.s = tab[j];
+    p.c = tab[(kSineEntries - 1) - j];
+    // theta = 2 pi (u mod 2^52) 2^-64 in units of 2^-73: 2 pi 2^61 = 0xc90f...
+    const u64 th = __umul64hi(u << 12, 0xc90fdaa22168c235ull);
+    const u64 t2 = __umul64hi(th, th);                  // theta^2, 2^-82
+    const unsigned t2h = (unsigned)(t2 >> 32);          // 2^-50
+    const unsigned t4 = __umulhi(t2h, t2h);             // theta^4, 2^-68
+    // theta^2/6 - theta^4/120 in units of 2^-52 (4/6 = 0xaaaaaaab 2^-32,
+    // 2^-16/120 = 546 2^-32)
+    const unsigned e = __umulhi(t2h, 0xaaaaaaabu) - (((t4 >> 16) * 546u) >> 16);
+    const u64 x3 = (u64)(unsigned)(th >> 32) * e;       // 2^-93
+    p.th = th - (x3 >> 20);
+    // theta^4/24: 2^14/24 = 44739243 2^-16
+    p.q = (t2 >> 1) - (((u64)t4 * 44739243u) >> 16);
+    return p;
+}
+
+// sine, units of 2^-62
+__device__ __forceinline__ long long sine_turn(const u64* tab, u64 F) {
+    // the second and third quarters mirror about a quarter turn
+    const unsigned fh = (unsigned)(F >> 32);
+    if ((fh ^ (fh << 1)) & 0x80000000u) F = 0x8000000000000000ull - F;
+    const bool neg = (long long)F < 0;
+    const SineParts p = sine_parts(tab, neg ? 0ull - F : F);
+    const long long d = (long long)(__umul64hi(p.c, p.th) -
+                                    (__umul64hi(p.s, p.q) >> 9));   // 2^-71
+    const long long r = (long long)p.s + ((d + 256) >> 9);
+    return neg ? -r : r;
+}
+
+// t turns (|t| < 2^31) as a fraction of a turn, truncated toward zero
+__device__ __forceinline__ u64 turn_fraction(double t) {
+    const int hi = __double2hiint(t), lo = __double2loint(t);
+    const int r = 1022 - biased_exp(hi);
+    const u64 m = mant64(hi, lo);
+    u64 F = r >= 0 ? shr_clamp(m, r) : m << -r;
+    if (hi < 0) F = 0ull - F;
+    return F;
+}
+
+// A constant of the phase for turn_product: K = mant 2^-exp
+struct TurnFactor {
+    u64 mant;
+    int32_t exp;
+    int32_t reserved;
+};
+
+// num / den as 64 significant bits: the quotient and, from its exact
+// remainder, what its rounding dropped (1 part in 2^64 against 2^53)
+__host__ __device__ inline bool turn_factor(double num, double den, TurnFactor* k) {
+    const double q = num / den;
+    const double lo = fma(-q, den, num) / den;
+    if (!(q > 1e-200 && q < 1e200)) return false;
+    int e = 0;
+    const double m = frexp(q, &e);            // q = m 2^e, m in [1/2, 1)
+    k->mant = ((u64)(m * 9007199254740992.0) << 11) +
+              (u64)(long long)rint(ldexp(lo, 64 - e));
+    k->exp = 64 - e;
+    k->reserved = 0;
+    return true;
+}
+
+// an angle in radians as a fraction of a turn (1 / 2 pi in two doubles)
+__host__ __device__ inline u64 angle_fraction(double rad) {
+    const double inv = 0.15915494309189535, inv_lo = -9.839338337591243e-18;
+    const double h = rad * inv;
+    const double l = fma(rad, inv_lo, fma(rad, inv, -h));
+    const double t = h - rint(h);             // exact, |t| <= 1/2
+    return ((u64)(long long)rint(t * 9223372036854775807.0) << 1) +
+           (u64)(long long)rint(l * 18446744073709551616.0);
+}
+
+// z K turns as a fraction of a turn, for a constant K = kmant 2^-kexp
+// (kmant left-aligned) and |z K| < 2^31: the product of the significands
+// keeps 62 bits and more, rounding nothing to 53
+__device__ __forceinline__ u64 turn_product(double z, u64 kmant, int kexp) {
+    const int hi = __double2hiint(z), lo = __double2loint(z);
+    const u64 m = __umul64hi(mant64(hi, lo), kmant);
+    const int r = 958 + kexp - biased_exp(hi);
+    u64 F = r >= 0 ? shr_clamp(m, r) : m << -r;
+    if (hi < 0) F = 0ull - F;
+    return F;
+}
+
+}  // namespace phk

@@ -3,18 +3,20 @@
 // phk_track_f32.cu / phk_track_f64.cu), the fixed-order merge of the
 // per-CTA partials, the wake convolution, the per-slice moment kernel and
 // the batched merge / wake kernels.
-#include "phk_track.cuh"
+#include "phk_track64.cuh"
 
 namespace phk {
 
 size_t track_smem_bytes(int32_t dtype, int32_t Sa, int32_t Sp) {
-    int nh, ks, st;
     // a turn's pending kicks: four dipolar kicks (resonator and resistive
-    // wall, both planes).  Launches stage one summed table per plane; the
-    // FP64 size is taken for all four tables, an upper bound (the launched
+    // wall, both planes), staged as one summed table per plane (the launched
     // grid is the caller's column count either way)
-    return dtype == PHK_F64 ? smem_for<double>(Sa, Sp, 4, false, &nh, &ks, &st)
-                            : smem_for<float>(Sa, Sp, 2, true, &nh, &ks, &st);
+    if (dtype == PHK_F64) {
+        const size_t tables = (size_t)2 * Sp * sizeof(double) <= 48 * 1024 ? 2 : 0;
+        return track64_smem(Sa, Sp, (int)tables, true, true).bytes;
+    }
+    int ks, st;
+    return smem_for(Sa, Sp, 2, true, &ks, &st);
 }
 
 // Compile-time shape of a program (see TrackShape), from its op kinds.

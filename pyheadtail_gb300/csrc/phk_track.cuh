@@ -1,5 +1,5 @@
-// The fused track kernel and the batched track kernel as templates, with
-// their launch helpers.  Included by the per-precision translation units
+// The FP32 fused track kernel, the batched track kernel and the element
+// arithmetic of both forms as templates, with their launch helpers.  Included by the per-precision translation units
 // (phk_track_f32.cu, phk_track_f64.cu), which instantiate and launch them,
 // and by phk_kernels.cu for the host-side planning helpers.
 #pragma once
@@ -14,6 +14,7 @@
 #include <type_traits>
 
 #include "phk_device.cuh"
+#include "phk_fixed.cuh"
 #include "phk_internal.h"
 
 namespace phk {
@@ -211,13 +212,14 @@ __device__ __forceinline__ void op_rfkick(const phk_op& op,
 // form.  The kick's per-particle sine makes the step inexact whatever the
 // evaluation order, so around it the arithmetic is regrouped to save FP64
 // operations (GB300 runs FP64 at a small fraction of the FP32 rate): the
-// drift is one multiply-add with eta0 * L, the phase one multiply-add with
-// h 2 pi / C, and the momentum update
+// drift is one multiply-add with eta0 * L, the phase and its sine are
+// fixed-point (turn_product, sine_turn), and the momentum update
 //   dp' = (dp p0_old + A sin(phi) - dp_inc) / p0_new
 // is dp (p0_old / p0_new) + (A / p0_new) sin(phi) - dp_inc / p0_new with
-// the ratios formed once per thread (the ratio is exactly 1 without
-// acceleration).  The separately rounded forms above remain for other
-// element sequences.
+// the ratios formed once (the ratio is exactly 1 without acceleration).
+// Five FP64 instructions a particle instead of 27 (a turn at 1e7
+// macroparticles and 500 slices, with FixHist64: 1.317 -> 0.873 ms).  The
+// separately rounded forms above remain for other element sequences.
 template <int VEC>
 __device__ __forceinline__ void op_drift_rf(const phk_op& op,
                                             Tile<double, VEC>& t) {
@@ -231,29 +233,64 @@ __device__ __forceinline__ void op_drift_rf(const phk_op& op,
     }
 }
 
-template <int VEC>
-__device__ __forceinline__ void op_rfkick_rf(const phk_op& op,
-                                             Tile<double, VEC>& t) {
+// The constants of op_rfkick_rf, made once per launch (batched form: once
+// per bunch and CTA).
+struct RfFix {
+    TurnFactor k;     // h / C, turns per metre
+    u64 off;          // phase offset and lock, fraction of a turn
+    double hk, offr;  // the same in radians, for far particles
+    double Ar;        // A / p0_new
+    double ratio;     // p0_old / p0_new
+    double pinc;      // dp_inc / p0_new
+};
+
+__host__ __device__ inline void rf_fix(const phk_op& op, RfFix* r) {
     const double* p = op.p;
     const int f = op.flags;
-    const double hk = p[0] * p[1] * p[11];   // h 2 pi / C
     double off = 0.0;
-    if (f & PHK_FLAG_PHI_OFFSET) off = add(off, p[3]);
-    if (f & PHK_FLAG_PHI_LOCK) off = add(off, p[4]);
-    const double Ar = p[5] * p[12];          // A / p0_new
-    const double ratio = p[6] == p[8] ? 1.0 : p[6] * p[12];
-    const double pinc = (f & PHK_FLAG_P_INC) ? p[7] * p[12] : 0.0;
-    const double Dx = p[9], Dy = p[10];
+    if (f & PHK_FLAG_PHI_OFFSET) off += p[3];
+    if (f & PHK_FLAG_PHI_LOCK) off += p[4];
+    // no usable factor: every particle takes the library's sine
+    if (!turn_factor(p[0], p[2], &r->k)) r->k.exp = -(1 << 20);
+    r->off = angle_fraction(off);
+    r->hk = p[0] * p[1] * p[11];
+    r->offr = off;
+    r->Ar = p[5] * p[12];
+    r->ratio = p[6] == p[8] ? 1.0 : p[6] * p[12];
+    r->pinc = (f & PHK_FLAG_P_INC) ? p[7] * p[12] : 0.0;
+}
+
+// phase of 2^10 turns and more, NaN and infinities (and factors without a
+// fixed-point form)
+static __device__ __noinline__ double rf_sine_far(double z, double hk, double off) {
+    return sin(fma(hk, z, off));
+}
+
+template <int VEC>
+__device__ __forceinline__ void op_rfkick_rf(const phk_op& op, const RfFix& rf,
+                                             const u64* sine,
+                                             Tile<double, VEC>& t) {
+    const bool disp = op.flags & PHK_FLAG_DISPERSION;
+    const double Dx = op.p[9], Dy = op.p[10];
+    const bool constant = rf.ratio == 1.0 && rf.pinc == 0.0;
+    const double A62 = rf.Ar * 0x1p-62;
 #pragma unroll
     for (int j = 0; j < VEC; ++j) {
         double& dp = t.c[PHK_DP][j];
-        if (f & PHK_FLAG_DISPERSION) {
+        if (disp) {
             t.c[PHK_X][j] = sub(t.c[PHK_X][j], mul(Dx, dp));
             t.c[PHK_Y][j] = sub(t.c[PHK_Y][j], mul(Dy, dp));
         }
-        const double s = sin(fma(hk, t.c[PHK_Z][j], off));
-        dp = fma(dp, ratio, fma(Ar, s, -pinc));
-        if (f & PHK_FLAG_DISPERSION) {
+        const double z = t.c[PHK_Z][j];
+        double s;      // sine, times 2^62
+        if (biased_exp(__double2hiint(z)) <= 968 + rf.k.exp) {
+            const u64 F = turn_product(z, rf.k.mant, rf.k.exp) + rf.off;
+            s = (double)sine_turn(sine, F);
+        } else {
+            s = rf_sine_far(z, rf.hk, rf.offr) * 0x1p62;
+        }
+        dp = constant ? fma(A62, s, dp) : fma(dp, rf.ratio, fma(A62, s, -rf.pinc));
+        if (disp) {
             t.c[PHK_X][j] = add(t.c[PHK_X][j], mul(Dx, dp));
             t.c[PHK_Y][j] = add(t.c[PHK_Y][j], mul(Dy, dp));
         }
@@ -748,8 +785,10 @@ enum TrackShape {
     SHAPE_T_LIN = 4,     // transverse, linear longitudinal map
 };
 
+// sine, rf: the staged quarter wave and the kick's constants (FP64 SHAPE_T_RF)
 template <typename T, int VEC, int SHAPE>
 __device__ __forceinline__ void run_program_shape(const phk_program& prog,
+                                                  const u64* sine, const RfFix* rf,
                                                   Tile<T, VEC>& t) {
     if constexpr (SHAPE == SHAPE_NONE) {
         return;
@@ -759,7 +798,7 @@ __device__ __forceinline__ void run_program_shape(const phk_program& prog,
         op_transverse<VEC, true>(prog.op[0], prog, t);
         if constexpr (std::is_same<T, double>::value) {
             op_drift_rf<VEC>(prog.op[1], t);
-            op_rfkick_rf<VEC>(prog.op[2], t);
+            op_rfkick_rf<VEC>(prog.op[2], *rf, sine, t);
             op_drift_rf<VEC>(prog.op[3], t);
         } else {
             op_drift<VEC>(prog.op[1], t);
@@ -777,18 +816,17 @@ __device__ __forceinline__ void run_program_shape(const phk_program& prog,
 // ===================================================================
 // per-slice accumulation in shared memory
 //
-// FP64 form and the batched kernels: each warp owns a private histogram
-//   (count, sum x, sum y per slice); lanes of a warp holding the same slice
-//   are serialised by bids (warp_accumulate), so a bin is updated in a fixed
-//   lane order and the sums do not depend on scheduling.  FP64: plain
-//   double sums; FP32 (batched kernel): Kahan (1965) compensated float sums,
-//   one (sum, compensation) float2 per bin.  When the per-warp copies do not
-//   fit the shared-memory plan, warps share copies through atomics; the
-//   order of the warps sharing a copy is then not fixed, so those sums can
-//   differ in their last bits between launches (FP64 single bunch: beyond
-//   511 slices with two kick tables, 573 without).
+// Batched kernels: each warp owns a private histogram (count, sum x, sum y
+//   per slice); lanes of a warp holding the same slice are serialised by
+//   bids (warp_accumulate), so a bin is updated in a fixed lane order and
+//   the sums do not depend on scheduling.  FP64: plain double sums; FP32:
+//   Kahan (1965) compensated float sums, one (sum, compensation) float2 per
+//   bin.  When the per-warp copies do not fit the shared-memory plan, warps
+//   share copies through atomics; the order of the warps sharing a copy is
+//   then not fixed, so those sums can differ in their last bits between
+//   launches.
 //
-// FP32 single-bunch kernel: exact fixed-point sums (FixHist below), one
+// Single-bunch kernel: fixed-point sums (FixHist below, FixHist64), one
 //   histogram per CTA updated with 32-bit integer atomics: integer addition
 //   is associative, so the sums are bit-identical whatever the order.
 // ===================================================================
@@ -969,6 +1007,13 @@ __device__ __forceinline__ float fix_scale(unsigned mbits) {
     return ldexpf(1.0f, k);
 }
 
+template <typename T>
+struct FixOf;
+template <>
+struct FixOf<float> { using type = FixHist; };
+template <>
+struct FixOf<double> { using type = FixHist64; };
+
 // the FP64 value of a slice sum from its 64-bit total and flag nibble
 __device__ __forceinline__ double fix_value(long long total, unsigned fl,
                                             float scale) {
@@ -1041,6 +1086,13 @@ struct TrackArgs {
     int32_t n_tables;      // kick tables staged (summed targets or kicks)
     int32_t reserved;
 };
+
+// element sequences whose FP64 form reads the staged quarter wave
+template <typename T, int SHAPE>
+constexpr bool needs_sine() {
+    return std::is_same<T, double>::value && SHAPE == SHAPE_T_RF;
+}
+constexpr size_t kSineBytes = ((size_t)kSineEntries * sizeof(u64) + 15) & ~(size_t)15;
 
 template <typename T>
 __device__ __forceinline__ T tadd(T a, T b);
@@ -1251,14 +1303,16 @@ __device__ __forceinline__ void vote_fast_path(Bins<T>& b, bool active,
 // when a.kicks_smem, their tables into `ktab`: one table per kick, or with
 // a.kick_comb one summed table per target (slot a.comb_slot[target]).
 // Called by all threads of a CTA; a __syncthreads() must follow.
+// edges_staged: the edge table is there already.
 template <typename T>
 __device__ __forceinline__ void stage_pending(const phk_kick_set& pk,
                                               const TrackArgs& a, T* epk,
-                                              T* ktab, int tid, int nthreads) {
+                                              T* ktab, int tid, int nthreads,
+                                              bool edges_staged = false) {
     const int Sp = pk.slicer.n_slices;
     const int nk = pk.n_kicks;
     const T* e = reinterpret_cast<const T*>(pk.slicer.edges);
-    for (int i = tid; i <= Sp; i += nthreads) stage_edge<T>(epk, i, e[i]);
+    if (!edges_staged) for (int i = tid; i <= Sp; i += nthreads) stage_edge<T>(epk, i, e[i]);
     if (a.kick_comb) {
         for (int i = tid; i < Sp; i += nthreads) {
             T v[3] = {T(0), T(0), T(0)};
@@ -1343,7 +1397,9 @@ struct TrackCtx {
     int* tag;
     unsigned epoch;
     bool shared_hist;
-    FixHist fix;          // FP32 single-bunch accumulation
+    typename FixOf<T>::type fix;   // single-bunch accumulation
+    const u64* sine;      // FP64, SHAPE_T_RF: staged quarter wave,
+    const RfFix* rf;      // constants of the RF kick
 };
 
 // One tile of VEC particles per thread, already in registers: pending
@@ -1360,7 +1416,7 @@ __device__ __forceinline__ void run_tile(const phk_program& prog,
     // 1. wake kicks of the previous WakeField.track, in kick order
     if (a.has_pk) apply_pending<T, VEC, FULL>(pk, a, cx.bpk, cx.ktab, t, i0);
     // 2. element program
-    run_program_shape<T, VEC, SHAPE>(prog, t);
+    run_program_shape<T, VEC, SHAPE>(prog, cx.sine, cx.rf, t);
     // 3. slice accumulation
     if (a.has_acc) {
         int sl[VEC];
@@ -1375,7 +1431,7 @@ __device__ __forceinline__ void run_tile(const phk_program& prog,
                            : outside_index((double)t.c[PHK_Z][j],
                                            acc.slicer.tail, acc.slicer.width);
             if constexpr (FIX) {
-                if (s >= 0) cx.fix.add(s, (float)t.c[PHK_X][j], (float)t.c[PHK_Y][j]);
+                if (s >= 0) cx.fix.add(s, t.c[PHK_X][j], t.c[PHK_Y][j]);
             } else {
                 warp_accumulate<T>(s, t.c[PHK_X][j], t.c[PHK_Y][j], cx.hx, cx.hy,
                                    cx.hc, cx.tag, cx.epoch, cx.shared_hist);
@@ -1428,7 +1484,6 @@ constexpr int kF32MinBlocks = 4;
 constexpr size_t kF32SmemBudget = 56 * 1024;
 // shared memory a CTA may use at three CTAs per SM
 constexpr size_t kF32SmemBudget3 = 75 * 1024;
-constexpr size_t kF64SmemBudget = 112 * 1024;
 
 // polls of one mbarrier phase before a kernel gives up (order of a second)
 constexpr unsigned kWaitLimit = 1u << 22;
@@ -1458,18 +1513,14 @@ __device__ __forceinline__ void fix_flush(const FixHist& f, int tid,
     }
 }
 
-// FP32 launches aim at four resident CTAs per SM (<= 64 registers), FP64
-// ones at two (<= 128 registers; the FP64 pipe needs the warps to hide
-// its latency)
+// The precision form's pass (T is float; the plain form's is track64_kernel):
+// four resident CTAs per SM (<= 64 registers)
 template <typename T, int VEC, int SHAPE>
-__global__ void __launch_bounds__(kTrackThreads, sizeof(T) == 4 ? kF32MinBlocks : 2)
+__global__ void __launch_bounds__(kTrackThreads, kF32MinBlocks)
 track_kernel(const __grid_constant__ phk_program prog,
              const __grid_constant__ phk_kick_set pk,
              const __grid_constant__ phk_accum acc, const TrackArgs a) {
-    using W = typename Hist<T>::Word;
-    // FP32: exact fixed-point slice sums (FixHist); FP64: bid-serialised
-    // per-warp histograms
-    constexpr bool FIX = std::is_same<T, float>::value;
+    static_assert(std::is_same<T, float>::value, "the precision form's pass");
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int TILE = kTrackThreads * VEC;
@@ -1477,16 +1528,13 @@ track_kernel(const __grid_constant__ phk_program prog,
     const int Sp = a.has_pk ? pk.slicer.n_slices : 0;
     size_t off[9];
     track_smem_layout<T>(Sa, Sp, a.n_hist, a.n_tables, a.kicks_smem, a.stages,
-                         TILE, off, FIX);
-    W* hsx = reinterpret_cast<W*>(smem + off[0]);
-    W* hsy = reinterpret_cast<W*>(smem + off[1]);
-    int* hcnt = reinterpret_cast<int*>(smem + (FIX ? off[0] : off[2]));
+                         TILE, off, true);
+    int* hcnt = reinterpret_cast<int*>(smem + off[0]);
     int* fdig = reinterpret_cast<int*>(smem + off[1]);
     unsigned* fflag = reinterpret_cast<unsigned*>(smem + off[2]);
     T* eacc = reinterpret_cast<T*>(smem + off[3]);
     T* epk = reinterpret_cast<T*>(smem + off[4]);
     T* ktab = reinterpret_cast<T*>(smem + off[5]);
-    int* htag = reinterpret_cast<int*>(smem + off[6]);
     T* ring = reinterpret_cast<T*>(smem + off[7]);
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + off[8]);
     __shared__ unsigned s_max[2];   // FixHist: largest finite |x|, |y| bits
@@ -1532,16 +1580,9 @@ track_kernel(const __grid_constant__ phk_program prog,
     if (a.has_acc) {
         const T* e = reinterpret_cast<const T*>(acc.slicer.edges);
         for (int i = tid; i <= Sa; i += blockDim.x) stage_edge<T>(eacc, i, e[i]);
-        if constexpr (FIX) {
-            for (int i = tid; i < Sa; i += blockDim.x) hcnt[i] = 0;
-            for (int i = tid; i < 4 * Sa; i += blockDim.x) fdig[i] = 0;
-            for (int i = tid; i < (Sa + 3) / 4; i += blockDim.x) fflag[i] = 0u;
-        } else {
-            for (int i = tid; i < a.n_hist * Sa; i += blockDim.x) {
-                Hist<T>::zero(hsx + i); Hist<T>::zero(hsy + i);
-                hcnt[i] = 0; htag[i] = 0;
-            }
-        }
+        for (int i = tid; i < Sa; i += blockDim.x) hcnt[i] = 0;
+        for (int i = tid; i < 4 * Sa; i += blockDim.x) fdig[i] = 0;
+        for (int i = tid; i < (Sa + 3) / 4; i += blockDim.x) fflag[i] = 0u;
     }
     if (a.has_pk) stage_pending<T>(pk, a, epk, ktab, tid, blockDim.x);
     __syncthreads();
@@ -1554,13 +1595,6 @@ track_kernel(const __grid_constant__ phk_program prog,
     vote_fast_path<T>(cx.bpk, a.has_pk, tid, blockDim.x);
     vote_fast_path<T>(cx.bac, a.has_acc, tid, blockDim.x);
     cx.ktab = ktab;
-    const int h = (a.n_hist > 1) ? (tid >> 5) % a.n_hist : 0;
-    cx.hx = hsx + h * Sa;
-    cx.hy = hsy + h * Sa;
-    cx.hc = hcnt + h * Sa;
-    cx.tag = htag + h * Sa;
-    cx.epoch = 0;
-    cx.shared_hist = a.n_hist < (int)(blockDim.x >> 5);
 
     // partial column of this CTA's cluster
     const bool clustered = a.has_acc && a.cluster > 1;
@@ -1571,82 +1605,80 @@ track_kernel(const __grid_constant__ phk_program prog,
 
     bool bad = false;   // a bounded copy wait of this thread gave up
 
-    if constexpr (FIX) {
-        if (a.has_acc) {
-            // ---- the cluster's scale: largest finite |x|, |y| of the inputs
-            // of every member's first tile (the maps change them by factors
-            // of order one; larger values take level B)
-            unsigned m[2] = {0u, 0u};
-            auto see = [&](float u, int q) {
-                const unsigned b = __float_as_uint(u) & 0x7fffffffu;
-                if (b < 0x7f800000u && b > m[q]) m[q] = b;
-            };
-            if (mine > 0) {
-                bad = !mbar_wait(bars, 0u, a.wait_limit);
-                if (!bad) {
-                    const T* src = ring + tid * VEC;
+    if (a.has_acc) {
+        // ---- the cluster's scale: largest finite |x|, |y| of the inputs
+        // of every member's first tile (the maps change them by factors
+        // of order one; larger values take level B)
+        unsigned m[2] = {0u, 0u};
+        auto see = [&](float u, int q) {
+            const unsigned b = __float_as_uint(u) & 0x7fffffffu;
+            if (b < 0x7f800000u && b > m[q]) m[q] = b;
+        };
+        if (mine > 0) {
+            bad = !mbar_wait(bars, 0u, a.wait_limit);
+            if (!bad) {
+                const T* src = ring + tid * VEC;
 #pragma unroll
-                    for (int j = 0; j < VEC; ++j) {
-                        see(src[(size_t)PHK_X * TILE + j], 0);
-                        see(src[(size_t)PHK_Y * TILE + j], 1);
+                for (int j = 0; j < VEC; ++j) {
+                    see(src[(size_t)PHK_X * TILE + j], 0);
+                    see(src[(size_t)PHK_Y * TILE + j], 1);
+                }
+            }
+        } else {
+            const int64_t i0 = (a.stages > 0 ? full_tiles * TILE
+                                             : (int64_t)blockIdx.x * TILE) +
+                               tid * VEC;
+            if (a.stages == 0 || has_partial) {
+#pragma unroll
+                for (int j = 0; j < VEC; ++j) {
+                    if (i0 + j < a.n) {
+                        see(cx.cp[PHK_X][i0 + j], 0);
+                        see(cx.cp[PHK_Y][i0 + j], 1);
                     }
                 }
-            } else {
-                const int64_t i0 = (a.stages > 0 ? full_tiles * TILE
-                                                 : (int64_t)blockIdx.x * TILE) +
-                                   tid * VEC;
-                if (a.stages == 0 || has_partial) {
-#pragma unroll
-                    for (int j = 0; j < VEC; ++j) {
-                        if (i0 + j < a.n) {
-                            see(cx.cp[PHK_X][i0 + j], 0);
-                            see(cx.cp[PHK_Y][i0 + j], 1);
-                        }
-                    }
-                }
             }
-            m[0] = __reduce_max_sync(0xffffffffu, m[0]);
-            m[1] = __reduce_max_sync(0xffffffffu, m[1]);
-            if ((tid & 31) == 0) {
-                atomicMax(&s_max[0], m[0]);
-                atomicMax(&s_max[1], m[1]);
-            }
-            if (tid == 0) {
-                s_spill.spill[0] = reinterpret_cast<long long*>(P) + (int64_t)Sa * G + column;
-                s_spill.spill[1] = reinterpret_cast<long long*>(P) + (int64_t)2 * Sa * G + column;
-                s_spill.stride = G;
-            }
-            // rank 0 clears its column's level-B sums before any member adds
-            if (crank == 0) {
-                for (int s = tid; s < Sa; s += blockDim.x) {
-                    reinterpret_cast<long long*>(P)[(int64_t)(Sa + s) * G + column] = 0;
-                    reinterpret_cast<long long*>(P)[(int64_t)(2 * Sa + s) * G + column] = 0;
-                }
-            }
-            unsigned M[2];
-            if (clustered) {
-                __threadfence();
-                cg::cluster_group cl = cg::this_cluster();
-                cl.sync();
-                M[0] = M[1] = 0u;
-                for (unsigned r = 0; r < cl.num_blocks(); ++r) {
-                    const unsigned* sm = cl.map_shared_rank(s_max, r);
-                    M[0] = max(M[0], sm[0]);
-                    M[1] = max(M[1], sm[1]);
-                }
-            } else {
-                __syncthreads();
-                M[0] = s_max[0];
-                M[1] = s_max[1];
-            }
-            cx.fix.cnt = hcnt;
-            cx.fix.dig = fdig;
-            cx.fix.flag = fflag;
-            cx.fix.sp = &s_spill;
-            cx.fix.S = Sa;
-            cx.fix.scale[0] = fix_scale(M[0]);
-            cx.fix.scale[1] = fix_scale(M[1]);
         }
+        m[0] = __reduce_max_sync(0xffffffffu, m[0]);
+        m[1] = __reduce_max_sync(0xffffffffu, m[1]);
+        if ((tid & 31) == 0) {
+            atomicMax(&s_max[0], m[0]);
+            atomicMax(&s_max[1], m[1]);
+        }
+        if (tid == 0) {
+            s_spill.spill[0] = reinterpret_cast<long long*>(P) + (int64_t)Sa * G + column;
+            s_spill.spill[1] = reinterpret_cast<long long*>(P) + (int64_t)2 * Sa * G + column;
+            s_spill.stride = G;
+        }
+        // rank 0 clears its column's level-B sums before any member adds
+        if (crank == 0) {
+            for (int s = tid; s < Sa; s += blockDim.x) {
+                reinterpret_cast<long long*>(P)[(int64_t)(Sa + s) * G + column] = 0;
+                reinterpret_cast<long long*>(P)[(int64_t)(2 * Sa + s) * G + column] = 0;
+            }
+        }
+        unsigned M[2];
+        if (clustered) {
+            __threadfence();
+            cg::cluster_group cl = cg::this_cluster();
+            cl.sync();
+            M[0] = M[1] = 0u;
+            for (unsigned r = 0; r < cl.num_blocks(); ++r) {
+                const unsigned* sm = cl.map_shared_rank(s_max, r);
+                M[0] = max(M[0], sm[0]);
+                M[1] = max(M[1], sm[1]);
+            }
+        } else {
+            __syncthreads();
+            M[0] = s_max[0];
+            M[1] = s_max[1];
+        }
+        cx.fix.cnt = hcnt;
+        cx.fix.dig = fdig;
+        cx.fix.flag = fflag;
+        cx.fix.sp = &s_spill;
+        cx.fix.S = Sa;
+        cx.fix.scale[0] = fix_scale(M[0]);
+        cx.fix.scale[1] = fix_scale(M[1]);
     }
 
     if (a.stages > 0) {
@@ -1684,7 +1716,7 @@ track_kernel(const __grid_constant__ phk_program prog,
                     }
                 }
                 const int64_t i0 = (blockIdx.x + k * gridDim.x) * TILE + tid * VEC;
-                run_tile<T, VEC, SHAPE, true, FIX>(prog, pk, acc, a, cx, t, i0, true);
+                run_tile<T, VEC, SHAPE, true, true>(prog, pk, acc, a, cx, t, i0, true);
             }
             __syncwarp();                    // this warp's part of stage st read
             if (lane == 0) {
@@ -1698,12 +1730,10 @@ track_kernel(const __grid_constant__ phk_program prog,
                 st = 0;
                 ph ^= 1u;
             }
-            if constexpr (FIX) {
-                if (a.has_acc && (k + 1) % fix_flush_tiles<TILE>() == 0) {
-                    __syncthreads();
-                    fix_flush(cx.fix, tid, blockDim.x);
-                    __syncthreads();
-                }
+            if (a.has_acc && (k + 1) % fix_flush_tiles<TILE>() == 0) {
+                __syncthreads();
+                fix_flush(cx.fix, tid, blockDim.x);
+                __syncthreads();
             }
         }
         __syncthreads();
@@ -1730,7 +1760,7 @@ track_kernel(const __grid_constant__ phk_program prog,
             const bool full = i0 + VEC <= a.n;
             Tile<T, VEC> t;
             load_tile_plain<T, VEC>(a, cx, t, i0, full);
-            run_tile<T, VEC, SHAPE, false, FIX>(prog, pk, acc, a, cx, t, i0, full);
+            run_tile<T, VEC, SHAPE, false, true>(prog, pk, acc, a, cx, t, i0, full);
         }
     } else {
         // ---- plain loads; every warp runs whole tiles (lanes past the end
@@ -1742,180 +1772,102 @@ track_kernel(const __grid_constant__ phk_program prog,
             const bool full = i0 + VEC <= a.n;
             Tile<T, VEC> t;
             load_tile_plain<T, VEC>(a, cx, t, i0, full);
-            run_tile<T, VEC, SHAPE, false, FIX>(prog, pk, acc, a, cx, t, i0, full);
-            if constexpr (FIX) {
-                if (a.has_acc && (it + 1) % fix_flush_tiles<TILE>() == 0) {
-                    __syncthreads();
-                    fix_flush(cx.fix, tid, blockDim.x);
-                    __syncthreads();
-                }
+            run_tile<T, VEC, SHAPE, false, true>(prog, pk, acc, a, cx, t, i0, full);
+            if (a.has_acc && (it + 1) % fix_flush_tiles<TILE>() == 0) {
+                __syncthreads();
+                fix_flush(cx.fix, tid, blockDim.x);
+                __syncthreads();
             }
         }
     }
 
     if (!a.has_acc) return;
-    if constexpr (FIX) {
-        // ---- rank 0 adds its cluster's counters and level-B sums as 64-bit
-        // integers and writes the partial column in FP64
-        unsigned nb = 1;
-        if (clustered) {
-            __threadfence();                 // level-B adds before the barrier
-            cg::cluster_group cl = cg::this_cluster();
-            cl.sync();
-            nb = cl.num_blocks();
-        } else {
-            __syncthreads();
-        }
-        if (crank == 0) {
-            const long long* lp = reinterpret_cast<const long long*>(P);
-            for (int s = tid; s < Sa; s += blockDim.x) {
-                long long c = 0, tq[2];
-                unsigned fl = 0;
-                tq[0] = __ldcg(lp + (int64_t)(Sa + s) * G + column);
-                tq[1] = __ldcg(lp + (int64_t)(2 * Sa + s) * G + column);
-                // unrolled over the cluster's members, so that the loads of
-                // every member are in flight together
-#pragma unroll
-                for (int r = 0; r < kCluster; ++r) {
-                    if (r >= (int)nb) break;
-                    const int* rc = hcnt;
-                    const int* rd = fdig;
-                    const unsigned* rf = fflag;
-                    if (clustered) {
-                        cg::cluster_group cl = cg::this_cluster();
-                        rc = cl.map_shared_rank(hcnt, r);
-                        rd = cl.map_shared_rank(fdig, r);
-                        rf = cl.map_shared_rank(fflag, r);
-                    }
-                    c += rc[s];
-                    fl |= (rf[s >> 2] >> (8 * (s & 3))) & 0xffu;
-#pragma unroll
-                    for (int q = 0; q < 2; ++q)
-                        tq[q] += FixHist::total(rd + 2 * q * Sa + s, Sa);
-                }
-                P[(int64_t)s * G + column] = (double)c;
-                P[(int64_t)(Sa + s) * G + column] =
-                    fix_value(tq[0], fl & 15u, cx.fix.scale[0]);
-                P[(int64_t)(2 * Sa + s) * G + column] =
-                    fix_value(tq[1], fl >> 4, cx.fix.scale[1]);
-            }
-        }
-        if (clustered) cg::this_cluster().sync();  // members keep their counters until read
-        return;
+    // ---- rank 0 adds its cluster's counters and level-B sums as 64-bit
+    // integers and writes the partial column in FP64
+    unsigned nb = 1;
+    if (clustered) {
+        __threadfence();                 // level-B adds before the barrier
+        cg::cluster_group cl = cg::this_cluster();
+        cl.sync();
+        nb = cl.num_blocks();
     } else {
         __syncthreads();
-        // fold the per-warp copies into copy 0 (fixed order)
+    }
+    if (crank == 0) {
+        const long long* lp = reinterpret_cast<const long long*>(P);
         for (int s = tid; s < Sa; s += blockDim.x) {
-            int c = hcnt[s];
-            for (int k = 1; k < a.n_hist; ++k) {
-                c += hcnt[k * Sa + s];
-                Hist<T>::merge(hsx + s, hsx + k * Sa + s);
-                Hist<T>::merge(hsy + s, hsy + k * Sa + s);
-            }
-            hcnt[s] = c;
-        }
-        if (clustered) {
-            // fold the CTAs of the thread-block cluster into its rank 0
-            // through distributed shared memory
-            cg::cluster_group cl = cg::this_cluster();
-            cl.sync();
-            if (crank == 0) {
-                for (int s = tid; s < Sa; s += blockDim.x) {
-                    int c = hcnt[s];
-                    for (unsigned r = 1; r < cl.num_blocks(); ++r) {
-                        c += *cl.map_shared_rank(hcnt + s, r);
-                        Hist<T>::merge(hsx + s, cl.map_shared_rank(hsx + s, r));
-                        Hist<T>::merge(hsy + s, cl.map_shared_rank(hsy + s, r));
-                    }
-                    hcnt[s] = c;
+            long long c = 0, tq[2];
+            unsigned fl = 0;
+            tq[0] = __ldcg(lp + (int64_t)(Sa + s) * G + column);
+            tq[1] = __ldcg(lp + (int64_t)(2 * Sa + s) * G + column);
+            // unrolled over the cluster's members, so that the loads of
+            // every member are in flight together
+#pragma unroll
+            for (int r = 0; r < kCluster; ++r) {
+                if (r >= (int)nb) break;
+                const int* rc = hcnt;
+                const int* rd = fdig;
+                const unsigned* rf = fflag;
+                if (clustered) {
+                    cg::cluster_group cl = cg::this_cluster();
+                    rc = cl.map_shared_rank(hcnt, r);
+                    rd = cl.map_shared_rank(fdig, r);
+                    rf = cl.map_shared_rank(fflag, r);
                 }
+                c += rc[s];
+                fl |= (rf[s >> 2] >> (8 * (s & 3))) & 0xffu;
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    tq[q] += FixHist::total(rd + 2 * q * Sa + s, Sa);
             }
-            cl.sync();  // members keep their shared memory until read
-            if (crank != 0) return;
-        } else {
-            __syncthreads();
-        }
-        for (int s = tid; s < Sa; s += blockDim.x) {
-            P[(int64_t)s * G + column] = (double)hcnt[s];
-            P[(int64_t)(Sa + s) * G + column] = Hist<T>::value(hsx + s);
-            P[(int64_t)(2 * Sa + s) * G + column] = Hist<T>::value(hsy + s);
+            P[(int64_t)s * G + column] = (double)c;
+            P[(int64_t)(Sa + s) * G + column] =
+                fix_value(tq[0], fl & 15u, cx.fix.scale[0]);
+            P[(int64_t)(2 * Sa + s) * G + column] =
+                fix_value(tq[1], fl >> 4, cx.fix.scale[1]);
         }
     }
+    if (clustered) cg::this_cluster().sync();  // members keep their counters until read
 }
 
 // ===================================================================
 // launch configuration
 // ===================================================================
 
-// Shared-memory plan of a launch: histogram copies (FP64: one private copy
-// per warp when they fit, else fewer copies shared with atomics; FP32: the
-// one FixHist of the CTA) and TMA ring stages (FP32 aligned launches),
+// Shared-memory plan of an FP32 launch: TMA ring stages (aligned launches),
 // chosen so that the occupancy the kernel is compiled for is reached
 // whenever possible.  n_tables: kick tables staged per CTA.
-template <typename T>
-static size_t smem_for(int Sa, int Sp, int n_tables, bool tma, int* n_hist,
-                       int* kicks_smem, int* stages, size_t budget_in = 0,
-                       int forced_stages = -1) {
-    constexpr bool fix = sizeof(T) == 4;
-    const int warps = kTrackThreads / 32;
-    const int tile = kTrackThreads * (sizeof(T) == 8 ? 2 : kF32Vec);
-    const size_t budget = budget_in ? budget_in
-                                    : (sizeof(T) == 8 ? kF64SmemBudget : kF32SmemBudget);
-    *kicks_smem = n_tables > 0 && (size_t)n_tables * Sp * sizeof(T) <= 48 * 1024;
-    const int hist_opts[4] = {warps, 4, 2, 1};
-    const int n_hist_opts = fix ? 1 : 4;
-    // ring stages by default: two (measured fastest at 500 slices; more
-    // stages take a launch plan), else plain loads (large slice counts)
-    const int stage_opts[2] = {2, 0};
-    size_t off[9];
-    if (tma && (forced_stages == 0 || (forced_stages >= 2 && forced_stages <= kMaxStages))) {
-        const int nh = 1;
-        const size_t b = track_smem_layout<T>(Sa, Sp, nh, n_tables, *kicks_smem,
-                                              forced_stages, tile, off, fix);
-        if (fix && b <= budget) {
-            *n_hist = nh;
+static inline size_t smem_for(int Sa, int Sp, int n_tables, bool tma,
+                              int* kicks_smem, int* stages, size_t budget_in = 0,
+                              int forced_stages = -1) {
+    const int tile = kTrackThreads * kF32Vec;
+    *kicks_smem = n_tables > 0 && (size_t)n_tables * Sp * sizeof(float) <= 48 * 1024;
+    auto bytes = [&](int st) {
+        size_t off[9];
+        return track_smem_layout<float>(Sa, Sp, 1, n_tables, *kicks_smem, st, tile,
+                                        off, true);
+    };
+    if (tma) {
+        const size_t budget = budget_in ? budget_in : kF32SmemBudget;
+        const bool forced = forced_stages == 0 ||
+                            (forced_stages >= 2 && forced_stages <= kMaxStages);
+        if (forced && bytes(forced_stages) <= budget) {
             *stages = forced_stages;
-            return b;
+            return bytes(forced_stages);
+        }
+        // by default two ring stages (measured fastest at 500 slices; more
+        // take a launch plan) at four CTAs per SM; where they do not fit
+        // (about 700 slices and more), two stages at three CTAs per SM,
+        // measured faster than plain loads at 1000 slices
+        const size_t most = budget_in == 0 && forced_stages < 0 ? kF32SmemBudget3
+                                                                : budget;
+        if (bytes(2) <= most) {
+            *stages = 2;
+            return bytes(2);
         }
     }
-    if (fix && tma && budget_in == 0 && forced_stages < 0) {
-        // FP32 default: two ring stages at four CTAs per SM; where they do
-        // not fit (about 700 slices and more), two stages at three CTAs
-        // per SM, measured faster than plain loads at 1000 slices
-        const size_t budgets[2] = {kF32SmemBudget, kF32SmemBudget3};
-        for (int bi = 0; bi < 2; ++bi) {
-            const size_t b = track_smem_layout<T>(Sa, Sp, 1, n_tables, *kicks_smem,
-                                                  2, tile, off, fix);
-            if (b <= budgets[bi]) {
-                *n_hist = 1;
-                *stages = 2;
-                return b;
-            }
-        }
-    }
-    size_t smallest = 0;
-    for (int hi = 0; hi < n_hist_opts; ++hi) {
-        for (int si = 0; si < (tma ? 2 : 1); ++si) {
-            const int nh = (Sa > 0 && !fix) ? hist_opts[hi] : 1;
-            const int st = tma ? stage_opts[si] : 0;
-            const size_t b = track_smem_layout<T>(Sa, Sp, nh, n_tables,
-                                                  *kicks_smem, st, tile, off,
-                                                  fix);
-            if (b <= budget) {
-                *n_hist = nh;
-                *stages = st;
-                return b;
-            }
-            if (smallest == 0 || b < smallest) {
-                // nothing fits the occupancy budget yet: keep the smallest
-                // plan (fewer resident CTAs per SM)
-                *n_hist = nh;
-                *stages = st;
-                smallest = b;
-            }
-        }
-    }
-    return smallest;
+    *stages = 0;
+    return bytes(0);
 }
 
 // Kick tables a launch stages: with dipolar kicks only, the kicks of one
@@ -2046,16 +1998,14 @@ static int launch_track_t(const phk_program* prog, const phk_coords* c,
     const int Sa = acc ? acc->slicer.n_slices : 0;
     const int Sp = pk ? pk->slicer.n_slices : 0;
     // the TMA ring needs 16-byte aligned coordinates (VEC > 1 launches)
-    // and pays off for the memory-bound FP32 form
-    const bool tma = VEC > 1 && sizeof(T) == 4;
+    const bool tma = VEC > 1;
     plan_kick_tables<T>(pk, &a);
     int kicks_smem = 0;
+    a.n_hist = 1;
     const TrackPlan pl = track_plan();
-    const bool planned = sizeof(T) == 4;
-    const size_t smem = smem_for<T>(
-        Sa, Sp, a.n_tables, tma, &a.n_hist, &kicks_smem, &a.stages,
-        planned && pl.smem_kb > 0 ? (size_t)pl.smem_kb * 1024 : 0,
-        planned ? pl.stages : -1);
+    const size_t smem = smem_for(Sa, Sp, a.n_tables, tma, &kicks_smem, &a.stages,
+                                 pl.smem_kb > 0 ? (size_t)pl.smem_kb * 1024 : 0,
+                                 pl.stages);
     if (kicks_smem != a.kicks_smem)
         return set_error(PHK_EPARAM, "phk_track: inconsistent kick-table plan");
     if (smem > track_dynamic_smem_limit<T, VEC, SHAPE>())
@@ -2145,6 +2095,12 @@ struct BatchArgs {
 };
 
 constexpr size_t kProgSmem = (sizeof(phk_program) + 15) & ~(size_t)15;
+// the quarter wave of an FP64 batch (reserved whatever the programs, so that
+// the grid follows from the sizes alone)
+template <typename T>
+constexpr size_t batch_head() {
+    return kProgSmem + (sizeof(T) == 8 ? kSineBytes : 0);
+}
 
 // Per CTA: its units in order.  When the bunch changes, the CTA's per-slice
 // sums of the previous bunch go to that bunch's partial column, and the new
@@ -2161,7 +2117,9 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
     const int Sp = a.has_pk ? pk.slicer.n_slices : 0;
     const int nk = a.has_pk ? pk.n_kicks : 0;
     phk_program* sprog = reinterpret_cast<phk_program*>(smem);
-    unsigned char* rest = smem + kProgSmem;
+    u64* sine = reinterpret_cast<u64*>(smem + kProgSmem);
+    __shared__ RfFix s_rf;
+    unsigned char* rest = smem + batch_head<T>();
     size_t off[9];
     track_smem_layout<T>(Sa, Sp, a.n_hist, nk, 1, 0, TILE, off);
     W* hsx = reinterpret_cast<W*>(rest + off[0]);
@@ -2185,8 +2143,11 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
         const T* e = reinterpret_cast<const T*>(pk.slicer.edges);
         for (int i = tid; i <= Sp; i += THREADS) stage_edge<T>(epk, i, e[i]);
     }
+    if (needs_sine<T, SHAPE>()) stage_sine(sine, tid, THREADS);
 
     TrackCtx<T, VEC> cx;
+    cx.sine = sine;
+    cx.rf = &s_rf;
 #pragma unroll
     for (int q = 0; q < 6; ++q) cx.cp[q] = reinterpret_cast<T*>(a.c[q]);
     cx.ktab = ktab;
@@ -2248,6 +2209,8 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
             int4* dst = reinterpret_cast<int4*>(sprog);
             for (int i = tid; i < (int)(sizeof(phk_program) / 16); i += THREADS)
                 dst[i] = src[i];
+            if (needs_sine<T, SHAPE>() && tid == 0)
+                rf_fix(b.programs[U.bunch].op[2], &s_rf);
             if (a.has_pk) {
                 const T* kt = reinterpret_cast<const T*>(b.kicks) +
                               (int64_t)U.bunch * nk * Sp;
@@ -2298,7 +2261,7 @@ static size_t batch_smem(int Sa, int Sp, int nk, int threads, int* n_hist) {
         bytes = track_smem_layout<T>(Sa, Sp, nh, nk, 1, 0, tile, off);
     }
     *n_hist = nh;
-    return kProgSmem + bytes;
+    return batch_head<T>() + bytes;
 }
 
 template <typename T, int VEC, int THREADS, int SHAPE>

@@ -1,5 +1,5 @@
 // Instantiations and launches of the track kernels for double coordinates.
-#include "phk_track.cuh"
+#include "phk_track64.cuh"
 
 namespace phk {
 
@@ -7,23 +7,23 @@ int launch_track_f64(const phk_program* prog, const phk_coords* c,
                      const phk_kick_set* pk, const phk_accum* acc, int ld,
                      int stm, bool vec_ok, cudaStream_t st) {
     if (!vec_ok)
-        return launch_track_t<double, 1, SHAPE_GENERIC>(prog, c, pk, acc, ld, stm, st);
+        return launch_track64_t<1, SHAPE_GENERIC>(prog, c, pk, acc, ld, stm, st);
     switch (program_shape(prog)) {
         case SHAPE_NONE:
-            return launch_track_t<double, 2, SHAPE_NONE>(prog, c, pk, acc, ld, stm, st);
+            return launch_track64_t<2, SHAPE_NONE>(prog, c, pk, acc, ld, stm, st);
         case SHAPE_T:
-            return launch_track_t<double, 2, SHAPE_T>(prog, c, pk, acc, ld, stm, st);
+            return launch_track64_t<2, SHAPE_T>(prog, c, pk, acc, ld, stm, st);
         case SHAPE_T_RF:
-            return launch_track_t<double, 2, SHAPE_T_RF>(prog, c, pk, acc, ld, stm, st);
+            return launch_track64_t<2, SHAPE_T_RF>(prog, c, pk, acc, ld, stm, st);
         case SHAPE_T_LIN:
-            return launch_track_t<double, 2, SHAPE_T_LIN>(prog, c, pk, acc, ld, stm, st);
+            return launch_track64_t<2, SHAPE_T_LIN>(prog, c, pk, acc, ld, stm, st);
         default:
-            return launch_track_t<double, 2, SHAPE_GENERIC>(prog, c, pk, acc, ld, stm, st);
+            return launch_track64_t<2, SHAPE_GENERIC>(prog, c, pk, acc, ld, stm, st);
     }
 }
 
 int track_clusters_f64(size_t smem) {
-    return occupancy_clusters<double, 2, SHAPE_GENERIC>(smem);
+    return track64_clusters<2, SHAPE_GENERIC>(smem);
 }
 
 // common program shape of every bunch of a batch (GENERIC unless all equal
