@@ -97,38 +97,6 @@ __device__ __forceinline__ double div_by(double a, double b, double y) {
     return dvd(a, b);
 }
 
-// sin and cos of phi = phi0 + d for a base phi0 whose sine s0 and cosine c0
-// are known (host, correctly rounded): angle addition with the Maclaurin
-// series of sin d (to d^11) and cos d (to d^12), whose truncation errors
-// are below 3e-18 and 5e-20 for |d| <= 1/4.  d = phi - phi0 is exact when
-// phi and phi0 are within a factor two (Sterbenz).  Larger |d| falls back
-// to the library sincos.
-__device__ __forceinline__ void sincos_about(double phi, double phi0,
-                                             double s0, double c0, double* s,
-                                             double* c) {
-    const double d = phi - phi0;
-    if (!(fabs(d) <= 0.25)) {
-        sincos(phi, s, c);
-        return;
-    }
-    const double d2 = d * d;
-    // sin d = d + d^3 (-1/3! + d^2 (1/5! + d^2 (-1/7! + d^2 (1/9! - d^2/11!))))
-    double ps = fma(d2, -1.0 / 39916800.0, 1.0 / 362880.0);
-    ps = fma(d2, ps, -1.0 / 5040.0);
-    ps = fma(d2, ps, 1.0 / 120.0);
-    ps = fma(d2, ps, -1.0 / 6.0);
-    const double sd = fma(d * d2, ps, d);
-    // cos d = 1 + d^2 (-1/2! + d^2 (1/4! + ... + d^2 / 12!))
-    double pc = fma(d2, 1.0 / 479001600.0, -1.0 / 3628800.0);
-    pc = fma(d2, pc, 1.0 / 40320.0);
-    pc = fma(d2, pc, -1.0 / 720.0);
-    pc = fma(d2, pc, 1.0 / 24.0);
-    pc = fma(d2, pc, -0.5);
-    const double cd = fma(d2, pc, 1.0);
-    *s = fma(s0, cd, c0 * sd);
-    *c = fma(c0, cd, -(s0 * sd));
-}
-
 // ---------------------------------------------------------------- binning
 // Exact reference slice index from the host-built lower-edge table
 // e[0..S]: inside iff e[0] <= z < e[S], index k with e[k] <= z < e[k+1].

@@ -1,8 +1,8 @@
-// FP64 work on the integer pipes.  GB300 starts one FP64 instruction of a
-// warp every 16 cycles per SM (measured: DFMA, conversions and compares
-// alike), an integer one every half cycle, so whatever a plain-form kernel
-// can evaluate exactly, or to more than 53 bits, in 64-bit integers is
-// cheaper there, and runs beside the FP64 pipe.
+// FP64 work on the integer pipes.  GB300 starts one FP64 addition,
+// multiplication or multiply-add of a warp every 19 cycles per SM and a
+// conversion every 16 (measured), an integer instruction every half cycle, so
+// whatever a plain-form kernel can evaluate exactly, or to more than 53 bits,
+// in 64-bit integers is cheaper there, and runs beside the FP64 pipe.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -118,8 +118,9 @@ __device__ __forceinline__ double fix64_value(long long L1, long long d2,
 // 1 - cos(theta) = theta^2/2 - theta^4/24 (next terms 4e-24 and 2e-20).
 // Fixed point throughout: the absolute error is below 2^-61 (4e-19), the
 // table's rounding and one truncation per product; a double near 1 resolves
-// 1.1e-16.  About 65 integer instructions, no FP64 one, against 21 FP64
-// multiply-adds (336 cycles of the FP64 pipe) for the library's sin.
+// 1.1e-16.  Measured per warp: 42 cycles for the sine, 54 for sine and cosine
+// with their conversions; the library's sin takes 21 FP64 multiply-adds
+// (about 400 cycles).
 // -------------------------------------------------------------------
 constexpr int kSineEntries = 1025;
 __device__ static const u64 kSineQuarter[kSineEntries] = {
@@ -169,6 +170,31 @@ __device__ __forceinline__ long long sine_turn(const u64* tab, u64 F) {
                                     (__umul64hi(p.s, p.q) >> 9));   // 2^-71
     const long long r = (long long)p.s + ((d + 256) >> 9);
     return neg ? -r : r;
+}
+
+// sine and cosine, times 2^62, as doubles
+__device__ __forceinline__ void sincos_turn(const u64* tab, u64 F, double* s,
+                                            double* c) {
+    const SineParts p = sine_parts(tab, F & 0x3fffffffffffffffull);
+    const long long d1 = (long long)(__umul64hi(p.c, p.th) -
+                                     (__umul64hi(p.s, p.q) >> 9));   // 2^-71
+    const long long d2 = (long long)(__umul64hi(p.s, p.th) +
+                                     (__umul64hi(p.c, p.q) >> 9));
+    const double sn = (double)((long long)p.s + ((d1 + 256) >> 9));
+    const double cs = (double)((long long)p.c - ((d2 + 256) >> 9));
+    // quadrants: (sn, cs), (cs, -sn), (-sn, -cs), (-cs, sn)
+    const unsigned k = (unsigned)(F >> 62);
+    const double a = (k & 1u) ? cs : sn, b = (k & 1u) ? sn : cs;
+    const int na = (int)((k & 2u) << 30), nb = (int)(((k + 1u) & 2u) << 30);
+    *s = __hiloint2double(__double2hiint(a) ^ na, __double2loint(a));
+    *c = __hiloint2double(__double2hiint(b) ^ nb, __double2loint(b));
+}
+
+// v 2^-62 for |v| >= 1 or v = 0 (integer work only)
+__device__ __forceinline__ double unscale62(double v) {
+    const int hi = __double2hiint(v);
+    return __hiloint2double((hi & 0x7fffffff) ? hi - (62 << 20) : hi,
+                            __double2loint(v));
 }
 
 // t turns (|t| < 2^31) as a fraction of a turn, truncated toward zero

@@ -34,6 +34,105 @@ struct Tile {
 // element arithmetic, plain FP64 form (reference evaluation order)
 // ===================================================================
 
+// An FP64 instruction takes its 16 cycles of the pipe even when a short
+// branch around it is compiled to predication and it is predicated off (16
+// of the 34 FP64 instructions a particle of the undetuned turn with RF were
+// such dispersion terms).  The element functions of the plain form are
+// therefore compiled twice: PLAIN for the common single-segment turn
+// (program_plain64: no dispersion, constant energy, equal optics functions
+// with alpha = 0 at both ends of a detuned segment), without any
+// alternative, and in full for the op loop.
+
+// Constants of an op's FP64 form that its parameter block holds in another
+// shape: made once per launch (batched form: once per bunch and CTA).
+struct OpFix {
+    TurnFactor k;    // RF kick: h / C, turns per metre
+    u64 off;         // RF kick: phase offset and lock, fraction of a turn
+    double c[5];     // RF kick: (A / p0_new) 2^-62, p0_old / p0_new,
+                     //   dp_inc / p0_new, h 2 pi / C, offset in radians
+                     // drift: eta0 L
+                     // detuned transverse: J01 J10 J23 J32, times 2^-62
+};
+// amplitude detuning: with j = g u^2 + t u u' + u'^2
+struct DetFix {
+    double gx, tx, gy, ty;
+    double axx, axy, ayy, ayx;   // dQ_x = axx j_x + axy j_y, dQ_y likewise
+};
+struct Aux64 {
+    const u64* sine;     // staged quarter wave (stage_sine)
+    const OpFix* op;     // by op
+    const DetFix* det;   // by detuner
+};
+
+__host__ __device__ inline void op_fix(const phk_op& op, OpFix* r) {
+    const double* p = op.p;
+    const int f = op.flags;
+    if (op.kind == PHK_OP_DRIFT) {
+        r->c[0] = p[1] * p[2];
+    } else if (op.kind == PHK_OP_TRANSVERSE) {
+        r->c[0] = p[9] * 0x1p-62;
+        r->c[1] = p[10] * 0x1p-62;
+        r->c[2] = p[13] * 0x1p-62;
+        r->c[3] = p[14] * 0x1p-62;
+    } else if (op.kind == PHK_OP_RF_KICK) {
+        double off = 0.0;
+        if (f & PHK_FLAG_PHI_OFFSET) off += p[3];
+        if (f & PHK_FLAG_PHI_LOCK) off += p[4];
+        // no usable factor: every particle takes the library's sine
+        if (!turn_factor(p[0], p[2], &r->k)) r->k.exp = -(1 << 20);
+        r->off = angle_fraction(off);
+        r->c[0] = p[5] * p[12] * 0x1p-62;
+        r->c[1] = p[6] == p[8] ? 1.0 : p[6] * p[12];
+        r->c[2] = (f & PHK_FLAG_P_INC) ? p[7] * p[12] : 0.0;
+        r->c[3] = p[0] * p[1] * p[11];
+        r->c[4] = off;
+    }
+}
+
+__host__ __device__ inline void det_fix(const phk_detuner& d, DetFix* f) {
+    const double* c = d.c;
+    f->gx = c[4] / c[6];
+    f->tx = c[5] / c[6];
+    f->gy = c[7] / c[9];
+    f->ty = c[8] / c[9];
+    f->axx = 0.5 * c[0] * c[6] / c[10];
+    f->axy = 0.5 * c[2] * c[9] / c[10];
+    f->ayy = 0.5 * c[1] * c[9] / c[10];
+    f->ayx = 0.5 * c[3] * c[6] / c[10];
+}
+
+// whether a program needs the quarter wave
+static inline bool program_has_phase(const phk_program& prog) {
+    for (int o = 0; o < prog.n_ops; ++o)
+        if (prog.op[o].kind == PHK_OP_RF_KICK ||
+            (prog.op[o].kind == PHK_OP_TRANSVERSE &&
+             (prog.op[o].flags & PHK_FLAG_DETUNED)))
+            return true;
+    return false;
+}
+
+// whether a program is within the PLAIN form (see above)
+static inline bool program_plain64(const phk_program& prog) {
+    for (int o = 0; o < prog.n_ops; ++o) {
+        const phk_op& op = prog.op[o];
+        if (op.flags & (PHK_FLAG_DISPERSION | PHK_FLAG_SHRINK | PHK_FLAG_P_INC))
+            return false;
+        if (op.kind == PHK_OP_RF_KICK && op.p[6] != op.p[8]) return false;
+        if (op.kind == PHK_OP_TRANSVERSE && (op.flags & PHK_FLAG_DETUNED)) {
+            // I the unit matrix, J without diagonal, no cross terms
+            if (op.ij_mask & ~(0x0609 | 0x6090)) return false;
+            if (op.p[0] != 1.0 || op.p[3] != 1.0 || op.p[4] != 1.0 || op.p[7] != 1.0)
+                return false;
+            for (int d = 0; d < op.det_count; ++d) {
+                const phk_detuner& t = prog.det[op.det_begin + d];
+                if (t.kind == PHK_DET_AMPLITUDE && (t.c[5] != 0.0 || t.c[8] != 0.0))
+                    return false;
+            }
+        }
+    }
+    return true;
+}
+
 // ChromaticitySegment detune: Horner with separately rounded steps, lowest
 // coefficient first, then the extra dp factors of the order > 3 path.
 __device__ __forceinline__ double chroma_poly(const double* c, int n, int z,
@@ -45,122 +144,132 @@ __device__ __forceinline__ double chroma_poly(const double* c, int n, int z,
     return r;
 }
 
-// The detuned map below feeds sin / cos of a per-particle phase, which no
-// FP64 evaluation reproduces bit for bit anyway; its products and sums are
-// therefore fused (one rounding per multiply-add) to save FP64 operations
-// on GB300's narrow FP64 pipe.  Maps without per-particle transcendentals
-// keep the reference's separately rounded order.
-__device__ __forceinline__ double amp_action(double c1, double twoa, double b,
-                                             double u, double up) {
-    // 1/2 * ((1+a^2)/b * u**2 + 2*a * u*up + b * up**2)
-    double s = c1 * u * u;
-    if (twoa != 0.0) s = fma(twoa * u, up, s);
-    s = fma(b * up, up, s);
-    return 0.5 * s;
+// phases of 2^12 radians and more, NaN and infinities: sine and cosine
+// times 2^62
+static __device__ __noinline__ void sincos_far(double phi, double* s, double* c) {
+    sincos(phi, s, c);
+    *s *= 0x1p62;
+    *c *= 0x1p62;
 }
 
-__device__ __forceinline__ double ij_term(double I, double J, bool hi,
-                                          bool hj, double cc, double ss) {
-    if (hi && hj) return fma(I, cc, J * ss);
-    if (hi) return I * cc;
-    if (hj) return J * ss;
-    return 0.0;
+// sine and cosine, times 2^62, of phi radians: phi / 2 pi as a fraction of a
+// turn (1 / 2 pi = 0xa2f9... 2^-66)
+__device__ __forceinline__ void phase_sincos(const u64* tab, double phi, double* s,
+                                             double* c) {
+    if (biased_exp(__double2hiint(phi)) < 1035)
+        sincos_turn(tab, turn_product(phi, 0xa2f9836e4e44152aull, 66), s, c);
+    else
+        sincos_far(phi, s, c);
 }
 
-// OP0 (unused here): see the FP32 form
-template <int VEC, bool OP0 = false>
-__device__ __forceinline__ void op_transverse(const phk_op& op,
+// (u, u') through one plane's detuned map, sine and cosine times 2^62
+__device__ __forceinline__ void detuned_plane(const double* I, const double* J,
+                                              double s, double c, double& u,
+                                              double& up) {
+    const double s1 = unscale62(s), c1 = unscale62(c);
+    const double M00 = fma(I[0], c1, J[0] * s1), M01 = fma(I[1], c1, J[1] * s1);
+    const double M10 = fma(I[2], c1, J[2] * s1), M11 = fma(I[3], c1, J[3] * s1);
+    const double nu = fma(M00, u, M01 * up);
+    up = fma(M10, u, M11 * up);
+    u = nu;
+}
+// the same with unit I and J without diagonal (j01, j10 times 2^-62)
+__device__ __forceinline__ void detuned_plane_unit(double j01, double j10, double s,
+                                                   double c, double& u, double& up) {
+    const double c1 = unscale62(c);
+    const double nu = fma(c1, u, (j01 * s) * up);
+    up = fma(c1, up, (j10 * s) * u);
+    u = nu;
+}
+
+// TransverseSegmentMap.track, plain form.  Without detuners every product
+// and sum is rounded separately in the reference's order.  With detuners the
+// phase (Q + detunings) 2 pi is rounded as the reference rounds it; around
+// the sine and cosine of a per-particle phase, which no evaluation
+// reproduces bit for bit, the arithmetic is regrouped into few multiply-adds
+// (constants from det_fix) and the sine and cosine are fixed-point.  With
+// chromaticity and amplitude detuning, PLAIN: 36 FP64 instructions a
+// particle, conversions included; before, about 110 and as many again in
+// warps with a lane beyond the quarter radian of the former series (a turn
+// of 1e6 macroparticles: 395 -> 122 us).
+template <int VEC, bool PLAIN>
+__device__ __forceinline__ void op_transverse(const phk_op& op, int o,
                                               const phk_program& prog,
+                                              const Aux64& aux,
                                               Tile<double, VEC>& t) {
     const double* p = op.p;
-    const bool disp = op.flags & PHK_FLAG_DISPERSION;
+    const bool disp = !PLAIN && (op.flags & PHK_FLAG_DISPERSION);
     const double Dx0 = p[16], Dx1 = p[17], Dy0 = p[18], Dy1 = p[19];
     double (&x)[VEC] = t.c[PHK_X];
     double (&xp)[VEC] = t.c[PHK_XP];
     double (&y)[VEC] = t.c[PHK_Y];
     double (&yp)[VEC] = t.c[PHK_YP];
     const double (&dp)[VEC] = t.c[PHK_DP];
-    if (!(op.flags & PHK_FLAG_DETUNED)) {
+    // the detuning sees the coordinates before the dispersion is taken out
+    double phx[VEC], phy[VEC];
+    const bool detuned = op.flags & PHK_FLAG_DETUNED;
+    if (detuned) {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) { phx[j] = p[20]; phy[j] = p[21]; }
+        for (int d = 0; d < op.det_count; ++d) {
+            const phk_detuner& dt = prog.det[op.det_begin + d];
+            if (dt.kind == PHK_DET_CHROMA) {
+#pragma unroll
+                for (int j = 0; j < VEC; ++j) {
+                    phx[j] = add(phx[j], chroma_poly(dt.c, dt.nx, dt.zx, dp[j]));
+                    phy[j] = add(phy[j], chroma_poly(dt.c + 8, dt.ny, dt.zy, dp[j]));
+                }
+            } else {
+                const DetFix& f = aux.det[op.det_begin + d];
+#pragma unroll
+                for (int j = 0; j < VEC; ++j) {
+                    double jx = f.gx * x[j], jy = f.gy * y[j];
+                    if (!PLAIN) {
+                        jx = fma(f.tx, xp[j], jx);
+                        jy = fma(f.ty, yp[j], jy);
+                    }
+                    jx = fma(jx, x[j], xp[j] * xp[j]);
+                    jy = fma(jy, y[j], yp[j] * yp[j]);
+                    phx[j] = add(phx[j], fma(f.axx, jx, f.axy * jy));
+                    phy[j] = add(phy[j], fma(f.ayy, jy, f.ayx * jx));
+                }
+            }
+        }
+    }
+    if (disp) {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+            x[j] = sub(x[j], mul(Dx0, dp[j]));
+            y[j] = sub(y[j], mul(Dy0, dp[j]));
+        }
+    }
+    if (detuned) {
+        const double* f = aux.op[o].c;
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+            double s, c;
+            phase_sincos(aux.sine, mul(phx[j], p[22]), &s, &c);
+            if (PLAIN) detuned_plane_unit(f[0], f[1], s, c, x[j], xp[j]);
+            else detuned_plane(p, p + 8, s, c, x[j], xp[j]);
+            phase_sincos(aux.sine, mul(phy[j], p[22]), &s, &c);
+            if (PLAIN) detuned_plane_unit(f[2], f[3], s, c, y[j], yp[j]);
+            else detuned_plane(p + 4, p + 12, s, c, y[j], yp[j]);
+        }
+    } else {
         const double M00 = p[0], M01 = p[1], M10 = p[2], M11 = p[3];
         const double M22 = p[4], M23 = p[5], M32 = p[6], M33 = p[7];
 #pragma unroll
         for (int j = 0; j < VEC; ++j) {
-            if (disp) {
-                x[j] = sub(x[j], mul(Dx0, dp[j]));
-                y[j] = sub(y[j], mul(Dy0, dp[j]));
-            }
             const double nx = add(mul(M00, x[j]), mul(M01, xp[j]));
             const double nxp = add(mul(M10, x[j]), mul(M11, xp[j]));
             const double ny = add(mul(M22, y[j]), mul(M23, yp[j]));
             const double nyp = add(mul(M32, y[j]), mul(M33, yp[j]));
             x[j] = nx; xp[j] = nxp; y[j] = ny; yp[j] = nyp;
-            if (disp) {
-                x[j] = add(x[j], mul(Dx1, dp[j]));
-                y[j] = add(y[j], mul(Dy1, dp[j]));
-            }
-        }
-        return;
-    }
-    double phx[VEC], phy[VEC];
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) { phx[j] = p[20]; phy[j] = p[21]; }
-    for (int d = 0; d < op.det_count; ++d) {
-        const phk_detuner& dt = prog.det[op.det_begin + d];
-        if (dt.kind == PHK_DET_CHROMA) {
-            const int nx = dt.nx, ny = dt.ny, zx = dt.zx, zy = dt.zy;
-#pragma unroll
-            for (int j = 0; j < VEC; ++j) {
-                phx[j] = add(phx[j], chroma_poly(dt.c, nx, zx, dp[j]));
-                phy[j] = add(phy[j], chroma_poly(dt.c + 8, ny, zy, dp[j]));
-            }
-        } else {
-            const double ax = dt.c[0], ay = dt.c[1], axy = dt.c[2], ayx = dt.c[3];
-            const double c1x = dt.c[4], tax = dt.c[5], bx = dt.c[6];
-            const double c1y = dt.c[7], tay = dt.c[8], by = dt.c[9];
-            const double p0 = dt.c[10], ip0 = dt.c[11];
-#pragma unroll
-            for (int j = 0; j < VEC; ++j) {
-                const double Jx = amp_action(c1x, tax, bx, x[j], xp[j]);
-                const double Jy = amp_action(c1y, tay, by, y[j], yp[j]);
-                phx[j] = add(phx[j], div_by(fma(ax, Jx, axy * Jy), p0, ip0));
-                phy[j] = add(phy[j], div_by(fma(ay, Jy, ayx * Jx), p0, ip0));
-            }
         }
     }
-    const double twopi = p[22];
-    const double phx0 = p[23], sx0 = p[24], cx0 = p[25];
-    const double phy0 = p[26], sy0 = p[27], cy0 = p[28];
-    const int m = op.ij_mask;
-    double I[8], J[8];
-    bool hI[8], hJ[8];
+    if (disp) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        I[e] = p[e]; J[e] = p[8 + e];
-        hI[e] = (m >> e) & 1; hJ[e] = (m >> (8 + e)) & 1;
-    }
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) {
-        double sx, cx, sy, cy;
-        sincos_about(mul(phx[j], twopi), phx0, sx0, cx0, &sx, &cx);
-        sincos_about(mul(phy[j], twopi), phy0, sy0, cy0, &sy, &cy);
-        const double M00 = ij_term(I[0], J[0], hI[0], hJ[0], cx, sx);
-        const double M01 = ij_term(I[1], J[1], hI[1], hJ[1], cx, sx);
-        const double M10 = ij_term(I[2], J[2], hI[2], hJ[2], cx, sx);
-        const double M11 = ij_term(I[3], J[3], hI[3], hJ[3], cx, sx);
-        const double M22 = ij_term(I[4], J[4], hI[4], hJ[4], cy, sy);
-        const double M23 = ij_term(I[5], J[5], hI[5], hJ[5], cy, sy);
-        const double M32 = ij_term(I[6], J[6], hI[6], hJ[6], cy, sy);
-        const double M33 = ij_term(I[7], J[7], hI[7], hJ[7], cy, sy);
-        if (disp) {
-            x[j] = sub(x[j], mul(Dx0, dp[j]));
-            y[j] = sub(y[j], mul(Dy0, dp[j]));
-        }
-        const double nx = fma(M00, x[j], M01 * xp[j]);
-        const double nxp = fma(M10, x[j], M11 * xp[j]);
-        const double ny = fma(M22, y[j], M23 * yp[j]);
-        const double nyp = fma(M32, y[j], M33 * yp[j]);
-        x[j] = nx; xp[j] = nxp; y[j] = ny; yp[j] = nyp;
-        if (disp) {
+        for (int j = 0; j < VEC; ++j) {
             x[j] = add(x[j], mul(Dx1, dp[j]));
             y[j] = add(y[j], mul(Dy1, dp[j]));
         }
@@ -180,100 +289,34 @@ __device__ __forceinline__ void op_drift(const phk_op& op,
     }
 }
 
+// Drift of an RFSystems element (Drift, Kick, Drift), PLAIN: beside the
+// kick's inexact sine, one multiply-add with eta0 L.  Other element
+// sequences keep the separately rounded form above.
 template <int VEC>
-__device__ __forceinline__ void op_rfkick(const phk_op& op,
-                                          Tile<double, VEC>& t) {
-    const double* p = op.p;
-    const int f = op.flags;
-    const double h = p[0], twopi = p[1], C = p[2], off = p[3], lock = p[4];
-    const double A = p[5], p0o = p[6], pinc = p[7], p0n = p[8];
-    const double Dx = p[9], Dy = p[10], iC = p[11], ip0n = p[12];
+__device__ __forceinline__ void op_drift_rf(const OpFix& f, Tile<double, VEC>& t) {
 #pragma unroll
-    for (int j = 0; j < VEC; ++j) {
-        double& dp = t.c[PHK_DP][j];
-        if (f & PHK_FLAG_DISPERSION) {
-            t.c[PHK_X][j] = sub(t.c[PHK_X][j], mul(Dx, dp));
-            t.c[PHK_Y][j] = sub(t.c[PHK_Y][j], mul(Dy, dp));
-        }
-        double phi = mul(h, div_by(mul(twopi, t.c[PHK_Z][j]), C, iC));
-        if (f & PHK_FLAG_PHI_OFFSET) phi = add(phi, off);
-        if (f & PHK_FLAG_PHI_LOCK) phi = add(phi, lock);
-        double s = mul(A, sin(phi));
-        if (f & PHK_FLAG_P_INC) s = sub(s, pinc);
-        dp = div_by(add(mul(dp, p0o), s), p0n, ip0n);
-        if (f & PHK_FLAG_DISPERSION) {
-            t.c[PHK_X][j] = add(t.c[PHK_X][j], mul(Dx, dp));
-            t.c[PHK_Y][j] = add(t.c[PHK_Y][j], mul(Dy, dp));
-        }
-    }
+    for (int j = 0; j < VEC; ++j)
+        t.c[PHK_Z][j] = fma(-f.c[0], t.c[PHK_DP][j], t.c[PHK_Z][j]);
 }
 
-// Drift and RF kick of an RFSystems element (Drift, Kick, Drift), plain
-// form.  The kick's per-particle sine makes the step inexact whatever the
-// evaluation order, so around it the arithmetic is regrouped to save FP64
-// operations (GB300 runs FP64 at a small fraction of the FP32 rate): the
-// drift is one multiply-add with eta0 * L, the phase and its sine are
-// fixed-point (turn_product, sine_turn), and the momentum update
+// phase of 2^9 turns and more, NaN and infinities (and factors without a
+// fixed-point form): the sine times 2^62
+static __device__ __noinline__ double rf_sine_far(double z, double hk, double off) {
+    return sin(fma(hk, z, off)) * 0x1p62;
+}
+
+// RF kick, plain form.  The per-particle sine makes the step inexact whatever
+// the evaluation order, so the phase and its sine are fixed-point
+// (turn_product, sine_turn) and the momentum update
 //   dp' = (dp p0_old + A sin(phi) - dp_inc) / p0_new
 // is dp (p0_old / p0_new) + (A / p0_new) sin(phi) - dp_inc / p0_new with
-// the ratios formed once (the ratio is exactly 1 without acceleration).
-// Five FP64 instructions a particle instead of 27 (a turn at 1e7
-// macroparticles and 500 slices, with FixHist64: 1.317 -> 0.873 ms).  The
-// separately rounded forms above remain for other element sequences.
-template <int VEC>
-__device__ __forceinline__ void op_drift_rf(const phk_op& op,
-                                            Tile<double, VEC>& t) {
-    const double br = op.p[0], etaL = op.p[1] * op.p[2];
-    const bool shrink = op.flags & PHK_FLAG_SHRINK;
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) {
-        const double z = t.c[PHK_Z][j];
-        const double zz = shrink ? mul(br, z) : z;
-        t.c[PHK_Z][j] = fma(-etaL, t.c[PHK_DP][j], zz);
-    }
-}
-
-// The constants of op_rfkick_rf, made once per launch (batched form: once
-// per bunch and CTA).
-struct RfFix {
-    TurnFactor k;     // h / C, turns per metre
-    u64 off;          // phase offset and lock, fraction of a turn
-    double hk, offr;  // the same in radians, for far particles
-    double Ar;        // A / p0_new
-    double ratio;     // p0_old / p0_new
-    double pinc;      // dp_inc / p0_new
-};
-
-__host__ __device__ inline void rf_fix(const phk_op& op, RfFix* r) {
-    const double* p = op.p;
-    const int f = op.flags;
-    double off = 0.0;
-    if (f & PHK_FLAG_PHI_OFFSET) off += p[3];
-    if (f & PHK_FLAG_PHI_LOCK) off += p[4];
-    // no usable factor: every particle takes the library's sine
-    if (!turn_factor(p[0], p[2], &r->k)) r->k.exp = -(1 << 20);
-    r->off = angle_fraction(off);
-    r->hk = p[0] * p[1] * p[11];
-    r->offr = off;
-    r->Ar = p[5] * p[12];
-    r->ratio = p[6] == p[8] ? 1.0 : p[6] * p[12];
-    r->pinc = (f & PHK_FLAG_P_INC) ? p[7] * p[12] : 0.0;
-}
-
-// phase of 2^10 turns and more, NaN and infinities (and factors without a
-// fixed-point form)
-static __device__ __noinline__ double rf_sine_far(double z, double hk, double off) {
-    return sin(fma(hk, z, off));
-}
-
-template <int VEC>
-__device__ __forceinline__ void op_rfkick_rf(const phk_op& op, const RfFix& rf,
-                                             const u64* sine,
-                                             Tile<double, VEC>& t) {
-    const bool disp = op.flags & PHK_FLAG_DISPERSION;
+// the ratios formed once: two FP64 instructions a particle instead of 27.
+template <int VEC, bool PLAIN>
+__device__ __forceinline__ void op_rfkick(const phk_op& op, const OpFix& f,
+                                          const u64* sine,
+                                          Tile<double, VEC>& t) {
+    const bool disp = !PLAIN && (op.flags & PHK_FLAG_DISPERSION);
     const double Dx = op.p[9], Dy = op.p[10];
-    const bool constant = rf.ratio == 1.0 && rf.pinc == 0.0;
-    const double A62 = rf.Ar * 0x1p-62;
 #pragma unroll
     for (int j = 0; j < VEC; ++j) {
         double& dp = t.c[PHK_DP][j];
@@ -283,13 +326,12 @@ __device__ __forceinline__ void op_rfkick_rf(const phk_op& op, const RfFix& rf,
         }
         const double z = t.c[PHK_Z][j];
         double s;      // sine, times 2^62
-        if (biased_exp(__double2hiint(z)) <= 968 + rf.k.exp) {
-            const u64 F = turn_product(z, rf.k.mant, rf.k.exp) + rf.off;
-            s = (double)sine_turn(sine, F);
-        } else {
-            s = rf_sine_far(z, rf.hk, rf.offr) * 0x1p62;
-        }
-        dp = constant ? fma(A62, s, dp) : fma(dp, rf.ratio, fma(A62, s, -rf.pinc));
+        if (biased_exp(__double2hiint(z)) <= 968 + f.k.exp)
+            s = (double)sine_turn(sine, turn_product(z, f.k.mant, f.k.exp) + f.off);
+        else
+            s = rf_sine_far(z, f.c[3], f.c[4]);
+        if (PLAIN) dp = fma(f.c[0], s, dp);
+        else dp = fma(dp, f.c[1], fma(f.c[0], s, -f.c[2]));
         if (disp) {
             t.c[PHK_X][j] = add(t.c[PHK_X][j], mul(Dx, dp));
             t.c[PHK_Y][j] = add(t.c[PHK_Y][j], mul(Dy, dp));
@@ -297,13 +339,13 @@ __device__ __forceinline__ void op_rfkick_rf(const phk_op& op, const RfFix& rf,
     }
 }
 
-template <int VEC>
+template <int VEC, bool PLAIN>
 __device__ __forceinline__ void op_linear_long(const phk_op& op,
                                                Tile<double, VEC>& t) {
     const double* p = op.p;
     const double cs = p[0], sn = p[1], lf = p[2], Dx = p[3], Dy = p[4];
     const double ilf = p[5];
-    const bool disp = op.flags & PHK_FLAG_DISPERSION;
+    const bool disp = !PLAIN && (op.flags & PHK_FLAG_DISPERSION);
 #pragma unroll
     for (int j = 0; j < VEC; ++j) {
         double& z = t.c[PHK_Z][j];
@@ -759,14 +801,29 @@ __device__ __forceinline__ void op_damper(const phk_op& op,
 // one dispatch per op per tile (uniform across the CTA)
 template <typename T, int VEC>
 __device__ __forceinline__ void run_program(const phk_program& prog,
-                                            Tile<T, VEC>& t) {
+                                            const Aux64& aux, Tile<T, VEC>& t) {
     for (int o = 0; o < prog.n_ops; ++o) {
         const phk_op& op = prog.op[o];
         switch (op.kind) {
-            case PHK_OP_TRANSVERSE: op_transverse<VEC>(op, prog, t); break;
+            case PHK_OP_TRANSVERSE:
+                if constexpr (std::is_same<T, double>::value)
+                    op_transverse<VEC, false>(op, o, prog, aux, t);
+                else
+                    op_transverse<VEC>(op, prog, t);
+                break;
             case PHK_OP_DRIFT: op_drift<VEC>(op, t); break;
-            case PHK_OP_RF_KICK: op_rfkick<VEC>(op, t); break;
-            case PHK_OP_LINEAR_LONG: op_linear_long<VEC>(op, t); break;
+            case PHK_OP_RF_KICK:
+                if constexpr (std::is_same<T, double>::value)
+                    op_rfkick<VEC, false>(op, aux.op[o], aux.sine, t);
+                else
+                    op_rfkick<VEC>(op, t);
+                break;
+            case PHK_OP_LINEAR_LONG:
+                if constexpr (std::is_same<T, double>::value)
+                    op_linear_long<VEC, false>(op, t);
+                else
+                    op_linear_long<VEC>(op, t);
+                break;
             case PHK_OP_SCALE_TRANS: op_scale<VEC>(op, t); break;
             case PHK_OP_DAMPER: op_damper<VEC>(op, t); break;
             default: break;
@@ -785,31 +842,30 @@ enum TrackShape {
     SHAPE_T_LIN = 4,     // transverse, linear longitudinal map
 };
 
-// sine, rf: the staged quarter wave and the kick's constants (FP64 SHAPE_T_RF)
 template <typename T, int VEC, int SHAPE>
 __device__ __forceinline__ void run_program_shape(const phk_program& prog,
-                                                  const u64* sine, const RfFix* rf,
+                                                  const Aux64& aux,
                                                   Tile<T, VEC>& t) {
-    if constexpr (SHAPE == SHAPE_NONE) {
-        return;
-    } else if constexpr (SHAPE == SHAPE_T) {
+    if constexpr (SHAPE == SHAPE_GENERIC) {
+        run_program<T, VEC>(prog, aux, t);
+    } else if constexpr (SHAPE != SHAPE_NONE && std::is_same<T, double>::value) {
+        op_transverse<VEC, true>(prog.op[0], 0, prog, aux, t);
+        if constexpr (SHAPE == SHAPE_T_RF) {
+            op_drift_rf<VEC>(aux.op[1], t);
+            op_rfkick<VEC, true>(prog.op[2], aux.op[2], aux.sine, t);
+            op_drift_rf<VEC>(aux.op[3], t);
+        } else if constexpr (SHAPE == SHAPE_T_LIN) {
+            op_linear_long<VEC, true>(prog.op[1], t);
+        }
+    } else if constexpr (SHAPE != SHAPE_NONE) {
         op_transverse<VEC, true>(prog.op[0], prog, t);
-    } else if constexpr (SHAPE == SHAPE_T_RF) {
-        op_transverse<VEC, true>(prog.op[0], prog, t);
-        if constexpr (std::is_same<T, double>::value) {
-            op_drift_rf<VEC>(prog.op[1], t);
-            op_rfkick_rf<VEC>(prog.op[2], *rf, sine, t);
-            op_drift_rf<VEC>(prog.op[3], t);
-        } else {
+        if constexpr (SHAPE == SHAPE_T_RF) {
             op_drift<VEC>(prog.op[1], t);
             op_rfkick<VEC>(prog.op[2], t);
             op_drift<VEC>(prog.op[3], t);
+        } else if constexpr (SHAPE == SHAPE_T_LIN) {
+            op_linear_long<VEC>(prog.op[1], t);
         }
-    } else if constexpr (SHAPE == SHAPE_T_LIN) {
-        op_transverse<VEC, true>(prog.op[0], prog, t);
-        op_linear_long<VEC>(prog.op[1], t);
-    } else {
-        run_program<T, VEC>(prog, t);
     }
 }
 
@@ -1087,11 +1143,6 @@ struct TrackArgs {
     int32_t reserved;
 };
 
-// element sequences whose FP64 form reads the staged quarter wave
-template <typename T, int SHAPE>
-constexpr bool needs_sine() {
-    return std::is_same<T, double>::value && SHAPE == SHAPE_T_RF;
-}
 constexpr size_t kSineBytes = ((size_t)kSineEntries * sizeof(u64) + 15) & ~(size_t)15;
 
 template <typename T>
@@ -1332,6 +1383,10 @@ __device__ __forceinline__ void stage_pending(const phk_kick_set& pk,
     }
 }
 
+static __device__ __noinline__ double add_cold(double a, double b) {
+    return add(a, b);
+}
+
 // Wake kicks left pending by the previous WakeField.track, applied in
 // kick order to the VEC particles of a tile in registers
 // (DipoleWakeKickX/Y.apply, impedances/wake_kicks.py:207-260, and the
@@ -1359,8 +1414,14 @@ __device__ __forceinline__ void apply_pending(const phk_kick_set& pk,
                 t.c[PHK_XP][j] = tadd<T>(t.c[PHK_XP][j], on ? ktab[a.comb_slot[0] * Sp + s] : T(0));
             if (a.comb_slot[1] >= 0)
                 t.c[PHK_YP][j] = tadd<T>(t.c[PHK_YP][j], on ? ktab[a.comb_slot[1] * Sp + s] : T(0));
-            if (a.comb_slot[2] >= 0)
-                t.c[PHK_DP][j] = tadd<T>(t.c[PHK_DP][j], on ? ktab[a.comb_slot[2] * Sp + s] : T(0));
+            if (a.comb_slot[2] >= 0) {
+                const T kick = on ? ktab[a.comb_slot[2] * Sp + s] : T(0);
+                // rarely there: out of line, it costs the FP64 pipe nothing
+                if constexpr (std::is_same<T, double>::value)
+                    t.c[PHK_DP][j] = add_cold(t.c[PHK_DP][j], kick);
+                else
+                    t.c[PHK_DP][j] = tadd<T>(t.c[PHK_DP][j], kick);
+            }
         }
     } else {
 #pragma unroll
@@ -1398,8 +1459,7 @@ struct TrackCtx {
     unsigned epoch;
     bool shared_hist;
     typename FixOf<T>::type fix;   // single-bunch accumulation
-    const u64* sine;      // FP64, SHAPE_T_RF: staged quarter wave,
-    const RfFix* rf;      // constants of the RF kick
+    Aux64 aux;            // FP64 form
 };
 
 // One tile of VEC particles per thread, already in registers: pending
@@ -1416,7 +1476,7 @@ __device__ __forceinline__ void run_tile(const phk_program& prog,
     // 1. wake kicks of the previous WakeField.track, in kick order
     if (a.has_pk) apply_pending<T, VEC, FULL>(pk, a, cx.bpk, cx.ktab, t, i0);
     // 2. element program
-    run_program_shape<T, VEC, SHAPE>(prog, cx.sine, cx.rf, t);
+    run_program_shape<T, VEC, SHAPE>(prog, cx.aux, t);
     // 3. slice accumulation
     if (a.has_acc) {
         int sl[VEC];
@@ -2118,7 +2178,9 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
     const int nk = a.has_pk ? pk.n_kicks : 0;
     phk_program* sprog = reinterpret_cast<phk_program*>(smem);
     u64* sine = reinterpret_cast<u64*>(smem + kProgSmem);
-    __shared__ RfFix s_rf;
+    constexpr bool F64 = sizeof(T) == 8;
+    __shared__ OpFix s_op[F64 ? PHK_MAX_OPS : 1];
+    __shared__ DetFix s_det[F64 ? PHK_MAX_DETUNERS : 1];
     unsigned char* rest = smem + batch_head<T>();
     size_t off[9];
     track_smem_layout<T>(Sa, Sp, a.n_hist, nk, 1, 0, TILE, off);
@@ -2143,11 +2205,10 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
         const T* e = reinterpret_cast<const T*>(pk.slicer.edges);
         for (int i = tid; i <= Sp; i += THREADS) stage_edge<T>(epk, i, e[i]);
     }
-    if (needs_sine<T, SHAPE>()) stage_sine(sine, tid, THREADS);
+    if (F64) stage_sine(sine, tid, THREADS);
 
     TrackCtx<T, VEC> cx;
-    cx.sine = sine;
-    cx.rf = &s_rf;
+    cx.aux = Aux64{sine, s_op, s_det};
 #pragma unroll
     for (int q = 0; q < 6; ++q) cx.cp[q] = reinterpret_cast<T*>(a.c[q]);
     cx.ktab = ktab;
@@ -2209,8 +2270,12 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
             int4* dst = reinterpret_cast<int4*>(sprog);
             for (int i = tid; i < (int)(sizeof(phk_program) / 16); i += THREADS)
                 dst[i] = src[i];
-            if (needs_sine<T, SHAPE>() && tid == 0)
-                rf_fix(b.programs[U.bunch].op[2], &s_rf);
+            if constexpr (F64) {
+                const phk_program& bp = b.programs[U.bunch];
+                if (tid < PHK_MAX_OPS) op_fix(bp.op[tid], s_op + tid);
+                if (tid < PHK_MAX_DETUNERS && bp.det[tid].kind == PHK_DET_AMPLITUDE)
+                    det_fix(bp.det[tid], s_det + tid);
+            }
             if (a.has_pk) {
                 const T* kt = reinterpret_cast<const T*>(b.kicks) +
                               (int64_t)U.bunch * nk * Sp;

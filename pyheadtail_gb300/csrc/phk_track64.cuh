@@ -13,7 +13,9 @@ namespace phk {
 
 struct Track64Args {
     TrackArgs t;
-    RfFix rf;              // SHAPE_T_RF
+    OpFix op[PHK_MAX_OPS];
+    DetFix det[PHK_MAX_DETUNERS];
+    int32_t sine;          // the program needs the quarter wave
     int32_t share_edges;   // the kicks' slicing is the accumulation's
 };
 
@@ -85,8 +87,7 @@ track64_kernel(const __grid_constant__ phk_program prog,
     const TrackArgs& a = ka.t;
     const int Sa = a.has_acc ? acc.slicer.n_slices : 0;
     const int Sp = a.has_pk ? pk.slicer.n_slices : 0;
-    const Track64Smem lay = track64_smem(Sa, Sp, a.n_tables, ka.share_edges,
-                                         needs_sine<double, SHAPE>());
+    const Track64Smem lay = track64_smem(Sa, Sp, a.n_tables, ka.share_edges, ka.sine);
     int* words = reinterpret_cast<int*>(smem + lay.words);
     unsigned* flags = reinterpret_cast<unsigned*>(smem + lay.flags);
     double* eacc = reinterpret_cast<double*>(smem + lay.eacc);
@@ -115,13 +116,12 @@ track64_kernel(const __grid_constant__ phk_program prog,
     }
     if (a.has_pk)
         stage_pending<double>(pk, a, epk, ktab, tid, kTrackThreads, ka.share_edges);
-    if (needs_sine<double, SHAPE>()) stage_sine(sine, tid, kTrackThreads);
+    if (ka.sine) stage_sine(sine, tid, kTrackThreads);
     __syncthreads();
     if (a.has_pk) cx.bpk.init(epk, Sp, pk.slicer.negate);
     if (a.has_acc) cx.bac.init(eacc, Sa, acc.slicer.negate);
     cx.ktab = ktab;
-    cx.sine = sine;
-    cx.rf = &ka.rf;
+    cx.aux = Aux64{sine, ka.op, ka.det};
 
     // partial column of this CTA's cluster
     const bool clustered = a.has_acc && a.cluster > 1;
@@ -331,10 +331,12 @@ static int launch_track64_t(const phk_program* prog, const phk_coords* c,
     a.cluster = 1;
     const int64_t per_tile = (int64_t)kTrackThreads * VEC;
     a.n_tiles = (c->n + per_tile - 1) / per_tile;
-    constexpr bool sine = needs_sine<double, SHAPE>();
-    if (sine) rf_fix(prog->op[2], &ka.rf);
+    ka.sine = program_has_phase(*prog);
+    for (int o = 0; o < prog->n_ops; ++o) op_fix(prog->op[o], ka.op + o);
+    for (int d = 0; d < prog->n_det; ++d)
+        if (prog->det[d].kind == PHK_DET_AMPLITUDE) det_fix(prog->det[d], ka.det + d);
     const size_t limit = track64_limit<VEC, SHAPE>();
-    const size_t smem = track64_plan(pk, acc, sine, limit, &ka);
+    const size_t smem = track64_plan(pk, acc, ka.sine, limit, &ka);
     if (smem > limit)
         return set_error(PHK_ESIZE, "phk_track: %zu bytes of shared memory "
                          "needed for %d + %d slices", smem,

@@ -8,7 +8,7 @@ int launch_track_f64(const phk_program* prog, const phk_coords* c,
                      int stm, bool vec_ok, cudaStream_t st) {
     if (!vec_ok)
         return launch_track64_t<1, SHAPE_GENERIC>(prog, c, pk, acc, ld, stm, st);
-    switch (program_shape(prog)) {
+    switch (program_plain64(*prog) ? program_shape(prog) : (int)SHAPE_GENERIC) {
         case SHAPE_NONE:
             return launch_track64_t<2, SHAPE_NONE>(prog, c, pk, acc, ld, stm, st);
         case SHAPE_T:
@@ -31,7 +31,8 @@ int track_clusters_f64(size_t smem) {
 static int batch_shape(const phk_batch* bt) {
     int sh = -1;
     for (int i = 0; i < bt->n_bunches; ++i) {
-        const int s = program_shape(bt->programs_host + i);
+        const int s = program_plain64(bt->programs_host[i])
+                          ? program_shape(bt->programs_host + i) : (int)SHAPE_GENERIC;
         if (sh < 0) sh = s;
         else if (s != sh) return SHAPE_GENERIC;
     }
