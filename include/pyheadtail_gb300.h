@@ -518,6 +518,16 @@ int phk_slice_moments(const phk_slicer *slicer, const void *z, int64_t n,
                       int32_t pass, const double *means, double *sums,
                       int32_t *counts, void *stream);
 
+/* The same for all six coordinates at once:
+ *   pass 0: sums[q][s] += u_q (double[6][S]), counts[s] += 1
+ *   pass 1: sums[pair][s] (double[13][S]), means double[6][S] given, for
+ *           (x,x) (y,y) (z,z) (dp,dp) (x,xp) (y,yp) (z,dp) (xp,xp) (yp,yp)
+ *           (x,dp) (y,dp) (xp,dp) (yp,dp)
+ * all accumulated.                                                        */
+int phk_slice_moments_all(const phk_slicer *slicer, const phk_coords *coords,
+                          int32_t pass, const double *means, double *sums,
+                          int32_t *counts, void *stream);
+
 /* Batched fused pass (see phk_batch): per unit, the pending kicks of its
  * bunch (tables batch->kicks; `pending` gives n_kicks, quad, target and the
  * slicer, its kick[] pointers are ignored), the bunch's program, binning

@@ -167,6 +167,10 @@ SIGNATURES = {
                           ctypes.POINTER(ctypes.c_void_p), ctypes.c_int32,
                           ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p,
                           ctypes.c_void_p, ctypes.c_void_p],
+    'phk_slice_moments_all': [ctypes.POINTER(Slicer), ctypes.POINTER(Coords),
+                              ctypes.c_int32, ctypes.c_void_p,
+                              ctypes.c_void_p, ctypes.c_void_p,
+                              ctypes.c_void_p],
     'phk_track_batch': [ctypes.POINTER(Batch), ctypes.POINTER(Coords),
                         ctypes.POINTER(KickSet), ctypes.POINTER(Accum),
                         ctypes.c_void_p],

@@ -404,6 +404,27 @@ int phk_slice_moments(const phk_slicer* slicer, const void* z, int64_t n,
                           sums, counts, (cudaStream_t)stream);
 }
 
+int phk_slice_moments_all(const phk_slicer* slicer, const phk_coords* coords,
+                          int32_t pass, const double* means, double* sums,
+                          int32_t* counts, void* stream) {
+    const char* who = "phk_slice_moments_all";
+    if (!slicer) return set_error(PHK_ENULL, "%s: slicer is NULL", who);
+    int r = check_slicer(slicer, who);
+    if (r) return r;
+    if ((r = check_coords(coords, who))) return r;
+    if ((r = check_edges(slicer, coords->dtype, who))) return r;
+    if (pass != 0 && pass != 1) return set_error(PHK_EPARAM, "%s: pass", who);
+    if (!sums) return set_error(PHK_ENULL, "%s: sums is NULL", who);
+    if (pass == 0 && !counts) return set_error(PHK_ENULL, "%s: counts", who);
+    if (pass == 1 && !means) return set_error(PHK_ENULL, "%s: means", who);
+    if (reinterpret_cast<uintptr_t>(sums) % 8 || reinterpret_cast<uintptr_t>(means) % 8 ||
+        reinterpret_cast<uintptr_t>(counts) % 4)
+        return set_error(PHK_EALIGN, "%s: sums, means or counts misaligned", who);
+    if (coords->n == 0) return PHK_OK;
+    return launch_moments_all(slicer, coords, pass, means, sums, counts,
+                              (cudaStream_t)stream);
+}
+
 int phk_track_batch(const phk_batch* batch, const phk_coords* coords,
                     const phk_kick_set* pending, const phk_accum* acc,
                     void* stream) {

@@ -52,6 +52,24 @@ __device__ __forceinline__ u64 shr_clamp(u64 v, int r) {
 // whatever the number of lanes left (19 cycles of the FP64 pipe each, 2 to
 // 5 rounds at 500 to 50 slices).
 // -------------------------------------------------------------------
+
+// adds u to the four digits at d (shared memory; k: the unit, fix64_k); false
+// if it is out of the fixed point's range
+__device__ __forceinline__ bool fix64_add(int* d, int k, double u) {
+    const int hi = __double2hiint(u), lo = __double2loint(u);
+    const int r = k - biased_exp(hi);
+    if (r < 2) return false;
+    u64 v = shr_clamp(mant64(hi, lo), r);
+    if (hi < 0) v = 0ull - v;
+    const unsigned vl = (unsigned)v;
+    const int vh = (int)(v >> 32);
+    atomicAdd(d, (int)(vl & 0xffffu));
+    atomicAdd(d + 1, (int)(vl >> 16));
+    atomicAdd(d + 2, vh & 0xffff);
+    atomicAdd(d + 3, vh >> 16);
+    return true;
+}
+
 constexpr int kFix64Words = 9;   // per slice: count, 4 digits of x, 4 of y
 
 struct FixHist64 {
@@ -61,22 +79,10 @@ struct FixHist64 {
     int k[2];             // v = mant64 >> (k[q] - e)
 
     __device__ __forceinline__ void add_q(int q, int s, double u) const {
-        const int hi = __double2hiint(u), lo = __double2loint(u);
-        const int r = k[q] - biased_exp(hi);
-        if (r < 2) {
+        if (!fix64_add(w + s * kFix64Words + 1 + 4 * q, k[q], u)) {
             atomicOr(flag + (s >> 2), 1u << (8 * (s & 3) + q));
             *any = 1;
-            return;
         }
-        u64 v = shr_clamp(mant64(hi, lo), r);
-        if (hi < 0) v = 0ull - v;
-        const unsigned vl = (unsigned)v;
-        const int vh = (int)(v >> 32);
-        int* d = w + s * kFix64Words + 1 + 4 * q;
-        atomicAdd(d, (int)(vl & 0xffffu));
-        atomicAdd(d + 1, (int)(vl >> 16));
-        atomicAdd(d + 2, vh & 0xffff);
-        atomicAdd(d + 3, vh >> 16);
     }
     __device__ __forceinline__ void add(int s, double x, double y) const {
         atomicAdd(w + s * kFix64Words, 1);

@@ -59,6 +59,10 @@ int launch_moments(const phk_slicer* s, const void* z, int64_t n,
                    int32_t pass, const double* means, double* sums,
                    int32_t* counts, cudaStream_t stream);
 
+int launch_moments_all(const phk_slicer* s, const phk_coords* c, int32_t pass,
+                       const double* means, double* sums, int32_t* counts,
+                       cudaStream_t stream);
+
 int plan_wake_tc(phk_wake_tc* w, int64_t* a_elems, int64_t* partial_elems);
 int launch_wake_tc_expand(const phk_wake_tc* w, cudaStream_t stream);
 int launch_wake_tc(const phk_wake_tc* w, cudaStream_t stream);

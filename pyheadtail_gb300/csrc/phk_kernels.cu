@@ -1,8 +1,8 @@
 // Host-side planning and the small kernels around the fused pass: the
 // launch dispatch of the track kernels (instantiated per precision in
 // phk_track_f32.cu / phk_track_f64.cu), the fixed-order merge of the
-// per-CTA partials, the wake convolution, the per-slice moment kernel and
-// the batched merge / wake kernels.
+// per-CTA partials, the wake convolution and the batched merge / wake
+// kernels.
 #include "phk_track64.cuh"
 
 namespace phk {
@@ -417,80 +417,6 @@ int launch_wake(const phk_wake_set* w, cudaStream_t st) {
     count_launches((int)any_conv + (int)any_dense);
     return PHK_OK;
 }
-
-// ===================================================================
-// per-slice moments for statistics (two passes, global FP64 atomics)
-// ===================================================================
-
-template <typename T>
-__global__ void moments_kernel(const __grid_constant__ phk_slicer sl,
-                               const T* __restrict__ z, int64_t n,
-                               const T* __restrict__ q0,
-                               const T* __restrict__ q1,
-                               const T* __restrict__ q2, int n_q, int pass,
-                               const double* __restrict__ means,
-                               double* sums, int32_t* counts) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int S = sl.n_slices;
-    T* e = reinterpret_cast<T*>(smem);
-    for (int i = threadIdx.x; i <= S; i += blockDim.x)
-        e[i] = reinterpret_cast<const T*>(sl.edges)[i];
-    __syncthreads();
-    const T tail = T(sl.est_tail), iw = T(sl.est_inv_w);
-    const T* qs[3] = {q0, q1, q2};
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int s = slice_of<T>(z[i], S, sl.negate, tail, iw, e);
-        if (s < 0) continue;
-        if (pass == 0) {
-            atomicAdd(counts + s, 1);
-            for (int q = 0; q < n_q; ++q)
-                atomicAdd(sums + (int64_t)q * S + s, (double)qs[q][i]);
-        } else {
-            double d[3];
-            for (int q = 0; q < n_q; ++q)
-                d[q] = (double)qs[q][i] - means[(int64_t)q * S + s];
-            // pairs (0,0) (0,1) (1,1) (0,2) (1,2) (2,2)
-            const int pa[6] = {0, 0, 1, 0, 1, 2}, pb[6] = {0, 1, 1, 2, 2, 2};
-            for (int p = 0; p < 6; ++p) {
-                if (pa[p] >= n_q || pb[p] >= n_q) continue;
-                atomicAdd(sums + (int64_t)(3 + p) * S + s, d[pa[p]] * d[pb[p]]);
-            }
-        }
-    }
-}
-
-int launch_moments(const phk_slicer* sl, const void* z, int64_t n,
-                   int32_t dtype, const void* const* q, int32_t n_q,
-                   int32_t pass, const double* means, double* sums,
-                   int32_t* counts, cudaStream_t st) {
-    const DeviceInfo& d = device_info();
-    const int threads = 256;
-    int64_t blocks = (n + threads - 1) / threads;
-    if (blocks > (int64_t)d.sm_count * 8) blocks = (int64_t)d.sm_count * 8;
-    if (blocks < 1) blocks = 1;
-    const void* qq[3] = {nullptr, nullptr, nullptr};
-    for (int i = 0; i < n_q; ++i) qq[i] = q[i];
-    if (dtype == PHK_F64) {
-        const size_t smem = sizeof(double) * (sl->n_slices + 1);
-        moments_kernel<double><<<(int)blocks, threads, smem, st>>>(
-            *sl, (const double*)z, n, (const double*)qq[0],
-            (const double*)qq[1], (const double*)qq[2], n_q, pass, means,
-            sums, counts);
-    } else {
-        const size_t smem = sizeof(float) * (sl->n_slices + 1);
-        moments_kernel<float><<<(int)blocks, threads, smem, st>>>(
-            *sl, (const float*)z, n, (const float*)qq[0], (const float*)qq[1],
-            (const float*)qq[2], n_q, pass, means, sums, counts);
-    }
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess)
-        return set_error(PHK_ECUDA, "phk_slice_moments launch: %s",
-                         cudaGetErrorString(e));
-    count_launches(1);
-    return PHK_OK;
-}
-
 
 // ===================================================================
 // batched form: dispatch, merge and wake

@@ -14,6 +14,7 @@ array ``slice_index_of_particle`` is produced on demand by a slicing pass;
 it can only be produced while the beam's z is still the one the SliceSet
 was made from (SliceSets describe a past state), otherwise it raises.
 """
+import ctypes
 from abc import ABCMeta, abstractmethod
 from functools import partial, wraps
 
@@ -609,7 +610,7 @@ def make_slice_set(slicer, beam, with_means=False, moments_out=None):
                                 E.stream_handle())
     else:
         a = acc.struct()
-        N.call('phk_slice_finalize', __import__('ctypes').byref(a),
+        N.call('phk_slice_finalize', ctypes.byref(a),
                counts.data_ptr(), 0 if mx is None else mx.data_ptr(),
                0 if my is None else my.data_ptr(),
                0 if moments_out is None else moments_out.data_ptr(),
@@ -635,7 +636,6 @@ ALL_STATS = ['mean_x', 'mean_y', 'mean_z', 'mean_xp', 'mean_yp', 'mean_dp',
 def _slice_moments(ss, beam, names):
     """Per-slice means and centred second moments of up to three
     coordinates (two passes of phk_slice_moments; stats.pyx:235-425)."""
-    import ctypes
     S = ss.n_slices
     dev = beam._device
     eng = beam._engine
@@ -662,11 +662,79 @@ def _slice_moments(ss, beam, names):
     return means, cov, counts
 
 
+def _all_slice_moments(ss, beam):
+    """Per-slice means of the six coordinates and the 13 centred second
+    moments some statistic uses (two passes of phk_slice_moments_all), in
+    that entry point's order."""
+    S = ss.n_slices
+    dev = beam._device
+    eng = beam._engine
+    if not eng.idle:
+        eng.flush()
+    coords = ctypes.byref(eng.coords_struct())
+    sl = ctypes.byref(ss._dslicer.struct)
+    sums = torch.zeros(19, S, dtype=torch.float64, device=dev)
+    counts = torch.zeros(S, dtype=torch.int32, device=dev)
+    N.call('phk_slice_moments_all', sl, coords, 0, None, sums.data_ptr(),
+           counts.data_ptr(), E.stream_handle())
+    n = counts.double()
+    means = torch.where(counts > 0, sums[:6] / n.clamp(min=1), 0.)
+    N.call('phk_slice_moments_all', sl, coords, 1, means.data_ptr(),
+           sums[6:].data_ptr(), None, E.stream_handle())
+    cov = torch.where(counts > 1, sums[6:] / (n - 1).clamp(min=1), sums[6:])
+    return means, cov, counts
+
+
+def _emittance(s11, s12, s22, counts, disp=None):
+    """stats.pyx:374-425; disp: covariances (u,dp) (up,dp) (dp,dp)."""
+    if disp is not None:
+        c1, c2, cdp2 = disp
+        ok = cdp2 != 0
+        safe = torch.where(ok, cdp2, 1.)
+        s11 = torch.where(ok, s11 - c1 * c1 / safe, s11)
+        s12 = torch.where(ok, s12 - c1 * c2 / safe, s12)
+        s22 = torch.where(ok, s22 - c2 * c2 / safe, s22)
+    return torch.where(counts > 1, torch.sqrt(s11 * s22 - s12 * s12), 0.)
+
+
+def _add_many_statistics(ss, beam, names):
+    """The named statistics from one set of moments; rows of shared
+    tensors."""
+    means, cov, counts = _all_slice_moments(ss, beam)
+    values = dict(zip(['mean_' + k for k in ('x', 'xp', 'y', 'yp', 'z', 'dp')],
+                      means.unbind()))
+    if any(k.startswith('sigma_') for k in names):
+        values.update(zip(['sigma_x', 'sigma_y', 'sigma_z', 'sigma_dp'],
+                          torch.sqrt(cov[:4]).unbind()))
+    s11, s12, s22 = cov[0:2], cov[4:6], cov[7:9]
+    if 'epsn_x' in names or 'epsn_y' in names:
+        em = _emittance(s11, s12, s22, counts, (cov[9:11], cov[11:13], cov[3]))
+        values.update(zip(['epsn_x', 'epsn_y'],
+                          (em * beam.betagamma).unbind()))
+    if 'eff_epsn_x' in names or 'eff_epsn_y' in names:
+        em = _emittance(s11, s12, s22, counts)
+        values.update(zip(['eff_epsn_x', 'eff_epsn_y'],
+                          (em * beam.betagamma).unbind()))
+    if 'epsn_z' in names:
+        em = _emittance(cov[2], cov[6], cov[3], counts)
+        values['epsn_z'] = 4. * np.pi * em * beam.p0 / e
+    for k in names:
+        setattr(ss, k, values[k])
+
+
 def add_statistics(ss, beam, statistics):
     """Slicer.add_statistics (slicing.py:443-529) for the GPU SliceSet."""
     if statistics is True:
         statistics = ALL_STATS
     sh = getattr(beam, '_shard', None)
+    # more than two statistics (more than four passes one by one): the
+    # moments of all of them in two passes
+    wanted = [k for k in dict.fromkeys(statistics) if not hasattr(ss, k)]
+    if len(wanted) > 2 and all(k in ALL_STATS for k in wanted) and \
+            (sh is None or sh.world <= 1) and \
+            all(k in beam._c for k in ('x', 'xp', 'y', 'yp', 'z', 'dp')):
+        _add_many_statistics(ss, beam, wanted)
+        return
     for stat in statistics:
         if hasattr(ss, stat):
             continue
@@ -691,16 +759,8 @@ def add_statistics(ss, beam, statistics):
                 disp = not stat.startswith('eff')
             _, cov, counts = _slice_moments(ss, beam, names)
             # pairs: 0 (u,u) 1 (u,up) 2 (up,up) 3 (u,dp) 4 (up,dp) 5 (dp,dp)
-            s11, s12, s22 = cov[0].clone(), cov[1].clone(), cov[2].clone()
-            if disp:
-                cdp2 = cov[5]
-                ok = cdp2 != 0
-                safe = torch.where(ok, cdp2, torch.ones_like(cdp2))
-                s11 = torch.where(ok, s11 - cov[3] * cov[3] / safe, s11)
-                s12 = torch.where(ok, s12 - cov[3] * cov[4] / safe, s12)
-                s22 = torch.where(ok, s22 - cov[4] * cov[4] / safe, s22)
-            em = torch.where(counts > 1, torch.sqrt(s11 * s22 - s12 * s12),
-                             torch.zeros_like(s11))
+            em = _emittance(cov[0], cov[1], cov[2], counts,
+                            cov[3:6] if disp else None)
             if stat == 'epsn_z':
                 em = 4. * np.pi * em * beam.p0 / e
             else:
