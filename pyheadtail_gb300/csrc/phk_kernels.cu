@@ -348,14 +348,14 @@ __device__ __forceinline__ void wake_dense_one(const phk_wake_set& w, int t) {
         reinterpret_cast<float*>(kk.out)[i] = (float)r;
 }
 
-// Single-bunch numpy path: one CTA of kConvWarps warps per (kick, target
-// slice); warp w takes the stored turns w, w + kConvWarps, ...; the warps'
+// Single-bunch numpy path, little work: one CTA of kDirectWarps warps per (kick, target
+// slice); warp w takes the stored turns w, w + kDirectWarps, ...; the warps'
 // partial sums are added in a fixed order.  (One warp per output leaves
 // too few warps on GB300 to cover the load latency of a 50-turn history.)
-constexpr int kConvWarps = 8;
-__global__ void __launch_bounds__(kConvWarps * 32)
-wake_conv_kernel(const __grid_constant__ phk_wake_set w) {
-    __shared__ double part_w[kConvWarps];
+constexpr int kDirectWarps = 8;
+__global__ void __launch_bounds__(kDirectWarps * 32)
+wake_direct_kernel(const __grid_constant__ phk_wake_set w) {
+    __shared__ double part_w[kDirectWarps];
     const int S = w.n_slices;
     const int k = blockIdx.x / S;
     const int i = blockIdx.x - k * S;
@@ -365,7 +365,7 @@ wake_conv_kernel(const __grid_constant__ phk_wake_set w) {
     if (kk.dense) return;
     const int L2 = 2 * S - 1;
     double p0 = 0.0, p1 = 0.0, p2 = 0.0, p3 = 0.0;
-    for (int a = warp; a < kk.n_lags; a += kConvWarps) {
+    for (int a = warp; a < kk.n_lags; a += kDirectWarps) {
         const int slot = ((w.head - a) % w.ring_len + w.ring_len) % w.ring_len;
         const double* m = w.moments + ((int64_t)slot * 3 + kk.source) * S;
         const double* v = kk.table + (int64_t)a * L2 + i + S - 1;
@@ -386,13 +386,163 @@ wake_conv_kernel(const __grid_constant__ phk_wake_set w) {
     __syncthreads();
     if (threadIdx.x == 0) {
         double acc = part_w[0];
-        for (int q = 1; q < kConvWarps; ++q) acc += part_w[q];
+        for (int q = 1; q < kDirectWarps; ++q) acc += part_w[q];
         const double r = mul(kk.factor, acc);
         if (w.out_dtype == PHK_F64)
             reinterpret_cast<double*>(kk.out)[i] = r;
         else
             reinterpret_cast<float*>(kk.out)[i] = (float)r;
     }
+}
+
+// Single-bunch numpy path, more work.  S^2 multiply-adds per stored turn
+// and kick, 25 million a turn with a 50-turn wake at 500 slices: 49 us of the
+// FP64 pipe alone.  As integers they are cheaper: the factors become 54-bit
+// fixed-point numbers in two 27-bit limbs, a product is four 32 x 32 + 64 bit
+// multiply-adds into 64-bit sums (high, two middle, low), exact over a unit of
+// up to 96 source slices, and one conversion and FP64 multiply-add takes a
+// unit's sum to the output.  Two 50-turn kicks at 500 slices: 95 -> 28 us
+// (the direct kernel below a million multiply-adds), bound by the wide
+// multiply-adds; errors against extended precision 2.3e-16 (2.5e-16 before).
+// Clusters of 8 would be packed two CTAs to an SM and leave half the SMs idle
+// (45 us).
+//
+// One cluster of kConvCluster CTAs per (kick, block of 32 target slices); its
+// warps share the (stored turn, chunk of source slices) units.  A warp loads
+// a unit's sources and its window of the table, finds the largest magnitude
+// of each (the unit's own scales, so a decaying wake keeps its relative
+// accuracy: each factor is off by at most 2^-54 of the largest in the window),
+// converts them into its part of shared memory and accumulates one target
+// per lane.  Warps, then CTAs, are added in a fixed order.  A unit with a
+// non-finite, subnormal or extreme factor runs in FP64 (conv_unit_fp64).
+constexpr int kConvWarps = 16;
+constexpr int kConvCluster = 4;
+constexpr int kConvTargets = 32;    // per cluster, one per lane
+constexpr int kConvSources = 96;    // per unit, at most (27 + 27 + 1 + 7 < 63 bits)
+constexpr int kConvWindow = kConvSources + kConvTargets - 1;
+
+// v as two 27-bit limbs of a 54-bit integer, r: mant64 shift
+__device__ __forceinline__ int2 conv_limbs(double v, int e_max) {
+    const int hi = __double2hiint(v), lo = __double2loint(v);
+    const int r = e_max + 10 - biased_exp(hi);       // 10 for the largest
+    long long q = (long long)((shr_clamp(mant64(hi, lo), r - 1) + 1) >> 1);
+    if (hi < 0) q = -q;
+    return make_int2((int)(q & 0x7ffffff), (int)(q >> 27));
+}
+
+__device__ __forceinline__ void conv_unit_fp64(const double* m, const double* tab,
+                                               int len, int i, int S, double& acc) {
+    if (i >= S) return;
+    for (int j = 0; j < len; ++j) acc = fma(m[j], tab[i - j], acc);
+}
+
+__global__ void __cluster_dims__(kConvCluster, 1, 1) __launch_bounds__(kConvWarps * 32)
+wake_conv_kernel(const __grid_constant__ phk_wake_set w) {
+    namespace cg = cooperative_groups;
+    __shared__ int2 s_tab[kConvWarps][kConvWindow + 1];
+    __shared__ int2 s_mom[kConvWarps][kConvSources];
+    __shared__ double s_acc[kConvWarps][kConvTargets];
+    __shared__ double s_sum[kConvTargets];
+    cg::cluster_group cl = cg::this_cluster();
+    const unsigned rank = cl.block_rank();
+    const int S = w.n_slices;
+    const int blocks = (S + kConvTargets - 1) / kConvTargets;
+    const int job = blockIdx.x / kConvCluster;
+    const int k = job / blocks, i0 = (job - k * blocks) * kConvTargets;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const phk_wake_kick& kk = w.kick[k];
+    const bool work = k < w.n_kicks && !kk.dense;
+    const int L2 = 2 * S - 1;
+    // as many sources a unit as leave every warp of the cluster one
+    const int most = kk.n_lags * S / (kConvWarps * kConvCluster);
+    const int per = most < 16 ? 16 : (most > kConvSources ? kConvSources : most);
+    const int chunks = (S + per - 1) / per;
+    const int units = work ? kk.n_lags * chunks : 0;
+    double acc = 0.0;
+    for (int u = warp * kConvCluster + rank; u < units; u += kConvWarps * kConvCluster) {
+        const int a = u / chunks, j0 = (u - a * chunks) * per;
+        const int len = min(per, S - j0);
+        if (len <= 0) continue;
+        const int slot = ((w.head - a) % w.ring_len + w.ring_len) % w.ring_len;
+        const double* m = w.moments + ((int64_t)slot * 3 + kk.source) * S + j0;
+        // target i, source j0 + j: table entry i + S - 1 - j0 - j; window
+        // entry t holds table entry base + t
+        const double* row = kk.table + (int64_t)a * L2;
+        const int base = i0 + S - j0 - len;
+        const int n_tab = min(len + kConvTargets - 1, L2 - base);
+        constexpr int NT = (kConvWindow + 31) / 32, NM = kConvSources / 32;
+        double tv[NT], mv[NM];
+#pragma unroll
+        for (int q = 0; q < NT; ++q) {
+            const int t = lane + 32 * q;
+            tv[q] = t < n_tab ? __ldg(row + base + t) : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < NM; ++q) {
+            const int j = lane + 32 * q;
+            mv[q] = j < len ? __ldg(m + j) : 0.0;
+        }
+        unsigned bt = 0u, bm = 0u;
+#pragma unroll
+        for (int q = 0; q < NT; ++q)
+            bt = max(bt, (unsigned)__double2hiint(tv[q]) & 0x7fffffffu);
+#pragma unroll
+        for (int q = 0; q < NM; ++q)
+            bm = max(bm, (unsigned)__double2hiint(mv[q]) & 0x7fffffffu);
+        const int et = (int)(__reduce_max_sync(0xffffffffu, bt) >> 20);
+        const int em = (int)(__reduce_max_sync(0xffffffffu, bm) >> 20);
+        const bool normal = et >= 100 && et < 2000 && em >= 100 && em < 2000 &&
+                            et + em > 1100 && et + em < 3100;
+        if (!normal) {
+            conv_unit_fp64(m, row + S - 1 - j0, len, i0 + lane, S, acc);
+            continue;
+        }
+        __syncwarp();                  // the previous unit's limbs are read
+#pragma unroll
+        for (int q = 0; q < NT; ++q)
+            if (lane + 32 * q < kConvWindow)
+                s_tab[warp][lane + 32 * q] = conv_limbs(tv[q], et);
+#pragma unroll
+        for (int q = 0; q < NM; ++q) s_mom[warp][lane + 32 * q] = conv_limbs(mv[q], em);
+        __syncwarp();
+        long long hh = 0, mid = 0, mil = 0, ll = 0;
+        const int2* tp = &s_tab[warp][lane + len - 1];
+        const int2* mp = s_mom[warp];
+#pragma unroll 8
+        for (int j = 0; j < len; ++j) {
+            const int2 f = mp[j], t = tp[-j];
+            hh += (long long)f.y * t.y;
+            mid += (long long)f.y * t.x;
+            mil += (long long)f.x * t.y;
+            ll += (long long)f.x * t.x;
+        }
+        // sum = hh 2^54 + mid 2^27 + ll in units of 2^(et + em - 2152); in
+        // units of 2^53 of these it fits 63 bits: one rounding
+        const double unit = __hiloint2double((et + em - 1076) << 20, 0);
+        acc = fma((double)((hh << 1) + ((mid + mil + (ll >> 27)) >> 26)), unit, acc);
+    }
+    s_acc[warp][lane] = acc;
+    __syncthreads();
+    if (threadIdx.x < kConvTargets) {
+        double sum = s_acc[0][threadIdx.x];
+        for (int q = 1; q < kConvWarps; ++q) sum += s_acc[q][threadIdx.x];
+        s_sum[threadIdx.x] = sum;
+    }
+    cl.sync();
+    if (rank == 0 && threadIdx.x < kConvTargets && work) {
+        const int i = i0 + threadIdx.x;
+        double sum = s_sum[threadIdx.x];
+        for (int r = 1; r < kConvCluster; ++r)
+            sum += cl.map_shared_rank(s_sum, r)[threadIdx.x];
+        if (i < S) {
+            const double r = mul(kk.factor, sum);
+            if (w.out_dtype == PHK_F64)
+                reinterpret_cast<double*>(kk.out)[i] = r;
+            else
+                reinterpret_cast<float*>(kk.out)[i] = (float)r;
+        }
+    }
+    cl.sync();                         // sums stay until rank 0 has read them
 }
 
 __global__ void wake_dense_kernel(const __grid_constant__ phk_wake_set w) {
@@ -406,7 +556,20 @@ int launch_wake(const phk_wake_set* w, cudaStream_t st) {
     }
     const int S = w->n_slices;
     if (any_conv)
-        wake_conv_kernel<<<w->n_kicks * S, kConvWarps * 32, 0, st>>>(*w);
+    {
+        // multiply-adds of the launch: below a million, the direct kernel's
+        // short chains win (50 slices, one turn: 4.4 against 6.4 us; 200
+        // slices: 5.6 / 6.4), above, the FP64 work does (1000 slices, 10
+        // turns: 66 / 21 us)
+        int64_t macs = 0;
+        for (int k = 0; k < w->n_kicks; ++k)
+            if (!w->kick[k].dense) macs += (int64_t)w->kick[k].n_lags * S * S;
+        if (macs < (1 << 20))
+            wake_direct_kernel<<<w->n_kicks * S, kDirectWarps * 32, 0, st>>>(*w);
+        else
+            wake_conv_kernel<<<w->n_kicks * ((S + kConvTargets - 1) / kConvTargets) *
+                                   kConvCluster, kConvWarps * 32, 0, st>>>(*w);
+    }
     if (any_dense) {
         const int n = w->n_kicks * S;
         wake_dense_kernel<<<(n + 127) / 128, 128, 0, st>>>(*w);
