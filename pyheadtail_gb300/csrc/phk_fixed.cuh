@@ -29,6 +29,62 @@ __device__ __forceinline__ u64 shr_clamp(u64 v, int r) {
 }
 
 // -------------------------------------------------------------------
+// FP64 product on the integer pipes, correctly rounded (to nearest, ties to
+// even): the same bits as __dmul_rn for normal operands and a normal result.
+// A factor is its left-aligned significand and its sign and exponent bits.
+// About 26 integer instructions.
+// -------------------------------------------------------------------
+struct Factor {
+    unsigned hi, lo;    // significand, top bit set
+    int e;              // sign and exponent bits of the high word
+};
+__host__ __device__ inline Factor factor_bits(unsigned hi, unsigned lo) {
+    return Factor{0x80000000u | (hi << 11) | (lo >> 21), lo << 11,
+                  (int)(hi & 0xfff00000u)};
+}
+__device__ __forceinline__ Factor factor_of(double v) {
+    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+    return Factor{__funnelshift_l(lo, hi, 11) | 0x80000000u, lo << 11,
+                  (int)(hi & 0xfff00000u)};
+}
+// magnitude outside [2^-256, 2^256) (zeros, subnormals, infinities and NaN
+// among them): one of the top three bits of the result
+__device__ __forceinline__ unsigned off_centre(double v) {
+    return ((unsigned)__double2hiint(v) & 0x7fffffffu) - (767u << 20);
+}
+constexpr unsigned kOffCentre = 0xe0000000u;
+// magnitude in [2^-511, 2^512): bit 30 of the result (zeros, subnormals,
+// infinities and NaN clear it)
+__device__ __forceinline__ unsigned mid_range(double v) {
+    return (unsigned)__double2hiint(v) + 0x20000000u;
+}
+
+__device__ __forceinline__ double mul_int(const Factor& a, const Factor& b) {
+    const u64 p0 = (u64)a.lo * b.lo;
+    const u64 p1 = (u64)a.hi * b.lo + (p0 >> 32);
+    const u64 p2 = (u64)a.lo * b.hi + (unsigned)p1;
+    const u64 p3 = (u64)a.hi * b.hi + (p1 >> 32) + (p2 >> 32);
+    const unsigned h = (unsigned)(p3 >> 32), l = (unsigned)p3;
+    // 53 bits of the product, the rest and whether anything is below it
+    const int top = (int)(h >> 31), s = 10 + top;
+    unsigned ml = __funnelshift_r(l, h, s), mh = h >> s;
+    const unsigned rest = (l << (32 - s)) | (((unsigned)p0 | (unsigned)p2) != 0u ? 1u : 0u);
+    const unsigned up = rest + (ml & 1u) > 0x80000000u ? 1u : 0u;
+    ml += up;
+    mh += ml < up ? 1u : 0u;
+    return __hiloint2double((int)mh + a.e + b.e + (top << 20) - (1024 << 20), (int)ml);
+}
+
+// the product as a factor again, 63 bits and more of it (truncated)
+__device__ __forceinline__ Factor mul_factor(const Factor& a, const Factor& b) {
+    u64 p = __umul64hi(((u64)a.hi << 32) | a.lo, ((u64)b.hi << 32) | b.lo);
+    const int top = (int)(p >> 63);
+    p <<= 1 - top;
+    return Factor{(unsigned)(p >> 32), (unsigned)p,
+                  a.e + b.e + (top << 20) - (1023 << 20)};
+}
+
+// -------------------------------------------------------------------
 // FixHist64: per-slice sums of FP64 coordinates as 64-bit fixed-point
 // integers, the FP64 counterpart of FixHist (phk_track.cuh).
 //
@@ -165,8 +221,27 @@ __device__ __forceinline__ SineParts sine_parts(const u64* tab, u64 u) {
     return p;
 }
 
-// sine, units of 2^-62
-__device__ __forceinline__ long long sine_turn(const u64* tab, u64 F) {
+// m 2^-62 with the given sign bit as a double, rounded to nearest (integer
+// work: a conversion takes the FP64 pipe 16 cycles); 0 for m = 0
+__device__ __forceinline__ double unit_double(u64 m, unsigned sign) {
+    const int lz = __clzll((long long)m);
+    const u64 f = m << lz;                       // top bit set
+    const u64 r = (f >> 11) + ((f >> 10) & 1ull);
+    const unsigned e = (unsigned)(1023 - lz) << 20;   // the top bit of r adds one
+    const double v = __hiloint2double((int)((unsigned)(r >> 32) + e | sign), (int)r);
+    return m ? v : 0.0;
+}
+
+// the same as a factor with 64 significant bits (m = 0: as 2^-62)
+__device__ __forceinline__ Factor unit_factor(u64 m, unsigned sign) {
+    m = m ? m : 1ull;
+    const int lz = __clzll((long long)m);
+    const u64 f = m << lz;
+    return Factor{(unsigned)(f >> 32), (unsigned)f, (int)(((1024 - lz) << 20) | sign)};
+}
+
+// sine, times 2^62, as magnitude and sign bit
+__device__ __forceinline__ u64 sine_turn(const u64* tab, u64 F, unsigned* sign) {
     // the second and third quarters mirror about a quarter turn
     const unsigned fh = (unsigned)(F >> 32);
     if ((fh ^ (fh << 1)) & 0x80000000u) F = 0x8000000000000000ull - F;
@@ -175,32 +250,28 @@ __device__ __forceinline__ long long sine_turn(const u64* tab, u64 F) {
     const long long d = (long long)(__umul64hi(p.c, p.th) -
                                     (__umul64hi(p.s, p.q) >> 9));   // 2^-71
     const long long r = (long long)p.s + ((d + 256) >> 9);
-    return neg ? -r : r;
+    *sign = neg ? 0x80000000u : 0u;
+    return (u64)(r < 0 ? 0 : r);
 }
 
-// sine and cosine, times 2^62, as doubles
-__device__ __forceinline__ void sincos_turn(const u64* tab, u64 F, double* s,
-                                            double* c) {
+// sine and cosine, times 2^62, as magnitudes and sign bits
+struct SinCos {
+    u64 s, c;
+    unsigned ns, nc;
+};
+__device__ __forceinline__ SinCos sincos_turn(const u64* tab, u64 F) {
     const SineParts p = sine_parts(tab, F & 0x3fffffffffffffffull);
     const long long d1 = (long long)(__umul64hi(p.c, p.th) -
                                      (__umul64hi(p.s, p.q) >> 9));   // 2^-71
     const long long d2 = (long long)(__umul64hi(p.s, p.th) +
                                      (__umul64hi(p.c, p.q) >> 9));
-    const double sn = (double)((long long)p.s + ((d1 + 256) >> 9));
-    const double cs = (double)((long long)p.c - ((d2 + 256) >> 9));
+    const long long a = (long long)p.s + ((d1 + 256) >> 9);
+    const long long b = (long long)p.c - ((d2 + 256) >> 9);
+    const u64 sn = (u64)(a < 0 ? 0 : a), cs = (u64)(b < 0 ? 0 : b);
     // quadrants: (sn, cs), (cs, -sn), (-sn, -cs), (-cs, sn)
     const unsigned k = (unsigned)(F >> 62);
-    const double a = (k & 1u) ? cs : sn, b = (k & 1u) ? sn : cs;
-    const int na = (int)((k & 2u) << 30), nb = (int)(((k + 1u) & 2u) << 30);
-    *s = __hiloint2double(__double2hiint(a) ^ na, __double2loint(a));
-    *c = __hiloint2double(__double2hiint(b) ^ nb, __double2loint(b));
-}
-
-// v 2^-62 for |v| >= 1 or v = 0 (integer work only)
-__device__ __forceinline__ double unscale62(double v) {
-    const int hi = __double2hiint(v);
-    return __hiloint2double((hi & 0x7fffffff) ? hi - (62 << 20) : hi,
-                            __double2loint(v));
+    return SinCos{(k & 1u) ? cs : sn, (k & 1u) ? sn : cs, (k & 2u) << 30,
+                  ((k + 1u) & 2u) << 30};
 }
 
 // t turns (|t| < 2^31) as a fraction of a turn, truncated toward zero

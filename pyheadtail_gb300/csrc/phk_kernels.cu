@@ -42,7 +42,7 @@ int track_grid(int64_t n, int32_t dtype, int32_t n_slices) {
     // size for an accumulation with a pending kick on the same slicing (the
     // largest shared-memory layout of a turn)
     const size_t smem = track_smem_bytes(dtype, n_slices, n_slices);
-    const int vec = dtype == PHK_F64 ? 2 : kF32Vec;
+    const int vec = dtype == PHK_F64 ? 1 : kF32Vec;
     const int nc = dtype == PHK_F64 ? track_clusters_f64(smem)
                                     : track_clusters_f32(smem);
     const int64_t tiles = (n + (int64_t)kTrackThreads * vec - 1) /

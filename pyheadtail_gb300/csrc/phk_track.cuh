@@ -51,13 +51,28 @@ struct OpFix {
     double c[5];     // RF kick: (A / p0_new) 2^-62, p0_old / p0_new,
                      //   dp_inc / p0_new, h 2 pi / C, offset in radians
                      // drift: eta0 L
-                     // detuned transverse: J01 J10 J23 J32, times 2^-62
+    Factor m[8];     // transverse: the matrix entries; detuned, J01 J10 J23 J32
+    int32_t m_ok;    //   all within range
 };
-// amplitude detuning: with j = g u^2 + t u u' + u'^2
+// amplitude detuning: with j = g u^2 + t u u' + b u'^2 (twice the action)
 struct DetFix {
-    double gx, tx, gy, ty;
+    double gx, tx, bx, gy, ty, by;
     double axx, axy, ayy, ayx;   // dQ_x = axx j_x + axy j_y, dQ_y likewise
+    // factors of the products on the integer pipes: amplitude detuning gx,
+    // gy, bx, by, axy, ayx; chromaticity of order one its two coefficients
+    Factor m[6];
+    int32_t m_ok;                // all within range
 };
+
+// v as a factor; false outside [2^-200, 2^200]
+__host__ __device__ inline bool host_factor(double v, Factor* f) {
+    u64 bits;
+    memcpy(&bits, &v, sizeof(bits));
+    *f = factor_bits((unsigned)(bits >> 32), (unsigned)bits);
+    const int e = (int)(bits >> 52) & 0x7ff;
+    return e > 1023 - 200 && e < 1023 + 200;
+}
+
 struct Aux64 {
     const u64* sine;     // staged quarter wave (stage_sine)
     const OpFix* op;     // by op
@@ -69,11 +84,12 @@ __host__ __device__ inline void op_fix(const phk_op& op, OpFix* r) {
     const int f = op.flags;
     if (op.kind == PHK_OP_DRIFT) {
         r->c[0] = p[1] * p[2];
+    } else if (op.kind == PHK_OP_TRANSVERSE && !(f & PHK_FLAG_DETUNED)) {
+        r->m_ok = 1;
+        for (int i = 0; i < 8; ++i) r->m_ok &= host_factor(p[i], r->m + i);
     } else if (op.kind == PHK_OP_TRANSVERSE) {
-        r->c[0] = p[9] * 0x1p-62;
-        r->c[1] = p[10] * 0x1p-62;
-        r->c[2] = p[13] * 0x1p-62;
-        r->c[3] = p[14] * 0x1p-62;
+        r->m_ok = host_factor(p[9], r->m) & host_factor(p[10], r->m + 1) &
+                  host_factor(p[13], r->m + 2) & host_factor(p[14], r->m + 3);
     } else if (op.kind == PHK_OP_RF_KICK) {
         double off = 0.0;
         if (f & PHK_FLAG_PHI_OFFSET) off += p[3];
@@ -91,14 +107,24 @@ __host__ __device__ inline void op_fix(const phk_op& op, OpFix* r) {
 
 __host__ __device__ inline void det_fix(const phk_detuner& d, DetFix* f) {
     const double* c = d.c;
-    f->gx = c[4] / c[6];
-    f->tx = c[5] / c[6];
-    f->gy = c[7] / c[9];
-    f->ty = c[8] / c[9];
-    f->axx = 0.5 * c[0] * c[6] / c[10];
-    f->axy = 0.5 * c[2] * c[9] / c[10];
-    f->ayy = 0.5 * c[1] * c[9] / c[10];
-    f->ayx = 0.5 * c[3] * c[6] / c[10];
+    if (d.kind == PHK_DET_CHROMA) {
+        f->m_ok = d.nx == 1 && d.ny == 1 && d.zx == 0 && d.zy == 0 &&
+                  host_factor(c[0], f->m) & host_factor(c[8], f->m + 1);
+        return;
+    }
+    f->gx = c[4];
+    f->tx = c[5];
+    f->bx = c[6];
+    f->gy = c[7];
+    f->ty = c[8];
+    f->by = c[9];
+    f->axx = 0.5 * c[0] / c[10];
+    f->axy = 0.5 * c[2] / c[10];
+    f->ayy = 0.5 * c[1] / c[10];
+    f->ayx = 0.5 * c[3] / c[10];
+    f->m_ok = host_factor(f->gx, f->m) & host_factor(f->gy, f->m + 1) &
+              host_factor(f->bx, f->m + 2) & host_factor(f->by, f->m + 3) &
+              host_factor(f->axy, f->m + 4) & host_factor(f->ayx, f->m + 5);
 }
 
 // whether a program needs the quarter wave
@@ -144,42 +170,116 @@ __device__ __forceinline__ double chroma_poly(const double* c, int n, int z,
     return r;
 }
 
-// phases of 2^12 radians and more, NaN and infinities: sine and cosine
-// times 2^62
+// whether the fixed-point phase takes phi radians (below 2^12, finite)
+__device__ __forceinline__ bool phase_near(double phi) {
+    return biased_exp(__double2hiint(phi)) < 1035;
+}
+// sine and cosine of phi radians: phi / 2 pi as a fraction of a turn
+// (1 / 2 pi = 0xa2f9... 2^-66)
+__device__ __forceinline__ SinCos phase_sincos(const u64* tab, double phi) {
+    return sincos_turn(tab, turn_product(phi, 0xa2f9836e4e44152aull, 66));
+}
 static __device__ __noinline__ void sincos_far(double phi, double* s, double* c) {
     sincos(phi, s, c);
-    *s *= 0x1p62;
-    *c *= 0x1p62;
 }
 
-// sine and cosine, times 2^62, of phi radians: phi / 2 pi as a fraction of a
-// turn (1 / 2 pi = 0xa2f9... 2^-66)
-__device__ __forceinline__ void phase_sincos(const u64* tab, double phi, double* s,
-                                             double* c) {
-    if (biased_exp(__double2hiint(phi)) < 1035)
-        sincos_turn(tab, turn_product(phi, 0xa2f9836e4e44152aull, 66), s, c);
-    else
-        sincos_far(phi, s, c);
-}
-
-// (u, u') through one plane's detuned map, sine and cosine times 2^62
+// (u, u') through one plane's detuned map
 __device__ __forceinline__ void detuned_plane(const double* I, const double* J,
-                                              double s, double c, double& u,
+                                              const u64* tab, double phi, double& u,
                                               double& up) {
-    const double s1 = unscale62(s), c1 = unscale62(c);
-    const double M00 = fma(I[0], c1, J[0] * s1), M01 = fma(I[1], c1, J[1] * s1);
-    const double M10 = fma(I[2], c1, J[2] * s1), M11 = fma(I[3], c1, J[3] * s1);
+    double s, c;
+    if (phase_near(phi)) {
+        const SinCos r = phase_sincos(tab, phi);
+        s = unit_double(r.s, r.ns);
+        c = unit_double(r.c, r.nc);
+    } else {
+        sincos_far(phi, &s, &c);
+    }
+    const double M00 = fma(I[0], c, J[0] * s), M01 = fma(I[1], c, J[1] * s);
+    const double M10 = fma(I[2], c, J[2] * s), M11 = fma(I[3], c, J[3] * s);
     const double nu = fma(M00, u, M01 * up);
     up = fma(M10, u, M11 * up);
     u = nu;
 }
-// the same with unit I and J without diagonal (j01, j10 times 2^-62)
-__device__ __forceinline__ void detuned_plane_unit(double j01, double j10, double s,
-                                                   double c, double& u, double& up) {
-    const double c1 = unscale62(c);
-    const double nu = fma(c1, u, (j01 * s) * up);
-    up = fma(c1, up, (j10 * s) * u);
+// the same with unit I and J without diagonal, the products with the sine on
+// the integer pipes: of u' and u, first the 64-bit product J s
+__device__ __forceinline__ void detuned_plane_unit(const Factor* J, const SinCos& r,
+                                                   const Factor& fu, const Factor& fup,
+                                                   double& u, double& up) {
+    const Factor s = unit_factor(r.s, r.ns);
+    const double c = unit_double(r.c, r.nc);
+    const double nu = fma(c, u, mul_int(mul_factor(J[0], s), fup));
+    up = fma(c, up, mul_int(mul_factor(J[1], s), fu));
     u = nu;
+}
+
+// the tune with its detunings, each added as the reference adds them
+__device__ __forceinline__ void detuned_tunes(const phk_op& op, const phk_program& prog,
+                                              const Aux64& aux, bool cross, double x,
+                                              double xp, double y, double yp, double dp,
+                                              double& qx, double& qy) {
+    qx = op.p[20];
+    qy = op.p[21];
+    for (int d = 0; d < op.det_count; ++d) {
+        const phk_detuner& dt = prog.det[op.det_begin + d];
+        if (dt.kind == PHK_DET_CHROMA) {
+            qx = add(qx, chroma_poly(dt.c, dt.nx, dt.zx, dp));
+            qy = add(qy, chroma_poly(dt.c + 8, dt.ny, dt.zy, dp));
+        } else {
+            const DetFix& f = aux.det[op.det_begin + d];
+            double jx = f.gx * x, jy = f.gy * y;
+            if (cross) {
+                jx = fma(f.tx, xp, jx);
+                jy = fma(f.ty, yp, jy);
+            }
+            jx = fma(jx, x, f.bx * xp * xp);
+            jy = fma(jy, y, f.by * yp * yp);
+            qx = add(qx, fma(f.axx, jx, f.axy * jy));
+            qy = add(qy, fma(f.ayy, jy, f.ayx * jx));
+        }
+    }
+}
+
+// the detuned map of one particle u = (x, xp, y, yp, dp), all FP64
+__device__ __forceinline__ void detuned_map(const phk_op& op, const phk_program& prog,
+                                            const Aux64& aux, double& x, double& xp,
+                                            double& y, double& yp, double qx, double qy) {
+    const double* p = op.p;
+    detuned_plane(p, p + 8, aux.sine, mul(qx, p[22]), x, xp);
+    detuned_plane(p + 4, p + 12, aux.sine, mul(qy, p[22]), y, yp);
+}
+// out of line: particles with a zero, subnormal, huge or non-finite coordinate
+// or a phase beyond the fixed point
+static __device__ __noinline__ void detuned_map_cold(const phk_op& op,
+                                                     const phk_program& prog,
+                                                     const Aux64& aux, double* u) {
+    double qx, qy;
+    detuned_tunes(op, prog, aux, false, u[0], u[1], u[2], u[3], u[4], qx, qy);
+    detuned_map(op, prog, aux, u[0], u[1], u[2], u[3], qx, qy);
+}
+
+// whether the products of a detuned segment's constants run on the integer
+// pipes
+__device__ __forceinline__ bool detuned_factors_ok(const phk_op& op, const Aux64& aux,
+                                                   int o) {
+    int ok = aux.op[o].m_ok;
+    for (int d = 0; d < op.det_count; ++d) ok &= aux.det[op.det_begin + d].m_ok;
+    return ok;
+}
+
+// the undetuned map, every product and sum rounded separately in the
+// reference's order
+__device__ __forceinline__ void linear_planes(const double* p, double& x, double& xp,
+                                              double& y, double& yp) {
+    const double nx = add(mul(p[0], x), mul(p[1], xp));
+    const double nxp = add(mul(p[2], x), mul(p[3], xp));
+    const double ny = add(mul(p[4], y), mul(p[5], yp));
+    const double nyp = add(mul(p[6], y), mul(p[7], yp));
+    x = nx; xp = nxp; y = ny; yp = nyp;
+}
+// out of line: particles with a zero, subnormal, huge or non-finite coordinate
+static __device__ __noinline__ void linear_planes_cold(const double* p, double* u) {
+    linear_planes(p, u[0], u[1], u[2], u[3]);
 }
 
 // TransverseSegmentMap.track, plain form.  Without detuners every product
@@ -192,7 +292,8 @@ __device__ __forceinline__ void detuned_plane_unit(double j01, double j10, doubl
 // particle, conversions included; before, about 110 and as many again in
 // warps with a lane beyond the quarter radian of the former series (a turn
 // of 1e6 macroparticles: 395 -> 122 us).
-template <int VEC, bool PLAIN>
+// DET (PLAIN): whether the segment is detuned
+template <int VEC, bool PLAIN, bool DET = false>
 __device__ __forceinline__ void op_transverse(const phk_op& op, int o,
                                               const phk_program& prog,
                                               const Aux64& aux,
@@ -205,37 +306,62 @@ __device__ __forceinline__ void op_transverse(const phk_op& op, int o,
     double (&y)[VEC] = t.c[PHK_Y];
     double (&yp)[VEC] = t.c[PHK_YP];
     const double (&dp)[VEC] = t.c[PHK_DP];
-    // the detuning sees the coordinates before the dispersion is taken out
-    double phx[VEC], phy[VEC];
-    const bool detuned = op.flags & PHK_FLAG_DETUNED;
-    if (detuned) {
+    if constexpr (PLAIN && DET) {
+        // FP64 keeps the additions, the multiply-adds and the phase's product
+        // (18 a particle of the segment's 36); products run on the integer
+        // pipes
+        const OpFix& f = aux.op[o];
+        const unsigned off = detuned_factors_ok(op, aux, o) ? 0u : kOffCentre;
 #pragma unroll
-        for (int j = 0; j < VEC; ++j) { phx[j] = p[20]; phy[j] = p[21]; }
-        for (int d = 0; d < op.det_count; ++d) {
-            const phk_detuner& dt = prog.det[op.det_begin + d];
-            if (dt.kind == PHK_DET_CHROMA) {
-#pragma unroll
-                for (int j = 0; j < VEC; ++j) {
-                    phx[j] = add(phx[j], chroma_poly(dt.c, dt.nx, dt.zx, dp[j]));
-                    phy[j] = add(phy[j], chroma_poly(dt.c + 8, dt.ny, dt.zy, dp[j]));
-                }
-            } else {
-                const DetFix& f = aux.det[op.det_begin + d];
-#pragma unroll
-                for (int j = 0; j < VEC; ++j) {
-                    double jx = f.gx * x[j], jy = f.gy * y[j];
-                    if (!PLAIN) {
-                        jx = fma(f.tx, xp[j], jx);
-                        jy = fma(f.ty, yp[j], jy);
+        for (int j = 0; j < VEC; ++j) {
+            bool cold = ((off_centre(x[j]) | off_centre(xp[j]) | off_centre(y[j]) |
+                          off_centre(yp[j]) | off_centre(dp[j]) | off) & kOffCentre) != 0u;
+            if (!cold) {
+                const Factor u = factor_of(x[j]), up = factor_of(xp[j]);
+                const Factor v = factor_of(y[j]), vp = factor_of(yp[j]);
+                double qx = p[20], qy = p[21];
+                for (int d = 0; d < op.det_count; ++d) {
+                    const phk_detuner& dt = prog.det[op.det_begin + d];
+                    const DetFix& g = aux.det[op.det_begin + d];
+                    if (dt.kind == PHK_DET_CHROMA) {
+                        const Factor w = factor_of(dp[j]);
+                        qx = add(qx, mul_int(g.m[0], w));
+                        qy = add(qy, mul_int(g.m[1], w));
+                    } else {
+                        const double jx = add(mul_int(mul_factor(g.m[0], u), u),
+                                              mul_int(mul_factor(g.m[2], up), up));
+                        const double jy = add(mul_int(mul_factor(g.m[1], v), v),
+                                              mul_int(mul_factor(g.m[3], vp), vp));
+                        qx = add(qx, fma(g.axx, jx, mul_int(g.m[4], factor_of(jy))));
+                        qy = add(qy, fma(g.ayy, jy, mul_int(g.m[5], factor_of(jx))));
                     }
-                    jx = fma(jx, x[j], xp[j] * xp[j]);
-                    jy = fma(jy, y[j], yp[j] * yp[j]);
-                    phx[j] = add(phx[j], fma(f.axx, jx, f.axy * jy));
-                    phy[j] = add(phy[j], fma(f.ayy, jy, f.ayx * jx));
+                }
+                const double phx = mul(qx, p[22]), phy = mul(qy, p[22]);
+                if (phase_near(phx) && phase_near(phy)) {
+                    detuned_plane_unit(f.m, phase_sincos(aux.sine, phx), u, up, x[j],
+                                       xp[j]);
+                    detuned_plane_unit(f.m + 2, phase_sincos(aux.sine, phy), v, vp, y[j],
+                                       yp[j]);
+                } else {
+                    cold = true;
                 }
             }
+            if (cold) {
+                double c[5] = {x[j], xp[j], y[j], yp[j], dp[j]};
+                detuned_map_cold(op, prog, aux, c);
+                x[j] = c[0]; xp[j] = c[1]; y[j] = c[2]; yp[j] = c[3];
+            }
         }
+        return;
     }
+    // the detuning sees the coordinates before the dispersion is taken out
+    const bool detuned = !PLAIN && (op.flags & PHK_FLAG_DETUNED);
+    double qx[VEC], qy[VEC];
+    if (detuned)
+#pragma unroll
+        for (int j = 0; j < VEC; ++j)
+            detuned_tunes(op, prog, aux, true, x[j], xp[j], y[j], yp[j], dp[j], qx[j],
+                          qy[j]);
     if (disp) {
 #pragma unroll
         for (int j = 0; j < VEC; ++j) {
@@ -244,28 +370,33 @@ __device__ __forceinline__ void op_transverse(const phk_op& op, int o,
         }
     }
     if (detuned) {
-        const double* f = aux.op[o].c;
+#pragma unroll
+        for (int j = 0; j < VEC; ++j)
+            detuned_map(op, prog, aux, x[j], xp[j], y[j], yp[j], qx[j], qy[j]);
+    } else if (PLAIN) {
+        // the products on the integer pipes, the same bits (mul_int): eight
+        // of the twelve FP64 instructions, which are what bounds the pass
+        const OpFix& f = aux.op[o];
+        const unsigned ok = f.m_ok ? 0x40000000u : 0u;
 #pragma unroll
         for (int j = 0; j < VEC; ++j) {
-            double s, c;
-            phase_sincos(aux.sine, mul(phx[j], p[22]), &s, &c);
-            if (PLAIN) detuned_plane_unit(f[0], f[1], s, c, x[j], xp[j]);
-            else detuned_plane(p, p + 8, s, c, x[j], xp[j]);
-            phase_sincos(aux.sine, mul(phy[j], p[22]), &s, &c);
-            if (PLAIN) detuned_plane_unit(f[2], f[3], s, c, y[j], yp[j]);
-            else detuned_plane(p + 4, p + 12, s, c, y[j], yp[j]);
+            if (mid_range(x[j]) & mid_range(xp[j]) & mid_range(y[j]) &
+                mid_range(yp[j]) & ok) {
+                const Factor u = factor_of(x[j]), up = factor_of(xp[j]);
+                const Factor v = factor_of(y[j]), vp = factor_of(yp[j]);
+                x[j] = add(mul_int(f.m[0], u), mul_int(f.m[1], up));
+                xp[j] = add(mul_int(f.m[2], u), mul_int(f.m[3], up));
+                y[j] = add(mul_int(f.m[4], v), mul_int(f.m[5], vp));
+                yp[j] = add(mul_int(f.m[6], v), mul_int(f.m[7], vp));
+            } else {
+                double c[4] = {x[j], xp[j], y[j], yp[j]};
+                linear_planes_cold(p, c);
+                x[j] = c[0]; xp[j] = c[1]; y[j] = c[2]; yp[j] = c[3];
+            }
         }
     } else {
-        const double M00 = p[0], M01 = p[1], M10 = p[2], M11 = p[3];
-        const double M22 = p[4], M23 = p[5], M32 = p[6], M33 = p[7];
 #pragma unroll
-        for (int j = 0; j < VEC; ++j) {
-            const double nx = add(mul(M00, x[j]), mul(M01, xp[j]));
-            const double nxp = add(mul(M10, x[j]), mul(M11, xp[j]));
-            const double ny = add(mul(M22, y[j]), mul(M23, yp[j]));
-            const double nyp = add(mul(M32, y[j]), mul(M33, yp[j]));
-            x[j] = nx; xp[j] = nxp; y[j] = ny; yp[j] = nyp;
-        }
+        for (int j = 0; j < VEC; ++j) linear_planes(p, x[j], xp[j], y[j], yp[j]);
     }
     if (disp) {
 #pragma unroll
@@ -326,10 +457,15 @@ __device__ __forceinline__ void op_rfkick(const phk_op& op, const OpFix& f,
         }
         const double z = t.c[PHK_Z][j];
         double s;      // sine, times 2^62
-        if (biased_exp(__double2hiint(z)) <= 968 + f.k.exp)
-            s = (double)sine_turn(sine, turn_product(z, f.k.mant, f.k.exp) + f.off);
-        else
+        if (biased_exp(__double2hiint(z)) <= 968 + f.k.exp) {
+            unsigned sign;
+            const u64 m = sine_turn(sine, turn_product(z, f.k.mant, f.k.exp) + f.off, &sign);
+            s = (double)(long long)m;
+            s = __hiloint2double((int)((unsigned)__double2hiint(s) | sign),
+                                 __double2loint(s));
+        } else {
             s = rf_sine_far(z, f.c[3], f.c[4]);
+        }
         if (PLAIN) dp = fma(f.c[0], s, dp);
         else dp = fma(dp, f.c[1], fma(f.c[0], s, -f.c[2]));
         if (disp) {
@@ -840,6 +976,11 @@ enum TrackShape {
     SHAPE_T = 2,         // one transverse segment
     SHAPE_T_RF = 3,      // transverse, drift, RF kick, drift (RFSystems)
     SHAPE_T_LIN = 4,     // transverse, linear longitudinal map
+    // FP64 form: the same with a detuned transverse segment
+    SHAPE_DETUNED = 8,   // flag
+    SHAPE_DT = SHAPE_T | SHAPE_DETUNED,
+    SHAPE_DT_RF = SHAPE_T_RF | SHAPE_DETUNED,
+    SHAPE_DT_LIN = SHAPE_T_LIN | SHAPE_DETUNED,
 };
 
 template <typename T, int VEC, int SHAPE>
@@ -849,12 +990,13 @@ __device__ __forceinline__ void run_program_shape(const phk_program& prog,
     if constexpr (SHAPE == SHAPE_GENERIC) {
         run_program<T, VEC>(prog, aux, t);
     } else if constexpr (SHAPE != SHAPE_NONE && std::is_same<T, double>::value) {
-        op_transverse<VEC, true>(prog.op[0], 0, prog, aux, t);
-        if constexpr (SHAPE == SHAPE_T_RF) {
+        constexpr bool DET = (SHAPE & SHAPE_DETUNED) != 0;
+        op_transverse<VEC, true, DET>(prog.op[0], 0, prog, aux, t);
+        if constexpr ((SHAPE & ~SHAPE_DETUNED) == SHAPE_T_RF) {
             op_drift_rf<VEC>(aux.op[1], t);
             op_rfkick<VEC, true>(prog.op[2], aux.op[2], aux.sine, t);
             op_drift_rf<VEC>(aux.op[3], t);
-        } else if constexpr (SHAPE == SHAPE_T_LIN) {
+        } else if constexpr ((SHAPE & ~SHAPE_DETUNED) == SHAPE_T_LIN) {
             op_linear_long<VEC, true>(prog.op[1], t);
         }
     } else if constexpr (SHAPE != SHAPE_NONE) {
@@ -2273,7 +2415,7 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
             if constexpr (F64) {
                 const phk_program& bp = b.programs[U.bunch];
                 if (tid < PHK_MAX_OPS) op_fix(bp.op[tid], s_op + tid);
-                if (tid < PHK_MAX_DETUNERS && bp.det[tid].kind == PHK_DET_AMPLITUDE)
+                if (tid < PHK_MAX_DETUNERS && tid < bp.n_det)
                     det_fix(bp.det[tid], s_det + tid);
             }
             if (a.has_pk) {
@@ -2437,6 +2579,13 @@ static inline void track_masks(const phk_program* prog, const phk_kick_set* pk,
 
 // ---- per-precision entry points (phk_track_f32.cu / phk_track_f64.cu)
 int program_shape(const phk_program* prog);
+// the FP64 form's: GENERIC unless PLAIN, with the detuned flag
+static inline int program_shape64(const phk_program* prog) {
+    const int s = program_plain64(*prog) ? program_shape(prog) : (int)SHAPE_GENERIC;
+    return s == SHAPE_GENERIC || s == SHAPE_NONE ||
+                   !(prog->op[0].flags & PHK_FLAG_DETUNED)
+               ? s : s | (int)SHAPE_DETUNED;
+}
 int launch_track_f32(const phk_program* prog, const phk_coords* c,
                      const phk_kick_set* pk, const phk_accum* acc, int ld,
                      int stm, bool vec_ok, cudaStream_t st);

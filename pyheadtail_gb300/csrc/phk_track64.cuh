@@ -69,10 +69,12 @@ __device__ __forceinline__ void fix64_carry(const FixHist64& f, int S,
     }
 }
 
-// Two CTAs per SM (128 registers): the 64-bit integer chains need them, and
-// 16 warps cover the FP64 pipe's latency.
+// Three CTAs per SM (80 registers): the FP64 pipe and the integer pipes are
+// each about half busy, and the more warps, the better their phases overlap
+// (two / three / four CTAs at 1e7 macroparticles with RF and a 50-turn wake:
+// 406 / 371 / 358 us a turn; with detuning at 1e6: 107 / 92 / 96 us).
 template <int VEC, int SHAPE>
-__global__ void __launch_bounds__(kTrackThreads, 2)
+__global__ void __launch_bounds__(kTrackThreads, 3)
 track64_kernel(const __grid_constant__ phk_program prog,
                const __grid_constant__ phk_kick_set pk,
                const __grid_constant__ phk_accum acc,
@@ -333,8 +335,7 @@ static int launch_track64_t(const phk_program* prog, const phk_coords* c,
     a.n_tiles = (c->n + per_tile - 1) / per_tile;
     ka.sine = program_has_phase(*prog);
     for (int o = 0; o < prog->n_ops; ++o) op_fix(prog->op[o], ka.op + o);
-    for (int d = 0; d < prog->n_det; ++d)
-        if (prog->det[d].kind == PHK_DET_AMPLITUDE) det_fix(prog->det[d], ka.det + d);
+    for (int d = 0; d < prog->n_det; ++d) det_fix(prog->det[d], ka.det + d);
     const size_t limit = track64_limit<VEC, SHAPE>();
     const size_t smem = track64_plan(pk, acc, ka.sine, limit, &ka);
     if (smem > limit)

@@ -3,27 +3,40 @@
 
 namespace phk {
 
+// One particle per thread: the 64-bit chains are long, and 24 warps of them
+// hide each other better than 16 with two (three CTAs per SM at 80 registers
+// against two at 128; 1e6 macroparticles with detuning 92 / 105 us, linear
+// maps 1e6 62 / 72 us).  Two where little is computed for what is loaded:
+// slicing alone, and the undetuned turn with RF from about 4e6 macroparticles
+// on (3e6: 130 / 131 us a turn, 1e7 with a 50-turn wake: 384 / 371 us).
 int launch_track_f64(const phk_program* prog, const phk_coords* c,
                      const phk_kick_set* pk, const phk_accum* acc, int ld,
                      int stm, bool vec_ok, cudaStream_t st) {
-    if (!vec_ok)
-        return launch_track64_t<1, SHAPE_GENERIC>(prog, c, pk, acc, ld, stm, st);
-    switch (program_plain64(*prog) ? program_shape(prog) : (int)SHAPE_GENERIC) {
+    switch (program_shape64(prog)) {
         case SHAPE_NONE:
-            return launch_track64_t<2, SHAPE_NONE>(prog, c, pk, acc, ld, stm, st);
+            if (vec_ok) return launch_track64_t<2, SHAPE_NONE>(prog, c, pk, acc, ld, stm, st);
+            return launch_track64_t<1, SHAPE_NONE>(prog, c, pk, acc, ld, stm, st);
         case SHAPE_T:
-            return launch_track64_t<2, SHAPE_T>(prog, c, pk, acc, ld, stm, st);
+            return launch_track64_t<1, SHAPE_T>(prog, c, pk, acc, ld, stm, st);
         case SHAPE_T_RF:
-            return launch_track64_t<2, SHAPE_T_RF>(prog, c, pk, acc, ld, stm, st);
+            if (vec_ok && c->n >= 4000000)
+                return launch_track64_t<2, SHAPE_T_RF>(prog, c, pk, acc, ld, stm, st);
+            return launch_track64_t<1, SHAPE_T_RF>(prog, c, pk, acc, ld, stm, st);
         case SHAPE_T_LIN:
-            return launch_track64_t<2, SHAPE_T_LIN>(prog, c, pk, acc, ld, stm, st);
+            return launch_track64_t<1, SHAPE_T_LIN>(prog, c, pk, acc, ld, stm, st);
+        case SHAPE_DT:
+            return launch_track64_t<1, SHAPE_DT>(prog, c, pk, acc, ld, stm, st);
+        case SHAPE_DT_RF:
+            return launch_track64_t<1, SHAPE_DT_RF>(prog, c, pk, acc, ld, stm, st);
+        case SHAPE_DT_LIN:
+            return launch_track64_t<1, SHAPE_DT_LIN>(prog, c, pk, acc, ld, stm, st);
         default:
-            return launch_track64_t<2, SHAPE_GENERIC>(prog, c, pk, acc, ld, stm, st);
+            return launch_track64_t<1, SHAPE_GENERIC>(prog, c, pk, acc, ld, stm, st);
     }
 }
 
 int track_clusters_f64(size_t smem) {
-    return track64_clusters<2, SHAPE_GENERIC>(smem);
+    return track64_clusters<1, SHAPE_GENERIC>(smem);
 }
 
 // common program shape of every bunch of a batch (GENERIC unless all equal
@@ -31,20 +44,24 @@ int track_clusters_f64(size_t smem) {
 static int batch_shape(const phk_batch* bt) {
     int sh = -1;
     for (int i = 0; i < bt->n_bunches; ++i) {
-        const int s = program_plain64(bt->programs_host[i])
-                          ? program_shape(bt->programs_host + i) : (int)SHAPE_GENERIC;
+        const int s = program_shape64(bt->programs_host + i);
         if (sh < 0) sh = s;
         else if (s != sh) return SHAPE_GENERIC;
     }
-    return sh == SHAPE_T_RF ? SHAPE_T_RF : SHAPE_GENERIC;
+    return sh == SHAPE_T_RF || sh == SHAPE_DT_RF ? sh : (int)SHAPE_GENERIC;
 }
 
 template <int THREADS>
 static int launch_batch_threads(const phk_batch* bt, const phk_coords* c,
                                 const phk_kick_set* pk, const phk_accum* acc,
                                 int ld, int stm, cudaStream_t st) {
-    if (batch_shape(bt) == SHAPE_T_RF)
-        return launch_batch_t<double, 2, THREADS, SHAPE_T_RF>(bt, c, pk, acc, ld, stm, st);
+    switch (batch_shape(bt)) {
+        case SHAPE_T_RF:
+            return launch_batch_t<double, 2, THREADS, SHAPE_T_RF>(bt, c, pk, acc, ld, stm, st);
+        case SHAPE_DT_RF:
+            return launch_batch_t<double, 2, THREADS, SHAPE_DT_RF>(bt, c, pk, acc, ld, stm, st);
+        default: break;
+    }
     return launch_batch_t<double, 2, THREADS, SHAPE_GENERIC>(bt, c, pk, acc, ld, stm, st);
 }
 
