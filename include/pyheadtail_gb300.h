@@ -500,6 +500,13 @@ int phk_slice_merge(const double *sums, int32_t n_shards, int32_t n_slices,
                     int32_t *counts, double *mean_x, double *mean_y,
                     double *moments_slot, void *stream);
 
+/* The exact lower edges of phk_slicer for cuts starting at `tail` (host
+ * computation): edges, a host array of n_slices + 1 values of `dtype`, gets
+ * the smallest representable u with floor((z - tail) / width) >= k, z = u
+ * (width < 0: z = -u, the mirrored table).  PHK_EPARAM if there is none. */
+int phk_exact_edges(double tail, double width, int32_t n_slices, int32_t dtype,
+                    void *edges);
+
 /* Wake convolution of every kick of `w` (see phk_wake_set). */
 int phk_wake(const phk_wake_set *w, void *stream);
 

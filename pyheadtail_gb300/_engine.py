@@ -54,22 +54,6 @@ def reference_index(z, tail, width):
     return np.floor((np.asarray(z, dtype=np.float64) - tail) / width)
 
 
-def _ordered_keys(x):
-    """Map floats to integers with the same order (sign-magnitude to two's
-    complement); +0 and -0 both map to 0."""
-    it = np.int64 if x.dtype == np.float64 else np.int32
-    b = x.view(it).astype(np.int64)
-    mag = b & (np.int64(2**63 - 1) if it is np.int64 else np.int64(2**31 - 1))
-    return np.where(b < 0, -mag, b)
-
-
-def _from_keys(k, dt):
-    it = np.int64 if dt == np.float64 else np.int32
-    sign = np.int64(-2**63) if it is np.int64 else np.int64(-2**31)
-    b = np.where(k < 0, (-k) | sign, k).astype(it)
-    return b.view(dt)
-
-
 def exact_edges(tail, width, n_slices, code):
     """Lower slice boundaries e_k, k = 0..S, in the coordinate dtype:
     e_k is the smallest representable z with reference_index(z) >= k.
@@ -79,43 +63,13 @@ def exact_edges(tail, width, n_slices, code):
     a particle is the k with e_k <= z < e_{k+1}.  For width < 0 the index is
     non-decreasing in -z; the table is then built for u = -z (negation is
     exact, and (z - tail)/width == (-z - -tail)/(-width) bit for bit).
-    Each e_k is found by bisection over the ordered float lattice."""
-    dt = np_dtype(code)
-    neg = width < 0
-    ks = np.arange(n_slices + 1, dtype=np.float64)
-
-    def ok(u):  # index(z(u)) >= k
-        z = -u.astype(np.float64) if neg else u.astype(np.float64)
-        with np.errstate(invalid='ignore', over='ignore'):
-            return reference_index(z, tail, width) >= ks
-
-    aw = abs(width)
-    mid = (-(tail + ks * width)) if neg else (tail + ks * width)
-    lo = (mid - aw).astype(dt)
-    hi = (mid + aw).astype(dt)
-    for _ in range(64):
-        bad = ok(lo)
-        if not bad.any():
-            break
-        lo[bad] = (lo[bad].astype(np.float64) - 4 * aw).astype(dt)
-    for _ in range(64):
-        bad = ~ok(hi)
-        if not bad.any():
-            break
-        hi[bad] = (hi[bad].astype(np.float64) + 4 * aw).astype(dt)
-    if ok(lo).any() or (~ok(hi)).any():
-        raise N.PhkError('slice edge bracket failed (tail %r width %r)'
-                         % (tail, width))
-    klo, khi = _ordered_keys(lo), _ordered_keys(hi)
-    while True:
-        open_ = khi - klo > 1
-        if not open_.any():
-            break
-        km = klo + (khi - klo) // 2
-        good = ok(_from_keys(km, dt))
-        khi = np.where(open_ & good, km, khi)
-        klo = np.where(open_ & ~good, km, klo)
-    return _from_keys(khi, dt), neg
+    Found by phk_exact_edges over the ordered float lattice (cuts that
+    follow the bunch need a new table every turn: 1.1 ms at 200 slices as
+    array bisection on the host, a few microseconds there)."""
+    e = np.empty(n_slices + 1, dtype=np_dtype(code))
+    N.call('phk_exact_edges', float(tail), float(width), n_slices, code,
+           e.ctypes.data)
+    return e, bool(width < 0)
 
 
 def ceil_to_dtype(v, code):

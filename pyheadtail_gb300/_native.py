@@ -159,6 +159,8 @@ SIGNATURES = {
     'phk_slice_finalize': [ctypes.POINTER(Accum), ctypes.c_void_p,
                            ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                            ctypes.c_void_p],
+    'phk_exact_edges': [ctypes.c_double, ctypes.c_double, ctypes.c_int32,
+                        ctypes.c_int32, ctypes.c_void_p],
     'phk_wake': [ctypes.POINTER(WakeSet), ctypes.c_void_p],
     'phk_kick': [ctypes.POINTER(Coords), ctypes.POINTER(KickSet),
                  ctypes.c_void_p],

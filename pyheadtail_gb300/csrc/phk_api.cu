@@ -2,11 +2,13 @@
 // argument before any launch, thread-local error messages, dispatch to the
 // launchers in phk_kernels.cu.
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <string.h>
 
 #include <atomic>
+#include <cmath>
 #include <mutex>
 #include <vector>
 
@@ -423,6 +425,93 @@ int phk_slice_moments_all(const phk_slicer* slicer, const phk_coords* coords,
     if (coords->n == 0) return PHK_OK;
     return launch_moments_all(slicer, coords, pass, means, sums, counts,
                               (cudaStream_t)stream);
+}
+
+}  // extern "C"
+
+namespace {
+
+// the floats of type T in order, as integers (both zeros are 0)
+template <typename T, typename I>
+int64_t edge_key(T v) {
+    I b;
+    memcpy(&b, &v, sizeof(b));
+    const int64_t mag = (int64_t)(b & (((uint64_t)1 << (8 * sizeof(T) - 1)) - 1));
+    return v < T(0) || b < 0 ? -mag : mag;
+}
+template <typename T, typename I>
+T edge_value(int64_t k) {
+    I b = (I)(k < 0 ? -k : k);
+    T v;
+    memcpy(&v, &b, sizeof(v));
+    return k < 0 ? -v : v;
+}
+
+// e[k], k = 0..n: the smallest representable u with
+// floor((z - tail) / width) >= k, z = u (width < 0: z = -u)
+template <typename T, typename I>
+bool exact_edges(double tail, double width, int n, T* e) {
+    const bool neg = width < 0;
+    const double aw = fabs(width);
+    for (int k = 0; k <= n; ++k) {
+        auto at = [&](T v) {
+            const double u = (double)v;
+            return floor(((neg ? -u : u) - tail) / width) >= (double)k;
+        };
+        auto ok = [&](int64_t key) { return at(edge_value<T, I>(key)); };
+        const double kw = k * width, pos = tail + kw, mid0 = neg ? -pos : pos;
+        // a bracket of a width either side, widened by at most 64 times four
+        // (a width far below the spacing of the floats there is refused)
+        T vlo = (T)(mid0 - aw), vhi = (T)(mid0 + aw);
+        for (int i = 0; i < 64 && at(vlo); ++i) vlo = (T)((double)vlo - 4 * aw);
+        for (int i = 0; i < 64 && !at(vhi); ++i) vhi = (T)((double)vhi + 4 * aw);
+        if (at(vlo) || !at(vhi)) return false;
+        int64_t lo = edge_key<T, I>(vlo), hi = edge_key<T, I>(vhi);
+        // inside it, steps that double from the guess, which is an ulp or two
+        // off; then bisection
+        const int64_t g = edge_key<T, I>((T)mid0);
+        auto gap = [&] { return (uint64_t)hi - (uint64_t)lo; };
+        if (g > lo && g < hi) {
+            const bool down = ok(g);
+            (down ? hi : lo) = g;
+            for (uint64_t step = 1; gap() > step; step *= 2) {
+                const int64_t m = (int64_t)(down ? (uint64_t)hi - step
+                                                 : (uint64_t)lo + step);
+                const bool at_m = ok(m);
+                (at_m ? hi : lo) = m;
+                if (at_m != down) break;
+            }
+        }
+        while (gap() > 1) {
+            const int64_t mid = (int64_t)((uint64_t)lo + gap() / 2);
+            if (ok(mid)) hi = mid; else lo = mid;
+        }
+        e[k] = edge_value<T, I>(hi);
+    }
+    return true;
+}
+
+}  // namespace
+
+extern "C" {
+
+int phk_exact_edges(double tail, double width, int32_t n_slices, int32_t dtype,
+                    void* edges) {
+    const char* who = "phk_exact_edges";
+    if (!edges) return set_error(PHK_ENULL, "%s: edges is NULL", who);
+    if (n_slices < 0)
+        return set_error(PHK_ESIZE, "%s: n_slices %d", who, n_slices);
+    const int r = check_dtype(dtype, who);
+    if (r) return r;
+    bool ok = std::isfinite(tail) && std::isfinite(width) && width != 0.0;
+    if (ok)
+        ok = dtype == PHK_F64
+                 ? exact_edges<double, int64_t>(tail, width, n_slices, (double*)edges)
+                 : exact_edges<float, int32_t>(tail, width, n_slices, (float*)edges);
+    if (!ok)
+        return set_error(PHK_EPARAM, "%s: slice edge bracket failed (tail %g width %g)",
+                         who, tail, width);
+    return PHK_OK;
 }
 
 int phk_track_batch(const phk_batch* batch, const phk_coords* coords,
