@@ -284,6 +284,28 @@ typedef struct phk_wake_set {
     phk_wake_kick kick[PHK_MAX_KICKS];
 } phk_wake_set;
 
+/* ---- resistive-wall samples of the dot path (ResistiveWall
+ *      .function_transverse, wakes.py:611-624): for n_tables tables
+ *   out[j * n_slices + i] = coef[1 + sign(dt + dt_min)]
+ *                           * sqrt(num / min(dt, -dt_min)) * post,
+ *   dt = times[i] - times[n_slices + j]  (target i, source j),
+ * every operation rounded as written (no fused multiply-adds).  times: device,
+ * 2 * n_slices FP64; dt_min > 0, num < 0; coef[2] must be a zero. */
+typedef struct phk_wall_table {
+    double coef[3];
+    double *out;
+} phk_wall_table;
+
+typedef struct phk_wall_tables {
+    int32_t n_slices;
+    int32_t n_tables;
+    double num;
+    double dt_min;
+    double post;
+    const double *times;
+    phk_wall_table table[PHK_MAX_KICKS];
+} phk_wall_tables;
+
 /* ---- multi-turn wake on the tensor cores (FP32 form) --------------------
  * The convolution of phk_wake (numpy path) for every kick of one WakeField
  * as one Toeplitz GEMM with split bfloat16 products (hi*hi + hi*lo + lo*hi
@@ -506,6 +528,9 @@ int phk_slice_merge(const double *sums, int32_t n_shards, int32_t n_slices,
  * (width < 0: z = -u, the mirrored table).  PHK_EPARAM if there is none. */
 int phk_exact_edges(double tail, double width, int32_t n_slices, int32_t dtype,
                     void *edges);
+
+/* The resistive-wall tables of `w` (see phk_wall_tables). */
+int phk_wall_samples(const phk_wall_tables *w, void *stream);
 
 /* Wake convolution of every kick of `w` (see phk_wake_set). */
 int phk_wake(const phk_wake_set *w, void *stream);

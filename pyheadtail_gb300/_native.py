@@ -97,6 +97,17 @@ class WakeSet(ctypes.Structure):
                 ('kick', WakeKick * PHK_MAX_KICKS)]
 
 
+class WallTable(ctypes.Structure):
+    _fields_ = [('coef', ctypes.c_double * 3), ('out', ctypes.c_void_p)]
+
+
+class WallTables(ctypes.Structure):
+    _fields_ = [('n_slices', ctypes.c_int32), ('n_tables', ctypes.c_int32),
+                ('num', ctypes.c_double), ('dt_min', ctypes.c_double),
+                ('post', ctypes.c_double), ('times', ctypes.c_void_p),
+                ('table', WallTable * PHK_MAX_KICKS)]
+
+
 class WakeTC(ctypes.Structure):
     _fields_ = [('n_slices', ctypes.c_int32), ('ring_len', ctypes.c_int32),
                 ('head', ctypes.c_int32), ('n_kicks', ctypes.c_int32),
@@ -161,6 +172,7 @@ SIGNATURES = {
                            ctypes.c_void_p],
     'phk_exact_edges': [ctypes.c_double, ctypes.c_double, ctypes.c_int32,
                         ctypes.c_int32, ctypes.c_void_p],
+    'phk_wall_samples': [ctypes.POINTER(WallTables), ctypes.c_void_p],
     'phk_wake': [ctypes.POINTER(WakeSet), ctypes.c_void_p],
     'phk_kick': [ctypes.POINTER(Coords), ctypes.POINTER(KickSet),
                  ctypes.c_void_p],

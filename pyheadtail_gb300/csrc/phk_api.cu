@@ -326,6 +326,31 @@ int phk_slice_merge(const double* sums, int32_t n_shards, int32_t n_slices,
                               moments_slot, (cudaStream_t)stream);
 }
 
+int phk_wall_samples(const phk_wall_tables* w, void* stream) {
+    const char* who = "phk_wall_samples";
+    if (!w) return set_error(PHK_ENULL, "%s: wall tables are NULL", who);
+    if (w->n_slices < 1 || w->n_slices > PHK_MAX_SLICES)
+        return set_error(PHK_ESIZE, "%s: n_slices %d outside [1, %d]", who,
+                         w->n_slices, PHK_MAX_SLICES);
+    if (w->n_tables < 0 || w->n_tables > PHK_MAX_KICKS)
+        return set_error(PHK_ESIZE, "%s: n_tables %d", who, w->n_tables);
+    if (!(w->dt_min > 0.0) || !(w->num < 0.0))
+        return set_error(PHK_EPARAM, "%s: dt_min %g num %g", who, w->dt_min,
+                         w->num);
+    if (!w->times) return set_error(PHK_ENULL, "%s: times is NULL", who);
+    int r = check_aligned(w->times, 8, who, "times");
+    if (r) return r;
+    for (int k = 0; k < w->n_tables; ++k) {
+        if (!w->table[k].out)
+            return set_error(PHK_ENULL, "%s: table %d is NULL", who, k);
+        if (w->table[k].coef[2] != 0.0)
+            return set_error(PHK_EPARAM, "%s: table %d coef[2]", who, k);
+        if ((r = check_aligned(w->table[k].out, 8, who, "a table"))) return r;
+    }
+    if (w->n_tables == 0) return PHK_OK;
+    return launch_wall_tables(w, (cudaStream_t)stream);
+}
+
 int phk_wake(const phk_wake_set* w, void* stream) {
     if (!w) return set_error(PHK_ENULL, "phk_wake: wake set is NULL");
     if (w->n_slices < 1 || w->n_slices > PHK_MAX_SLICES)

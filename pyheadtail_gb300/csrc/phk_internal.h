@@ -54,6 +54,8 @@ int launch_slice_merge(const double* sums, int n_shards, int S,
 int launch_finalize(const phk_accum* acc, int32_t* counts, double* mean_x,
                     double* mean_y, double* moments, cudaStream_t stream);
 int launch_wake(const phk_wake_set* w, cudaStream_t stream);
+void launch_wake_dense(const phk_wake_set* w, cudaStream_t stream);
+int launch_wall_tables(const phk_wall_tables* w, cudaStream_t stream);
 int launch_moments(const phk_slicer* s, const void* z, int64_t n,
                    int32_t dtype, const void* const* q, int32_t n_q,
                    int32_t pass, const double* means, double* sums,

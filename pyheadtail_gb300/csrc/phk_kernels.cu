@@ -324,7 +324,8 @@ __device__ __forceinline__ void wake_conv_one(const phk_wake_set& w, int gw,
     }
 }
 
-// dot-product path: one thread per (kick, target slice); coalesced over i
+// dot-product path of the batched wake: one thread per (kick, target slice);
+// coalesced over i
 __device__ __forceinline__ void wake_dense_one(const phk_wake_set& w, int t) {
     const int S = w.n_slices;
     const int k = t / S;
@@ -545,10 +546,6 @@ wake_conv_kernel(const __grid_constant__ phk_wake_set w) {
     cl.sync();                         // sums stay until rank 0 has read them
 }
 
-__global__ void wake_dense_kernel(const __grid_constant__ phk_wake_set w) {
-    wake_dense_one(w, blockIdx.x * blockDim.x + threadIdx.x);
-}
-
 int launch_wake(const phk_wake_set* w, cudaStream_t st) {
     bool any_dense = false, any_conv = false;
     for (int k = 0; k < w->n_kicks; ++k) {
@@ -570,10 +567,7 @@ int launch_wake(const phk_wake_set* w, cudaStream_t st) {
             wake_conv_kernel<<<w->n_kicks * ((S + kConvTargets - 1) / kConvTargets) *
                                    kConvCluster, kConvWarps * 32, 0, st>>>(*w);
     }
-    if (any_dense) {
-        const int n = w->n_kicks * S;
-        wake_dense_kernel<<<(n + 127) / 128, 128, 0, st>>>(*w);
-    }
+    if (any_dense) launch_wake_dense(w, st);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return set_error(PHK_ECUDA, "phk_wake launch: %s", cudaGetErrorString(e));

@@ -13,12 +13,14 @@ device.  The convolution over all stored turns runs in ``phk_wake``; the
 resulting per-slice kick is left pending on the beam and applied to the
 particles at the start of the next fused pass.
 """
+import ctypes
 from abc import ABCMeta
 
 import numpy as np
 import torch
 from scipy.constants import c
 
+from .. import _engine as E
 from .. import _native as N
 from ..general.element import Printing
 
@@ -66,27 +68,31 @@ class WakeKick(Printing, metaclass=ABCMeta):
                                  (target_times - source_times[0])[1:]))
         return self.wake_function(dt, beta=source_beta)
 
-    def _sync_tables(self, times, ages, betas, n_slices, device):
-        """Make table[a] = wake samples of stored turn a for every lag in
-        use; upload only the lags whose inputs changed."""
-        n_lags = min(len(ages), self.n_turns_wake)
+    def _stale_lags(self, times, ages, betas, n_slices, device):
+        """(lag, key) of the table rows in use whose inputs changed."""
         width = n_slices * n_slices if self._dense else 2 * n_slices - 1
         if (self._table is None or self._table.shape[1] != width or
                 self._table.device != device):
             self._table = torch.zeros(self.n_turns_wake, width,
                                       dtype=torch.float64, device=device)
             self._keys = [None] * self.n_turns_wake
-        for a in range(n_lags):
+        for a in range(min(len(ages), self.n_turns_wake)):
             key = (times[0], times[a], float(ages[a]), float(betas[a]))
             old = self._keys[a]
             if (old is not None and old[0] is key[0] and old[1] is key[1]
                     and old[2] == key[2] and old[3] == key[3]):
                 continue
+            yield a, key
+
+    def _sync_tables(self, times, ages, betas, n_slices, device):
+        """Make table[a] = wake samples of stored turn a for every lag in
+        use; upload only the lags whose inputs changed."""
+        for a, key in self._stale_lags(times, ages, betas, n_slices, device):
             w = self._samples(times[0], times[a] + ages[a], betas[a])
             self._table[a].copy_(torch.from_numpy(
                 np.ascontiguousarray(w, dtype=np.float64).ravel()))
             self._keys[a] = key
-        return n_lags
+        return min(len(ages), self.n_turns_wake)
 
     def _fill(self, st, bunch, slice_sets, ages, out):
         """Fill the phk_wake_kick block of this kick for the current turn."""
@@ -109,6 +115,44 @@ class WakeKick(Printing, metaclass=ABCMeta):
         """Standalone use (outside a WakeField): convolve and kick now."""
         from .wakes import _run_kicks
         _run_kicks([self], bunch, slice_set_list, slice_set_age_list)
+
+
+def sync_wall_tables(kicks, slice_sets, ages, device):
+    """Make the stale resistive-wall tables of the dot-product path on the
+    device (phk_wall_samples), one launch per stored turn and set of wall
+    constants.  They need S x S samples a turn: in NumPy, with the uploads,
+    7 ms a turn for four kicks of 500 slices.  Wakes that are not a
+    resistive wall's are left to _sync_tables."""
+    times = [s._times for s in slice_sets]
+    betas = [s.beta for s in slice_sets]
+    n_slices = slice_sets[0].n_slices
+    launches = {}
+    for kick in kicks:
+        wall = getattr(kick.wake_function, 'wall', None)
+        if not kick._dense or wall is None:
+            continue
+        for a, key in kick._stale_lags(times, ages, betas, n_slices, device):
+            constants = wall(betas[a])
+            if constants is None:
+                break
+            coef, rest = constants
+            launches.setdefault((a,) + rest, []).append((kick, key, coef))
+    on_device = {}
+    for (a, num, dt_min, post), group in launches.items():
+        if a not in on_device:
+            on_device[a] = torch.from_numpy(np.stack(
+                (times[0], times[a] + ages[a])).astype(np.float64)
+                ).pin_memory().to(device, non_blocking=True)
+        w = N.WallTables()
+        w.n_slices = n_slices
+        w.num, w.dt_min, w.post = num, dt_min, post
+        w.times = on_device[a].data_ptr()
+        w.n_tables = len(group)
+        for entry, (kick, key, coef) in zip(w.table, group):
+            entry.coef[:] = coef
+            entry.out = kick._table[a].data_ptr()
+            kick._keys[a] = key
+        N.call('phk_wall_samples', ctypes.byref(w), E.stream_handle())
 
 
 class ConstantWakeKickX(WakeKick):

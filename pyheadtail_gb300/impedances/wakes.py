@@ -30,7 +30,8 @@ from .. import _native as N
 from ..general.element import Element, Printing
 from ..particles.slicing import make_slice_set
 from .wake_kicks import (ConstantWakeKickZ, DipoleWakeKickX, DipoleWakeKickY,
-                         QuadrupoleWakeKickX, QuadrupoleWakeKickY)
+                         QuadrupoleWakeKickX, QuadrupoleWakeKickY,
+                         sync_wall_tables)
 
 sin = np.sin
 cos = np.cos
@@ -154,6 +155,7 @@ def _run_kicks(kicks, bunch, slice_sets, ages, state=None):
     ws.out_dtype = bunch._code
     ws.moments = state.moments.data_ptr()
     entries = []
+    sync_wall_tables(kicks, slice_sets, ages, state.moments.device)
     for k, kick in enumerate(kicks):
         out = state.kick_out[k]
         kick._fill(ws.kick[k], bunch, slice_sets, ages, out)
@@ -383,6 +385,26 @@ class ResistiveWall(WakeSource):
                      -mu_r / np.pi / self.conductivity /
                      dt.clip(max=-abs(self.dt_min)))) * np.sqrt(Z_0 * c)
             return y
+
+        def wall(beta):
+            """wake(dt) as (coefficients of the signs of dt + dt_min,
+            (dividend under the root, dt_min, last factor)) for
+            phk_wall_samples, or None where these are not plain numbers of
+            the signs it takes.  The products are wake's own, in its order."""
+            before = (Yokoya_factor * (np.array([-1., 0., 1.]) - 1) / 2. *
+                      np.sqrt(beta) * self.resistive_wall_length /
+                      np.pi / self.pipe_radius**3)
+            num = -mu_r / np.pi / self.conductivity
+            dt_min = abs(self.dt_min)
+            if (self.pipe_radius.size != 1 or before.shape != (3,) or
+                    np.ndim(num) or np.ndim(dt_min) or
+                    not np.all(np.isfinite(before)) or
+                    not -np.inf < num < 0 or not 0 < dt_min < np.inf):
+                return None
+            return before.tolist(), (float(num), float(dt_min),
+                                     float(np.sqrt(Z_0 * c)))
+
+        wake.wall = wall
         return wake
 
 
