@@ -1014,66 +1014,21 @@ __device__ __forceinline__ void run_program_shape(const phk_program& prog,
 // ===================================================================
 // per-slice accumulation in shared memory
 //
-// Batched kernels: each warp owns a private histogram (count, sum x, sum y
-//   per slice); lanes of a warp holding the same slice are serialised by
-//   bids (warp_accumulate), so a bin is updated in a fixed lane order and
-//   the sums do not depend on scheduling.  FP64: plain double sums; FP32:
-//   Kahan (1965) compensated float sums, one (sum, compensation) float2 per
-//   bin.  When the per-warp copies do not fit the shared-memory plan, warps
-//   share copies through atomics; the order of the warps sharing a copy is
-//   then not fixed, so those sums can differ in their last bits between
-//   launches.
+// Fixed-point sums (FixHist below, FixHist64), one histogram per CTA updated
+//   with 32-bit integer atomics: integer addition is associative, so the
+//   sums are bit-identical whatever the order.
 //
-// Single-bunch kernel: fixed-point sums (FixHist below, FixHist64), one
-//   histogram per CTA updated with 32-bit integer atomics: integer addition
-//   is associative, so the sums are bit-identical whatever the order.
+// FP64 batch: each warp owns a private histogram (count, sum x, sum y per
+//   slice) of plain double sums; lanes of a warp holding the same slice are
+//   serialised by bids (warp_accumulate), so a bin is updated in a fixed lane
+//   order and the sums do not depend on scheduling.  When the per-warp copies
+//   do not fit the shared-memory plan, warps share copies through atomics; the
+//   order of the warps sharing a copy is then not fixed, so those sums can
+//   differ in their last bits between launches.  (In the FP32 batch, bids
+//   with compensated float sums took 40 % of the shared-memory pipe and a
+//   fifth of the instructions: 207 us a pass at 64 bunches and 1.03e7
+//   particles against 181 us as fixed-point sums.)
 // ===================================================================
-
-template <typename T>
-struct Hist;
-
-template <>
-struct Hist<double> {
-    using Word = double;
-    static __device__ __forceinline__ void zero(Word* w) { *w = 0.0; }
-    static __device__ __forceinline__ void add(Word* w, double v) {
-        *w = ::phk::add(*w, v);
-    }
-    static __device__ __forceinline__ void add_atomic(Word* w, double v) {
-        atomicAdd(w, v);
-    }
-    static __device__ __forceinline__ void merge(Word* dst, const Word* src) {
-        *dst = ::phk::add(*dst, *src);
-    }
-    static __device__ __forceinline__ double value(const Word* w) { return *w; }
-};
-
-template <>
-struct Hist<float> {
-    using Word = float2;  // x: running sum, y: Kahan compensation
-    static __device__ __forceinline__ void zero(Word* w) {
-        *w = make_float2(0.f, 0.f);
-    }
-    static __device__ __forceinline__ void add(Word* w, float v) {
-        float2 a = *w;
-        const float yk = v - a.y;
-        const float tk = a.x + yk;
-        a.y = (tk - a.x) - yk;
-        a.x = tk;
-        *w = a;
-    }
-    static __device__ __forceinline__ void add_atomic(Word* w, float v) {
-        atomicAdd(&w->x, v);
-    }
-    static __device__ __forceinline__ void merge(Word* dst, const Word* src) {
-        const float2 b = *src;
-        add(dst, b.x - b.y);
-    }
-    static __device__ __forceinline__ double value(const Word* w) {
-        const float2 a = *w;
-        return (double)(a.x - a.y);
-    }
-};
 
 // All 32 lanes of the warp must call this together; s < 0 means "no bin".
 // Lanes of a warp that hold the same slice are serialised by bids: in each
@@ -1081,18 +1036,16 @@ struct Hist<float> {
 // warp's private tag array; the standing bid (the highest pending lane of
 // that slice) updates the bin with plain loads and stores.  A bin is thus
 // always updated in descending lane order: the sums are deterministic.
-template <typename T>
-__device__ __forceinline__ void warp_accumulate(int s, T vx, T vy,
-                                                typename Hist<T>::Word* hx,
-                                                typename Hist<T>::Word* hy,
+__device__ __forceinline__ void warp_accumulate(int s, double vx, double vy,
+                                                double* hx, double* hy,
                                                 int* hc, int* tag,
                                                 unsigned& epoch,
                                                 bool shared_hist) {
     if (shared_hist) {
         if (s >= 0) {
             atomicAdd(hc + s, 1);
-            Hist<T>::add_atomic(hx + s, vx);
-            Hist<T>::add_atomic(hy + s, vy);
+            atomicAdd(hx + s, vx);
+            atomicAdd(hy + s, vy);
         }
         return;
     }
@@ -1105,8 +1058,8 @@ __device__ __forceinline__ void warp_accumulate(int s, T vx, T vy,
         __syncwarp();
         if (pending && tag[s] == bid) {
             hc[s] += 1;
-            Hist<T>::add(hx + s, vx);
-            Hist<T>::add(hy + s, vy);
+            hx[s] = add(hx[s], vx);
+            hy[s] = add(hy[s], vy);
             pending = false;
         }
         __syncwarp();
@@ -1116,9 +1069,9 @@ __device__ __forceinline__ void warp_accumulate(int s, T vx, T vy,
 // -------------------------------------------------------------------
 // FixHist: exact, order-independent per-slice sums of FP32 coordinates.
 //
-// Every thread-block cluster agrees on one power-of-two scale per
-// coordinate, 2^k with k chosen from the largest finite |u| of the
-// cluster's first tiles so that it maps to [2^26, 2^27).  A value
+// Every thread-block cluster (batch: every CTA, for each bunch it works on)
+// agrees on one power-of-two scale per coordinate, 2^k with k chosen from the
+// largest finite |u| of its first tiles so that it maps to [2^26, 2^27).  A value
 // u becomes the integer v = rint(u 2^k) (u 2^k is exact; the rounding is
 // the only approximation, at most 2^-27 of that largest value, the order
 // of the FP32 rounding of u itself).  Level A, |u 2^k| < 2^30: v is split into two
@@ -1301,10 +1254,10 @@ template <>
 __device__ __forceinline__ float tmul<float>(float a, float b) { return a * b; }
 
 // shared memory layout, in this order (every region 16-byte aligned):
-//   histogram: bid-serialised words [3][n_hist][Sa] (sum x, sum y as
-//              Hist<T>::Word; count as int in the third region), or with
-//              `fix` (FP32 single bunch) the FixHist counters: count [Sa],
-//              digits [4][Sa], flag bytes [Sa] (ints)
+//   histogram: bid-serialised words [3][n_hist][Sa] (sum x, sum y as double;
+//              count as int in the third region), or with `fix` (FP32) the
+//              FixHist counters: count [Sa], digits [4][Sa], flag bytes [Sa]
+//              (ints)
 //   accumulation edges [Sa + 1] T, pending-kick edges [Sp + 1] T,
 //   kick tables [n_tables][Sp] T (when staged), bid tags [n_hist][Sa] int
 //   (none with `fix`), TMA ring [stages][6][tile] T, one mbarrier per stage
@@ -1590,36 +1543,42 @@ __device__ __forceinline__ void apply_pending(const phk_kick_set& pk,
 // Per-CTA state shared by the tile loops of the track kernel.
 template <typename T, int VEC>
 struct TrackCtx {
-    using W = typename Hist<T>::Word;
     T* cp[6];
     Bins<T> bpk, bac;
     const T* ktab;
-    W* hx;
-    W* hy;
+    double* hx;           // FP64 batch
+    double* hy;
     int* hc;
     int* tag;
     unsigned epoch;
     bool shared_hist;
-    typename FixOf<T>::type fix;   // single-bunch accumulation
+    typename FixOf<T>::type fix;   // single bunch, FP32 batch
     Aux64 aux;            // FP64 form
 };
 
-// One tile of VEC particles per thread, already in registers: pending
-// kicks, element program, slice accumulation; then the stores.  All threads
-// of the CTA call this together (the accumulation is warp-synchronous);
-// lanes whose particles are past the end pass live = false.
-template <typename T, int VEC, int SHAPE, bool FULL, bool FIX = false>
-__device__ __forceinline__ void run_tile(const phk_program& prog,
-                                         const phk_kick_set& pk,
-                                         const phk_accum& acc,
-                                         const TrackArgs& a,
-                                         TrackCtx<T, VEC>& cx, Tile<T, VEC>& t,
-                                         int64_t i0, bool full) {
-    // 1. wake kicks of the previous WakeField.track, in kick order
+// One tile of VEC particles per thread, already in registers.  All threads
+// of the CTA call this together (the FP64 batch's accumulation is
+// warp-synchronous); lanes whose particles are past the end pass live = false.
+
+// 1. wake kicks of the previous WakeField.track, in kick order;
+// 2. element program
+template <typename T, int VEC, int SHAPE, bool FULL>
+__device__ __forceinline__ void tile_advance(const phk_program& prog,
+                                             const phk_kick_set& pk,
+                                             const TrackArgs& a,
+                                             TrackCtx<T, VEC>& cx,
+                                             Tile<T, VEC>& t, int64_t i0) {
     if (a.has_pk) apply_pending<T, VEC, FULL>(pk, a, cx.bpk, cx.ktab, t, i0);
-    // 2. element program
     run_program_shape<T, VEC, SHAPE>(prog, cx.aux, t);
-    // 3. slice accumulation
+}
+
+// 3. slice accumulation; 4. stores
+template <typename T, int VEC, bool FULL, bool FIX>
+__device__ __forceinline__ void tile_finish(const phk_accum& acc,
+                                            const TrackArgs& a,
+                                            TrackCtx<T, VEC>& cx,
+                                            Tile<T, VEC>& t, int64_t i0,
+                                            bool full) {
     if (a.has_acc) {
         int sl[VEC];
         cx.bac.index_vec(t.c[PHK_Z], sl);
@@ -1635,7 +1594,7 @@ __device__ __forceinline__ void run_tile(const phk_program& prog,
             if constexpr (FIX) {
                 if (s >= 0) cx.fix.add(s, t.c[PHK_X][j], t.c[PHK_Y][j]);
             } else {
-                warp_accumulate<T>(s, t.c[PHK_X][j], t.c[PHK_Y][j], cx.hx, cx.hy,
+                warp_accumulate(s, t.c[PHK_X][j], t.c[PHK_Y][j], cx.hx, cx.hy,
                                    cx.hc, cx.tag, cx.epoch, cx.shared_hist);
             }
         }
@@ -1652,6 +1611,17 @@ __device__ __forceinline__ void run_tile(const phk_program& prog,
                 if (i0 + j < a.n) cx.cp[q][i0 + j] = t.c[q][j];
         }
     }
+}
+
+template <typename T, int VEC, int SHAPE, bool FULL, bool FIX = false>
+__device__ __forceinline__ void run_tile(const phk_program& prog,
+                                         const phk_kick_set& pk,
+                                         const phk_accum& acc,
+                                         const TrackArgs& a,
+                                         TrackCtx<T, VEC>& cx, Tile<T, VEC>& t,
+                                         int64_t i0, bool full) {
+    tile_advance<T, VEC, SHAPE, FULL>(prog, pk, a, cx, t, i0);
+    tile_finish<T, VEC, FULL, FIX>(acc, a, cx, t, i0, full);
 }
 
 template <typename T, int VEC>
@@ -2311,24 +2281,29 @@ template <typename T, int VEC, int THREADS, int SHAPE>
 __global__ void __launch_bounds__(THREADS, (sizeof(T) == 4 ? 1024 : 512) / THREADS)
 batch_track_kernel(const __grid_constant__ phk_kick_set pk,
                    const __grid_constant__ phk_accum acc, const BatchArgs b) {
-    using W = typename Hist<T>::Word;
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int TILE = THREADS * VEC;
+    constexpr bool F64 = sizeof(T) == 8;
+    constexpr bool FIX = !F64;
     const TrackArgs& a = b.a;
     const int Sa = a.has_acc ? acc.slicer.n_slices : 0;
     const int Sp = a.has_pk ? pk.slicer.n_slices : 0;
     const int nk = a.has_pk ? pk.n_kicks : 0;
     phk_program* sprog = reinterpret_cast<phk_program*>(smem);
     u64* sine = reinterpret_cast<u64*>(smem + kProgSmem);
-    constexpr bool F64 = sizeof(T) == 8;
     __shared__ OpFix s_op[F64 ? PHK_MAX_OPS : 1];
     __shared__ DetFix s_det[F64 ? PHK_MAX_DETUNERS : 1];
     unsigned char* rest = smem + batch_head<T>();
     size_t off[9];
-    track_smem_layout<T>(Sa, Sp, a.n_hist, nk, 1, 0, TILE, off);
-    W* hsx = reinterpret_cast<W*>(rest + off[0]);
-    W* hsy = reinterpret_cast<W*>(rest + off[1]);
-    int* hcnt = reinterpret_cast<int*>(rest + off[2]);
+    track_smem_layout<T>(Sa, Sp, a.n_hist, nk, 1, 0, TILE, off, FIX);
+    // FIX: one set of counters per CTA, level B in the partial column
+    double* hsx = reinterpret_cast<double*>(rest + off[0]);
+    double* hsy = reinterpret_cast<double*>(rest + off[1]);
+    int* hcnt = reinterpret_cast<int*>(rest + (FIX ? off[0] : off[2]));
+    int* fdig = reinterpret_cast<int*>(rest + off[1]);
+    unsigned* fflag = reinterpret_cast<unsigned*>(rest + off[2]);
+    __shared__ FixSpill s_spill;
+    __shared__ unsigned s_max[2];
     T* eacc = reinterpret_cast<T*>(rest + off[3]);
     T* epk = reinterpret_cast<T*>(rest + off[4]);
     T* ktab = reinterpret_cast<T*>(rest + off[5]);
@@ -2338,11 +2313,20 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
     if (a.has_acc) {
         const T* e = reinterpret_cast<const T*>(acc.slicer.edges);
         for (int i = tid; i <= Sa; i += THREADS) stage_edge<T>(eacc, i, e[i]);
-        for (int i = tid; i < a.n_hist * Sa; i += THREADS) {
-            Hist<T>::zero(hsx + i); Hist<T>::zero(hsy + i);
-            hcnt[i] = 0; htag[i] = 0;
-        }
     }
+    auto clear = [&]() {
+        if constexpr (FIX) {
+            for (int i = tid; i < Sa; i += THREADS) hcnt[i] = 0;
+            for (int i = tid; i < 4 * Sa; i += THREADS) fdig[i] = 0;
+            for (int i = tid; i < (Sa + 3) / 4; i += THREADS) fflag[i] = 0u;
+        } else {
+            for (int i = tid; i < a.n_hist * Sa; i += THREADS) {
+                hsx[i] = 0.0; hsy[i] = 0.0;
+                hcnt[i] = 0; htag[i] = 0;
+            }
+        }
+    };
+    clear();
     if (a.has_pk) {
         const T* e = reinterpret_cast<const T*>(pk.slicer.edges);
         for (int i = tid; i <= Sp; i += THREADS) stage_edge<T>(epk, i, e[i]);
@@ -2354,13 +2338,22 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
 #pragma unroll
     for (int q = 0; q < 6; ++q) cx.cp[q] = reinterpret_cast<T*>(a.c[q]);
     cx.ktab = ktab;
-    const int h = (a.n_hist > 1) ? (tid >> 5) % a.n_hist : 0;
-    cx.hx = hsx + h * Sa;
-    cx.hy = hsy + h * Sa;
-    cx.hc = hcnt + h * Sa;
-    cx.tag = htag + h * Sa;
-    cx.epoch = 0;
-    cx.shared_hist = a.n_hist < THREADS / 32;
+    if constexpr (FIX) {
+        cx.fix.cnt = hcnt;
+        cx.fix.dig = fdig;
+        cx.fix.flag = fflag;
+        cx.fix.sp = &s_spill;
+        cx.fix.S = Sa;
+        cx.fix.scale[0] = cx.fix.scale[1] = 1.f;
+    } else {
+        const int h = (a.n_hist > 1) ? (tid >> 5) % a.n_hist : 0;
+        cx.hx = hsx + h * Sa;
+        cx.hy = hsy + h * Sa;
+        cx.hc = hcnt + h * Sa;
+        cx.tag = htag + h * Sa;
+        cx.epoch = 0;
+        cx.shared_hist = a.n_hist < THREADS / 32;
+    }
     __syncthreads();
     if (a.has_pk) cx.bpk.init(epk, Sp, pk.slicer.negate);
     if (a.has_acc) cx.bac.init(eacc, Sa, acc.slicer.negate);
@@ -2373,27 +2366,38 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
         u0 = u1 = 0;
     }
     int cur = -1, col = -1;
+    int tiles = -1;              // FIX: since the last carry; -1: a new run
     // write the CTA's sums of the current bunch to its column, then zero
     auto flush = [&]() {
         __syncthreads();
+        const int G = b.n_columns;
+        double* P = acc.partials;
         for (int s = tid; s < Sa; s += THREADS) {
             int c = hcnt[s];
-            for (int k = 1; k < a.n_hist; ++k) {
-                c += hcnt[k * Sa + s];
-                Hist<T>::merge(hsx + s, hsx + k * Sa + s);
-                Hist<T>::merge(hsy + s, hsy + k * Sa + s);
+            double v[2];
+            if constexpr (FIX) {
+                const unsigned fl = (fflag[s >> 2] >> (8 * (s & 3))) & 0xffu;
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    v[q] = fix_value(
+                        __ldcg(s_spill.spill[q] + (int64_t)s * G) +
+                            FixHist::total(fdig + 2 * q * Sa + s, Sa),
+                        q ? fl >> 4 : fl & 15u, cx.fix.scale[q]);
+            } else {
+                v[0] = hsx[s];
+                v[1] = hsy[s];
+                for (int k = 1; k < a.n_hist; ++k) {
+                    c += hcnt[k * Sa + s];
+                    v[0] = add(v[0], hsx[k * Sa + s]);
+                    v[1] = add(v[1], hsy[k * Sa + s]);
+                }
             }
-            const int G = b.n_columns;
-            double* P = acc.partials;
             P[(int64_t)s * G + col] = (double)c;
-            P[(int64_t)(Sa + s) * G + col] = Hist<T>::value(hsx + s);
-            P[(int64_t)(2 * Sa + s) * G + col] = Hist<T>::value(hsy + s);
+            P[(int64_t)(Sa + s) * G + col] = v[0];
+            P[(int64_t)(2 * Sa + s) * G + col] = v[1];
         }
         __syncthreads();
-        for (int i = tid; i < a.n_hist * Sa; i += THREADS) {
-            Hist<T>::zero(hsx + i); Hist<T>::zero(hsy + i);
-            hcnt[i] = 0; htag[i] = 0;
-        }
+        clear();
     };
     for (int u = u0; u < u1; ++u) {
         const phk_unit U = b.units[u];
@@ -2436,9 +2440,22 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
                     for (int i = tid; i < nk * Sp; i += THREADS) ktab[i] = kt[i];
                 }
             }
-            __syncthreads();
             cur = U.bunch;
             col = U.column;
+            if (FIX && a.has_acc) {
+                const int G = b.n_columns;
+                long long* P = reinterpret_cast<long long*>(acc.partials);
+                if (tid == 0) {
+                    s_spill.spill[0] = P + (int64_t)Sa * G + col;
+                    s_spill.spill[1] = P + (int64_t)2 * Sa * G + col;
+                    s_spill.stride = G;
+                    s_max[0] = s_max[1] = 0u;
+                }
+                for (int s = tid; s < 2 * Sa; s += THREADS)
+                    P[(int64_t)(Sa + s) * G + col] = 0;
+                tiles = -1;
+            }
+            __syncthreads();
         }
         TrackArgs ua = a;
         ua.n = U.end;
@@ -2447,7 +2464,36 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
             const bool full = i0 + VEC <= U.end;
             Tile<T, VEC> t;
             load_tile_plain<T, VEC>(ua, cx, t, i0, full);
-            run_tile<T, VEC, SHAPE, false>(*sprog, pk, acc, ua, cx, t, i0, full);
+            tile_advance<T, VEC, SHAPE, false>(*sprog, pk, ua, cx, t, i0);
+            if constexpr (FIX) {
+                if (a.has_acc && tiles < 0) {
+                    // the scale of the run, from its first tile
+                    unsigned m[2] = {0u, 0u};
+#pragma unroll
+                    for (int j = 0; j < VEC; ++j) {
+                        const unsigned x = __float_as_uint(fabsf(t.c[PHK_X][j]));
+                        const unsigned y = __float_as_uint(fabsf(t.c[PHK_Y][j]));
+                        if (i0 + j < ua.n && x < 0x7f800000u) m[0] = max(m[0], x);
+                        if (i0 + j < ua.n && y < 0x7f800000u) m[1] = max(m[1], y);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        m[q] = __reduce_max_sync(~0u, m[q]);
+                        if ((tid & 31) == 0) atomicMax(s_max + q, m[q]);
+                    }
+                    __syncthreads();
+                    cx.fix.scale[0] = fix_scale(s_max[0]);
+                    cx.fix.scale[1] = fix_scale(s_max[1]);
+                    tiles = 0;
+                } else if (a.has_acc && tiles == fix_flush_tiles<TILE>()) {
+                    __syncthreads();
+                    fix_flush(cx.fix, tid, THREADS);
+                    __syncthreads();
+                    tiles = 0;
+                }
+                ++tiles;
+            }
+            tile_finish<T, VEC, false, FIX>(acc, ua, cx, t, i0, full);
         }
     }
     if (cur >= 0 && a.has_acc) flush();
@@ -2460,12 +2506,14 @@ static size_t batch_smem(int Sa, int Sp, int nk, int threads, int* n_hist) {
     const int tile = threads * (sizeof(T) == 8 ? 2 : kF32Vec);
     size_t off[9];
     const int warps = threads / 32;
-    // one private histogram copy per warp when it stays within 48 KB
-    int nh = Sa > 0 ? warps : 1;
-    size_t bytes = track_smem_layout<T>(Sa, Sp, nh, nk, 1, 0, tile, off);
-    if (bytes > 48 * 1024 && Sa > 0) {
+    // FP32: one set of fixed-point counters; FP64: one private histogram copy
+    // per warp when it stays within 48 KB
+    constexpr bool fix = sizeof(T) == 4;
+    int nh = Sa > 0 && !fix ? warps : 1;
+    size_t bytes = track_smem_layout<T>(Sa, Sp, nh, nk, 1, 0, tile, off, fix);
+    if (bytes > 48 * 1024 && Sa > 0 && !fix) {
         nh = 1;
-        bytes = track_smem_layout<T>(Sa, Sp, nh, nk, 1, 0, tile, off);
+        bytes = track_smem_layout<T>(Sa, Sp, nh, nk, 1, 0, tile, off, fix);
     }
     *n_hist = nh;
     return batch_head<T>() + bytes;
