@@ -70,10 +70,14 @@ def bunch_offsets(counts, align=ALIGN):
     return off, int(pos)
 
 
-def plan_units(offsets, counts, grid, unit_particles):
+def plan_units(offsets, counts, grid, unit_particles, tile=ALIGN):
     """Split every bunch into units of at most ``unit_particles`` (a multiple
     of ALIGN) and give CTA g the contiguous unit range
-    cta_first[g] .. cta_first[g+1]-1 holding about 1/grid of the particles.
+    cta_first[g] .. cta_first[g+1]-1 holding about 1/grid of the particles:
+    units also end where a CTA's share does, rounded down to whole tiles of
+    ``tile`` particles (a multiple of ALIGN) of the bunch.  (Shares of whole
+    units gave CTAs four or five of them at 64 bunches of 1e4 to 1e6
+    particles: SMs were busy between 321 and 409 thousand cycles.)
 
     Returns dict(units: int64[n_units, 3] (start, end, bunch), column:
     int32[n_units], cta_first: int32[grid+1], bunch_columns: int32[nb+1],
@@ -84,22 +88,32 @@ def plan_units(offsets, counts, grid, unit_particles):
         raise ValueError('unit_particles must be a positive multiple of %d'
                          % ALIGN)
     nb = len(counts)
+    ends = np.cumsum(np.asarray(counts, dtype=np.int64))
+    cuts = [set() for _ in range(nb)]
+    targets = (np.arange(1, grid) * (int(ends[-1]) if nb else 0)) // grid
+    firsts = np.zeros(grid + 1, dtype=np.int64)   # first particle of a CTA
+    for g, t in enumerate(targets.tolist(), 1):
+        b = int(np.searchsorted(ends, t, side='right'))
+        if b == nb:
+            firsts[g] = t
+            continue
+        at = (t - int(ends[b]) + int(counts[b])) // tile * tile
+        cuts[b].add(at)
+        firsts[g] = int(ends[b]) - int(counts[b]) + at
     units = []
     for b in range(nb):
         n = int(counts[b])
-        for s in range(0, n, unit_particles):
-            units.append((int(offsets[b]) + s,
-                          int(offsets[b]) + min(s + unit_particles, n), b))
+        at = sorted(cuts[b].union(range(0, n, unit_particles)) | {n})
+        for s, e in zip(at[:-1], at[1:]):
+            units.append((int(offsets[b]) + s, int(offsets[b]) + e, b))
     units = np.array(units, dtype=np.int64).reshape(-1, 3)
     nu = len(units)
     sizes = units[:, 1] - units[:, 0] if nu else np.zeros(0, np.int64)
-    total = int(sizes.sum())
-    # cut the unit sequence where the running particle count crosses g/grid
     cta_first = np.zeros(grid + 1, dtype=np.int32)
     if nu:
         before = np.concatenate(([0], np.cumsum(sizes)[:-1]))
-        targets = (np.arange(1, grid) * total) // grid
-        cta_first[1:grid] = np.searchsorted(before, targets, side='left')
+        cta_first[1:grid] = np.searchsorted(before, firsts[1:grid],
+                                            side='left')
     cta_first[grid] = nu
     column = np.zeros(nu, dtype=np.int32)
     bunch_columns = np.zeros(nb + 1, dtype=np.int32)
@@ -411,7 +425,7 @@ class BatchedTurn(object):
         sm = torch.cuda.get_device_properties(bt.device).multi_processor_count
         cps = int(config.get('ctas_per_sm', 0))
         grid = max_g if cps <= 0 else min(max_g, cps * sm)
-        plan = plan_units(bt.offsets, bt.counts, grid, unit)
+        plan = plan_units(bt.offsets, bt.counts, grid, unit, tile)
         dev = bt.device
         p = {'threads': threads, 'grid': grid, 'plan': plan,
              'units': unit_table(plan, dev),
