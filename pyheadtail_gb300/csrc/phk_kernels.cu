@@ -74,7 +74,9 @@ int launch_track(const phk_program* prog, const phk_coords* c,
 // ===================================================================
 
 // Fixed-order sum of the partial columns [g0, g1) of slice s (P laid out
-// [3][S][G]) and the finalised outputs; all 32 lanes of the warp call it.
+// [3][S][G]) and the finalised outputs, by LANES adjacent lanes (`lane` of
+// them); all 32 lanes of the warp call it.
+template <int LANES>
 __device__ __forceinline__ void merge_slice(const double* __restrict__ P,
                                             int S, int G, int s, int g0,
                                             int g1, int32_t* counts,
@@ -87,15 +89,15 @@ __device__ __forceinline__ void merge_slice(const double* __restrict__ P,
     // combined in a fixed order: the result does not depend on timing
     double c[4] = {0, 0, 0, 0}, sx[4] = {0, 0, 0, 0}, sy[4] = {0, 0, 0, 0};
     int g = g0 + lane;
-    for (; g + 96 < g1; g += 128) {
+    for (; g + 3 * LANES < g1; g += 4 * LANES) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            c[u] += pc[g + 32 * u];
-            sx[u] += px[g + 32 * u];
-            sy[u] += py[g + 32 * u];
+            c[u] += pc[g + LANES * u];
+            sx[u] += px[g + LANES * u];
+            sy[u] += py[g + LANES * u];
         }
     }
-    for (; g < g1; g += 32) {
+    for (; g < g1; g += LANES) {
         c[0] += pc[g];
         sx[0] += px[g];
         sy[0] += py[g];
@@ -104,7 +106,7 @@ __device__ __forceinline__ void merge_slice(const double* __restrict__ P,
     double tx = (sx[0] + sx[1]) + (sx[2] + sx[3]);
     double ty = (sy[0] + sy[1]) + (sy[2] + sy[3]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = LANES / 2; o > 0; o >>= 1) {
         tc += __shfl_xor_sync(0xffffffffu, tc, o);
         tx += __shfl_xor_sync(0xffffffffu, tx, o);
         ty += __shfl_xor_sync(0xffffffffu, ty, o);
@@ -131,7 +133,7 @@ __global__ void finalize_kernel(const double* __restrict__ P, int S, int G,
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp >= S) return;
-    merge_slice(P, S, G, warp, 0, G, counts, mean_x, mean_y, moments, lane);
+    merge_slice<32>(P, S, G, warp, 0, G, counts, mean_x, mean_y, moments, lane);
 }
 
 int launch_finalize(const phk_accum* acc, int32_t* counts, double* mean_x,
@@ -322,31 +324,6 @@ __device__ __forceinline__ void wake_conv_one(const phk_wake_set& w, int gw,
         else
             reinterpret_cast<float*>(kk.out)[i] = (float)r;
     }
-}
-
-// dot-product path of the batched wake: one thread per (kick, target slice);
-// coalesced over i
-__device__ __forceinline__ void wake_dense_one(const phk_wake_set& w, int t) {
-    const int S = w.n_slices;
-    const int k = t / S;
-    const int i = t - k * S;
-    if (k >= w.n_kicks) return;
-    const phk_wake_kick& kk = w.kick[k];
-    if (!kk.dense) return;
-    double acc = 0.0;
-    for (int a = 0; a < kk.n_lags; ++a) {
-        const int slot = ((w.head - a) % w.ring_len + w.ring_len) % w.ring_len;
-        const double* m = w.moments + ((int64_t)slot * 3 + kk.source) * S;
-        const double* W = kk.table + (int64_t)a * S * S;
-        double part = 0.0;
-        for (int j = 0; j < S; ++j) part = fma(m[j], W[(int64_t)j * S + i], part);
-        acc = add(acc, part);
-    }
-    const double r = mul(kk.factor, acc);
-    if (w.out_dtype == PHK_F64)
-        reinterpret_cast<double*>(kk.out)[i] = r;
-    else
-        reinterpret_cast<float*>(kk.out)[i] = (float)r;
 }
 
 // Single-bunch numpy path, little work: one CTA of kDirectWarps warps per (kick, target
@@ -605,26 +582,32 @@ int batch_max_grid(int32_t dtype, int32_t threads, int32_t S, int32_t nk) {
     return per_sm * device_info().sm_count;
 }
 
+// LANES lanes per (bunch, slice).  Bound by FP64 (about 20 cycles per warp
+// instruction and SM): with a warp per slice, its 15 shuffled additions, two
+// divisions and conversions were 256000 warp instructions at 64 bunches of
+// 100 slices; four lanes share them among eight slices (25 to 9.4 us).
+template <int LANES>
 __global__ void batch_finalize_kernel(const double* __restrict__ P, int S,
                                       int G, int nb,
                                       const int32_t* __restrict__ bcols,
                                       int32_t* counts, double* mean_x,
                                       double* mean_y, double* moments,
                                       int64_t mstride, int32_t* status) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const int bunch = warp / S;
-    const int s = warp - bunch * S;
-    if (bunch >= nb) return;
+    const int64_t group = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+    const int lane = threadIdx.x & (LANES - 1);
+    const bool on = group < (int64_t)nb * S;     // the warp's shuffles need all
+    const int bunch = on ? (int)(group / S) : 0;
+    const int s = on ? (int)(group - (int64_t)bunch * S) : 0;
     int g0 = bcols[bunch], g1 = bcols[bunch + 1];
     if (g0 < 0 || g1 > G || g0 > g1) {
         if (lane == 0 && status) atomicMax(status, PHK_DEV_BAD_TABLE);
         g0 = g1 = 0;
     }
     const int64_t o = (int64_t)bunch * S;
-    merge_slice(P, S, G, s, g0, g1, counts ? counts + o : nullptr,
-                mean_x ? mean_x + o : nullptr, mean_y ? mean_y + o : nullptr,
-                moments ? moments + bunch * mstride : nullptr, lane);
+    merge_slice<LANES>(P, S, G, s, g0, g1, counts && on ? counts + o : nullptr,
+                       mean_x && on ? mean_x + o : nullptr,
+                       mean_y && on ? mean_y + o : nullptr,
+                       moments && on ? moments + bunch * mstride : nullptr, lane);
 }
 
 int launch_batch_finalize(const phk_accum* acc, int nb, const int32_t* bcols,
@@ -632,12 +615,15 @@ int launch_batch_finalize(const phk_accum* acc, int nb, const int32_t* bcols,
                           double* moments, int64_t mstride, int32_t* status,
                           cudaStream_t st) {
     const int S = acc->slicer.n_slices;
-    const int64_t warps = (int64_t)nb * S;
-    const int threads = 256;
-    const int64_t blocks = (warps * 32 + threads - 1) / threads;
-    batch_finalize_kernel<<<(unsigned)blocks, threads, 0, st>>>(
-        acc->partials, S, acc->grid, nb, bcols, counts, mean_x, mean_y,
-        moments, mstride, status);
+    // four lanes while a bunch has at most 64 columns on average (up to 16
+    // terms a lane); a warp where bunches span more of the grid
+    const int lanes = acc->grid <= 64 * (int64_t)nb ? 4 : 32;
+    const int threads = 128;
+    const int64_t blocks = ((int64_t)nb * S * lanes + threads - 1) / threads;
+    auto kern = lanes == 4 ? batch_finalize_kernel<4> : batch_finalize_kernel<32>;
+    kern<<<(unsigned)blocks, threads, 0, st>>>(acc->partials, S, acc->grid, nb, bcols,
+                                               counts, mean_x, mean_y, moments,
+                                               mstride, status);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return set_error(PHK_ECUDA, "phk_batch_finalize launch: %s",
@@ -646,33 +632,73 @@ int launch_batch_finalize(const phk_accum* acc, int nb, const int32_t* bcols,
     return PHK_OK;
 }
 
-// one warp per (bunch, kick, target slice), numpy path; one thread per
-// (bunch, kick, target slice), dot-product path
-__global__ void batch_wake_kernel(const phk_wake_set* __restrict__ sets,
-                                  int nb, int S, int nk) {
-    const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const int per = nk * S;
-    const int64_t bunch = gw / per;
-    if (bunch >= nb) return;
+// One CTA per (bunch, kick, 32 target slices): lanes are targets, the warps
+// split the sources of every stored turn, four sums in flight each; fixed
+// order.  Bound by FP64: a warp per target spent 9 of its 13 additions on
+// adding its lanes up (64 bunches, 2 kicks, 100 slices: 19 us, now 9.2).  Above
+// kBatchTerms terms per target that share is small, and the lane-split sums
+// (wake_conv_one) have the shorter chains: those targets go one to a warp.
+constexpr int kBatchWarps = 8;
+constexpr int kBatchTerms = 512;
+
+__global__ void __launch_bounds__(kBatchWarps * 32)
+batch_wake_kernel(const phk_wake_set* __restrict__ sets, int nb, int S, int nk) {
+    __shared__ double part[kBatchWarps][32];
+    const int blocks = (S + 31) / 32;
+    const int bunch = blockIdx.x / (nk * blocks);
+    const int r = blockIdx.x - bunch * nk * blocks;
+    const int k = r / blocks, i0 = (r - k * blocks) * 32;
     const phk_wake_set& w = sets[bunch];
     if (w.n_slices != S || w.n_kicks > nk || w.n_kicks < 0 ||
         w.ring_len < 1 || w.head < 0 || w.head >= w.ring_len)
         return;
-    const int r = (int)(gw - bunch * per);
-    wake_conv_one(w, r, lane);
-    // dense kicks: the warp's lanes take target slices r*32+lane of the
-    // warp-major numbering (warps [0, per/32] cover all nk*S targets)
-    const int t = r * 32 + lane;
-    if (t < per) wake_dense_one(w, t);
+    if (k >= w.n_kicks) return;
+    const phk_wake_kick& kk = w.kick[k];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (!kk.dense && (int64_t)kk.n_lags * S > kBatchTerms) {
+        for (int i = i0 + warp; i < i0 + 32 && i < S; i += kBatchWarps)
+            wake_conv_one(w, k * S + i, lane);
+        return;
+    }
+    const int i = i0 + lane < S ? i0 + lane : S - 1;
+    const int j0 = S * warp / kBatchWarps, j1 = S * (warp + 1) / kBatchWarps;
+    // the sample of source j: numpy path table[i + S - 1 - j], dot path [j][i]
+    const int64_t row = kk.dense ? (int64_t)S * S : 2 * S - 1;
+    const int64_t dj = kk.dense ? S : -1;
+    const double* v = kk.table + i + (kk.dense ? 0 : S - 1);
+    double p[4] = {0.0, 0.0, 0.0, 0.0};
+    int slot = (w.head % w.ring_len + w.ring_len) % w.ring_len;
+    for (int a = 0; a < kk.n_lags; ++a, v += row) {
+        const double* m = w.moments + ((int64_t)slot * 3 + kk.source) * S;
+        int j = j0;
+        for (; j + 3 < j1; j += 4)
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                p[u] = fma(__ldg(m + j + u), __ldg(v + (j + u) * dj), p[u]);
+        for (; j < j1; ++j) p[0] = fma(__ldg(m + j), __ldg(v + j * dj), p[0]);
+        slot = slot == 0 ? w.ring_len - 1 : slot - 1;
+    }
+    part[warp][lane] = (p[0] + p[1]) + (p[2] + p[3]);
+    __syncthreads();
+    if (warp != 0 || i0 + lane >= S) return;
+    double t[kBatchWarps];
+#pragma unroll
+    for (int q = 0; q < kBatchWarps; ++q) t[q] = part[q][lane];
+#pragma unroll
+    for (int d = kBatchWarps / 2; d > 0; d >>= 1)
+#pragma unroll
+        for (int q = 0; q < d; ++q) t[q] = add(t[q], t[q + d]);
+    const double res = mul(kk.factor, t[0]);
+    if (w.out_dtype == PHK_F64)
+        reinterpret_cast<double*>(kk.out)[i] = res;
+    else
+        reinterpret_cast<float*>(kk.out)[i] = (float)res;
 }
 
 int launch_wake_batch(const phk_wake_set* sets, int nb, int S, int nk,
                       cudaStream_t st) {
-    const int64_t warps = (int64_t)nb * nk * S;
-    const int threads = 256;
-    const int64_t blocks = (warps * 32 + threads - 1) / threads;
-    batch_wake_kernel<<<(unsigned)blocks, threads, 0, st>>>(sets, nb, S, nk);
+    const int64_t blocks = (int64_t)nb * nk * ((S + 31) / 32);
+    batch_wake_kernel<<<(unsigned)blocks, kBatchWarps * 32, 0, st>>>(sets, nb, S, nk);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return set_error(PHK_ECUDA, "phk_wake_batch launch: %s",
