@@ -127,21 +127,22 @@ __device__ __forceinline__ void merge_slice(const double* __restrict__ P,
     }
 }
 
+// One warp, one CTA per slice.  Bound by FP64, 64 instructions of 20 cycles
+// for a slice, so the slices are spread over the SMs: eight to a CTA kept 7 of
+// them busy at 50 slices and 63 at 500 (50 slices: 9.4 us, now 6.9 from cold
+// caches; 16 or 8 lanes per slice have fewer instructions but longer chains: 200
+// slices, the whole turn 42.2 and 43.5 us against 41.3).
 __global__ void finalize_kernel(const double* __restrict__ P, int S, int G,
                                 int32_t* counts, double* mean_x,
                                 double* mean_y, double* moments) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= S) return;
-    merge_slice<32>(P, S, G, warp, 0, G, counts, mean_x, mean_y, moments, lane);
+    merge_slice<32>(P, S, G, blockIdx.x, 0, G, counts, mean_x, mean_y, moments,
+                    threadIdx.x);
 }
 
 int launch_finalize(const phk_accum* acc, int32_t* counts, double* mean_x,
                     double* mean_y, double* moments, cudaStream_t st) {
     const int S = acc->slicer.n_slices;
-    const int threads = 256;
-    const int blocks = (S * 32 + threads - 1) / threads;
-    finalize_kernel<<<blocks, threads, 0, st>>>(acc->partials, S, acc->grid,
+    finalize_kernel<<<S, 32, 0, st>>>(acc->partials, S, acc->grid,
                                                 counts, mean_x, mean_y,
                                                 moments);
     const cudaError_t e = cudaGetLastError();
@@ -356,15 +357,19 @@ wake_direct_kernel(const __grid_constant__ phk_wake_set w) {
         }
         for (; j < S; j += 32) p0 = fma(__ldg(m + j), __ldg(v - j), p0);
     }
-    double part = (p0 + p1) + (p2 + p3);
+    if (warp < kk.n_lags) {             // warps without a turn add nothing up
+        double part = (p0 + p1) + (p2 + p3);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0) part_w[warp] = part;
+        for (int o = 16; o > 0; o >>= 1)
+            part += __shfl_xor_sync(0xffffffffu, part, o);
+        if (lane == 0) part_w[warp] = part;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double acc = part_w[0];
-        for (int q = 1; q < kDirectWarps; ++q) acc += part_w[q];
+        const int turns = kk.n_lags < kDirectWarps ? kk.n_lags : kDirectWarps;
+        double acc = 0.0;
+        if (turns > 0) acc = part_w[0];
+        for (int q = 1; q < turns; ++q) acc += part_w[q];
         const double r = mul(kk.factor, acc);
         if (w.out_dtype == PHK_F64)
             reinterpret_cast<double*>(kk.out)[i] = r;
