@@ -1646,7 +1646,12 @@ __device__ __forceinline__ void load_tile_plain(const TrackArgs& a,
     }
 }
 
-// CTAs per thread-block cluster of an accumulating launch
+// CTAs per thread-block cluster of an accumulating launch.  The cluster's
+// barrier releases and acquires at cluster scope (its default), global memory
+// included, and only the cluster touches its partial column until the kernel
+// ends: no fence of the whole device is needed beside it.  Two of those waited
+// for the particles' stores: 1.5 us of a pass (100000 particles of FP64, the
+// turn 26.3 to 24.8 us; 1e6 of FP32, 39.1 to 37.3 us).
 constexpr int kCluster = 4;
 
 // FP32 single-bunch kernel: particles per thread, resident CTAs per SM it
@@ -1830,9 +1835,8 @@ track_kernel(const __grid_constant__ phk_program prog,
         }
         unsigned M[2];
         if (clustered) {
-            __threadfence();
             cg::cluster_group cl = cg::this_cluster();
-            cl.sync();
+            cl.sync();                   // orders the clears, see kCluster
             M[0] = M[1] = 0u;
             for (unsigned r = 0; r < cl.num_blocks(); ++r) {
                 const unsigned* sm = cl.map_shared_rank(s_max, r);
@@ -1958,7 +1962,7 @@ track_kernel(const __grid_constant__ phk_program prog,
     // integers and writes the partial column in FP64
     unsigned nb = 1;
     if (clustered) {
-        __threadfence();                 // level-B adds before the barrier
+        // level-B adds before the barrier (see kCluster)
         cg::cluster_group cl = cg::this_cluster();
         cl.sync();
         nb = cl.num_blocks();

@@ -157,9 +157,8 @@ track64_kernel(const __grid_constant__ phk_program prog,
             for (int s = tid; s < 2 * Sa; s += kTrackThreads) PL[(Sa + s) * G] = 0;
         unsigned M[2];
         if (clustered) {
-            __threadfence();
             cg::cluster_group cl = cg::this_cluster();
-            cl.sync();
+            cl.sync();                   // orders the clears, see kCluster
             M[0] = M[1] = ~0u;
             for (unsigned r = 0; r < cl.num_blocks(); ++r) {
                 const unsigned* sm = cl.map_shared_rank(s_typ, r);
@@ -199,7 +198,7 @@ track64_kernel(const __grid_constant__ phk_program prog,
     unsigned nb = 1;
     int any = 0;
     if (clustered) {
-        __threadfence();                 // adds to the column before the barrier
+        // adds to the column before the barrier (see kCluster)
         cg::cluster_group cl = cg::this_cluster();
         cl.sync();
         nb = cl.num_blocks();
