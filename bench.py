@@ -304,7 +304,7 @@ def profile_traffic(kernel_key):
     return d.get(kernel_key)
 
 
-def last_launch():
+def last_launch(precision='fp32'):
     """Kernel, ring stages and shared memory of the last fused pass."""
     import ctypes
     from pyheadtail_gb300 import _native as N
@@ -312,6 +312,7 @@ def last_launch():
     N.call('phk_last_track_launch', ctypes.byref(v), ctypes.byref(s),
            ctypes.byref(m))
     return {'kernel': 'phk::stream_kernel' if v.value == 1
+            else 'phk::track64_kernel' if precision == 'fp64'
             else 'phk::track_kernel', 'stages': s.value,
             'smem_bytes': m.value}
 
@@ -389,7 +390,7 @@ def _time_form(w, coords, precision, steps, warmup, flush, tune):
     evs = beam._engine.track_events
     beam._engine.track_events = None
     track_ms = [a.elapsed_time(b) for a, b in evs]
-    launch = dict(last_launch(), tuned=tune)
+    launch = dict(last_launch(precision), tuned=tune)
     if tune:
         from pyheadtail_gb300 import tuning
         tuned = list(tuning.timings().values())
@@ -511,7 +512,7 @@ def run_eager(a):
         evs = beam._engine.track_events or []
         print(json.dumps({'form': precision, 'turns': a.eager_turns,
                           'track_ms': [x.elapsed_time(y) for x, y in evs],
-                          'launch': last_launch(),
+                          'launch': last_launch(precision),
                           'tuning': tuning.timings()
                           if tuning.enabled() else None,
                           'mean_x': float(beam.mean_x())}))
@@ -558,9 +559,10 @@ def run_ours(a, rank, world):
                          'kernel': r['launch']['kernel'],
                          'kernel_ms': track_avg,
                          'algorithmic_bytes_per_launch': bytes_pp * w['n'],
-                         'note': ('HBM fraction of a kernel bound by the FP64 '
-                                  'pipe (GB300 runs FP64 at 1/59 of the FP32 '
-                                  'rate); forms.fp32 is the HBM-bound form'
+                         'note': ('HBM fraction of a kernel bound by '
+                                  'arithmetic (GB300 runs FP64 at 1/59 of the '
+                                  'FP32 rate; products in 64-bit integers); '
+                                  'forms.fp32 is the HBM-bound form'
                                   if precision == 'fp64' else
                                   'HBM-bound form')},
             'e2e': {'value': w['n'] * r['e2e_turns_per_step'] *
