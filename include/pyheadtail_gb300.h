@@ -229,9 +229,10 @@ typedef struct phk_kick_set {
 
 /* ---- per-slice accumulation (Slicer.slice + add_statistics for the
  * dipole moments: slicing.py:348-381, 443-470; stats.pyx:192-253).
- * An accumulating phk_track runs `grid` thread-block clusters; each cluster
- * folds its CTAs' histograms through distributed shared memory and writes
- * its per-slice count / sum x / sum y to the partial column
+ * An accumulating phk_track runs `grid` thread-block clusters (of one CTA in
+ * the FP64 form, unless there are fewer columns than SMs); each cluster folds
+ * its CTAs' histograms through distributed shared memory and writes its
+ * per-slice count / sum x / sum y to the partial column
  * partials[q * n_slices * grid + s * grid + column] (q = 0,1,2).  Use
  * phk_track_grid() for `grid`; size partials >= 3 * n_slices * grid.
  * Reproducibility: values are summed as integers in a power-of-two unit per

@@ -43,12 +43,14 @@ int track_grid(int64_t n, int32_t dtype, int32_t n_slices) {
     // largest shared-memory layout of a turn)
     const size_t smem = track_smem_bytes(dtype, n_slices, n_slices);
     const int vec = dtype == PHK_F64 ? 1 : kF32Vec;
-    const int nc = dtype == PHK_F64 ? track_clusters_f64(smem)
+    // FP64: a column per CTA; FP32: a column per cluster
+    const int cluster = dtype == PHK_F64 ? 1 : kCluster;
+    const int nc = dtype == PHK_F64 ? track_ctas_f64(smem)
                                     : track_clusters_f32(smem);
     const int64_t tiles = (n + (int64_t)kTrackThreads * vec - 1) /
                           ((int64_t)kTrackThreads * vec);
     int64_t g = nc;
-    const int64_t need = (tiles + kCluster - 1) / kCluster;
+    const int64_t need = (tiles + cluster - 1) / cluster;
     if (need < g) g = need;
     if (g < 1) g = 1;
     return (int)g;

@@ -1646,12 +1646,13 @@ __device__ __forceinline__ void load_tile_plain(const TrackArgs& a,
     }
 }
 
-// CTAs per thread-block cluster of an accumulating launch.  The cluster's
+// CTAs per thread-block cluster of an accumulating FP32 launch (FP64: see
+// launch_track64_t).  The cluster's
 // barrier releases and acquires at cluster scope (its default), global memory
 // included, and only the cluster touches its partial column until the kernel
 // ends: no fence of the whole device is needed beside it.  Two of those waited
-// for the particles' stores: 1.5 us of a pass (100000 particles of FP64, the
-// turn 26.3 to 24.8 us; 1e6 of FP32, 39.1 to 37.3 us).
+// for the particles' stores: 1.8 us of a pass (1e6 particles, the turn 39.1 to
+// 37.3 us).
 constexpr int kCluster = 4;
 
 // FP32 single-bunch kernel: particles per thread, resident CTAs per SM it
@@ -2645,7 +2646,7 @@ int launch_track_f64(const phk_program* prog, const phk_coords* c,
                      const phk_kick_set* pk, const phk_accum* acc, int ld,
                      int stm, bool vec_ok, cudaStream_t st);
 int track_clusters_f32(size_t smem);
-int track_clusters_f64(size_t smem);
+int track_ctas_f64(size_t smem);
 int launch_batch_f32(const phk_batch* bt, const phk_coords* c,
                      const phk_kick_set* pk, const phk_accum* acc, int ld,
                      int stm, cudaStream_t st);

@@ -351,11 +351,19 @@ static int launch_track64_t(const phk_program* prog, const phk_coords* c,
     cfg.stream = st;
     cudaLaunchAttribute attr;
     if (acc) {
-        // one partial column per cluster of kCluster CTAs
-        a.cluster = kCluster;
-        cfg.gridDim = dim3((unsigned)acc->grid * kCluster, 1, 1);
+        // One partial column per CTA: folding four CTAs into a column costs two
+        // cluster barriers, and only 440 of 456 CTAs found room (a turn with
+        // linear maps of 1e5 macroparticles at 50 / 500 / 1000 slices 24.8 / 63 /
+        // 97 us, now 22.8 / 37 / 53; 1e7 with RF and a 50-turn wake 371 us, now
+        // 354).  A caller with fewer columns than SMs and tiles (the
+        // workspace-free pass) gets clusters of kCluster CTAs per column.
+        // Launched as clusters of one too: their CTAs are spread better than
+        // those of a plain launch (1e6 with detuning 90.1 / 92.2 us).
+        const int64_t sms = device_info().sm_count;
+        a.cluster = acc->grid < (a.n_tiles < sms ? a.n_tiles : sms) ? kCluster : 1;
+        cfg.gridDim = dim3((unsigned)acc->grid * a.cluster, 1, 1);
         attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = kCluster;
+        attr.val.clusterDim.x = a.cluster;
         attr.val.clusterDim.y = 1;
         attr.val.clusterDim.z = 1;
         cfg.attrs = &attr;
@@ -378,28 +386,18 @@ static int launch_track64_t(const phk_program* prog, const phk_coords* c,
     return PHK_OK;
 }
 
-// clusters of kCluster CTAs that can be resident at once
+// CTAs that can be resident at once (clusters of one)
 template <int VEC, int SHAPE>
-static int track64_clusters(size_t smem) {
+static int track64_ctas(size_t smem) {
     track64_limit<VEC, SHAPE>();
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kCluster * device_info().sm_count, 1, 1);
-    cfg.blockDim = dim3(kTrackThreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = kCluster;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, track64_kernel<VEC, SHAPE>, &cfg) !=
-            cudaSuccess || n < 1) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &n, track64_kernel<VEC, SHAPE>, kTrackThreads, smem) != cudaSuccess ||
+        n < 1) {
         cudaGetLastError();
-        n = device_info().sm_count / kCluster;
+        n = 1;
     }
-    return n < 1 ? 1 : n;
+    return n * device_info().sm_count;
 }
 
 }  // namespace phk

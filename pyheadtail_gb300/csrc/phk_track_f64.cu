@@ -35,8 +35,8 @@ int launch_track_f64(const phk_program* prog, const phk_coords* c,
     }
 }
 
-int track_clusters_f64(size_t smem) {
-    return track64_clusters<1, SHAPE_GENERIC>(smem);
+int track_ctas_f64(size_t smem) {
+    return track64_ctas<1, SHAPE_GENERIC>(smem);
 }
 
 // common program shape of every bunch of a batch (GENERIC unless all equal
