@@ -170,6 +170,99 @@ __device__ __forceinline__ double fix64_value(long long L1, long long d2,
 }
 
 // -------------------------------------------------------------------
+// Exact sums of doubles as fixed-point integers.
+//
+// A value u = w 2^(e - 1075) (w: its 53-bit significand, e: its biased
+// exponent) is the integer w 2^(e - base) of at most 78 bits and a sign, where
+// base <= e <= base + 25; it is split into three unsigned 20-bit digits and
+// the signed rest, added to 32-bit counters.  Nothing is rounded, so the sum
+// of such values is exact and does not depend on their order.  Every other
+// value (smaller than 2^-18 or more than 2^7 times the typical value that
+// sets the base, subnormal, infinite, NaN) is left to the caller, who adds it
+// in FP64: a sum is never less accurate than a floating-point loop's.
+// A window of 64 bits that truncates what lies below it is a digit's work
+// cheaper but loses the slices whose values are all small.
+// -------------------------------------------------------------------
+constexpr int kFix80Values = 4095;      // at most, between two carries
+constexpr int kFix80None = 1 << 16;     // base: no value is representable
+
+// base for a typical magnitude, given as the high word of the double (sign
+// cleared; 0 or ~0: none seen)
+__device__ __forceinline__ int fix80_base(unsigned mhi) {
+    if (mhi == 0u || mhi == ~0u) return kFix80None;
+    const int e = (int)(mhi >> 20);
+    return (e < 100 ? 100 : (e > 2000 ? 2000 : e)) - 18;
+}
+
+// adds u to the four digits at d (shared memory); false if it is not
+// representable (zeros add nothing)
+__device__ __forceinline__ bool fix80_add(int* d, int base, double u) {
+    const int hi = __double2hiint(u);
+    const unsigned wl = (unsigned)__double2loint(u);
+    if ((((unsigned)hi << 1) | wl) == 0u) return true;
+    const int s = biased_exp(hi) - base;
+    if ((unsigned)s > 25u) return false;
+    const unsigned wh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+    unsigned v0 = wl << s, v1 = __funnelshift_l(wl, wh, s), v2 = (wh >> 7) >> (25 - s);
+    if (hi < 0) {
+        v2 = ~v2 + ((v0 | v1) == 0u ? 1u : 0u);
+        v1 = ~v1 + (v0 == 0u ? 1u : 0u);
+        v0 = 0u - v0;
+    }
+    atomicAdd(d, (int)(v0 & 0xfffffu));
+    atomicAdd(d + 1, (int)(__funnelshift_r(v0, v1, 20) & 0xfffffu));
+    atomicAdd(d + 2, (int)((v1 >> 8) & 0xfffffu));
+    atomicAdd(d + 3, (int)__funnelshift_r(v1, v2, 28));
+    return true;
+}
+
+// carries the digits at d upwards, at least every kFix80Values values; a top
+// digit that might overflow before the next carry is taken out and returned
+// (in units of 2^60)
+__device__ __forceinline__ int fix80_carry(int* d) {
+    u64 c = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        c += (unsigned)d[i];
+        d[i] = (int)((unsigned)c & 0xfffffu);
+        c >>= 20;
+    }
+    const int top = d[3] + (int)c;
+    const int out = top >= (1 << 30) || top <= -(1 << 30) ? top : 0;
+    d[3] = top - out;
+    return out;
+}
+
+// the FP64 value of the digits at d and of a carried-out top digit
+__device__ __forceinline__ double fix80_scale(int base) {
+    return __hiloint2double(((base == kFix80None ? 1023 : base) - 52) << 20, 0);
+}
+__device__ __forceinline__ double fix80_value(const int* d, int base) {
+    const long long h = (long long)d[3] * (1 << 20) + (unsigned)d[2];
+    const long long l = ((long long)(unsigned)d[1] << 20) + (unsigned)d[0];
+    return fma((double)h, 0x1p40, (double)l) * fix80_scale(base);
+}
+__device__ __forceinline__ double fix80_top(int top, int base) {
+    return (double)top * 0x1p60 * fix80_scale(base);
+}
+
+// Particle t (0 .. THREADS - 1) of a sample of those that this CTA works on,
+// the tiles blockIdx.x, blockIdx.x + gridDim.x, ... of TILE particles; -1 if
+// it has none.  A warp's 32 are spread over all of them: in a bunch that is
+// ordered by a coordinate, a tile is no sample.
+template <int THREADS, int TILE>
+__device__ __forceinline__ int64_t own_sample(int t, int64_t n) {
+    const int64_t tiles = (n + TILE - 1) / TILE;
+    if ((int64_t)blockIdx.x >= tiles) return -1;
+    const int64_t own = (tiles - 1 - blockIdx.x) / gridDim.x + 1;
+    const int64_t last = blockIdx.x + (own - 1) * gridDim.x;
+    const int64_t live = n - last * TILE;
+    const int64_t count = (own - 1) * TILE + (live < TILE ? live : TILE);
+    const int64_t j = ((t & 31) * (THREADS / 32) + (t >> 5)) * count / THREADS;
+    return ((int64_t)blockIdx.x + j / TILE * gridDim.x) * TILE + j % TILE;
+}
+
+// -------------------------------------------------------------------
 // Sine and cosine of 2 pi F 2^-64, F an unsigned 64-bit fraction of a turn
 // (the integer turns drop out by themselves), in units of 2^-62.
 //

@@ -2,11 +2,11 @@
 // phk_slice_moments_all): the sums behind every statistic of a slice, two
 // passes over the particles (sums and counts, then centred products).
 //
-// The values are summed per CTA as 64-bit fixed-point digits in shared memory
-// (fix64_add; the unit of each value from the CTA's first tile) and the CTA
-// adds its totals to the caller's FP64 arrays, one global atomic per slice
-// and value; a value outside the fixed point's range (more than 32 times the
-// typical one, infinite, NaN) is added there on its own.  Before, every
+// The values are summed per CTA as exact fixed-point digits in shared memory
+// (fix80_add; the window of each value from a sample of the CTA's particles)
+// and the CTA adds its totals to the caller's FP64 arrays, one global atomic
+// per slice and value; a value outside the window (2^7 times the typical one,
+// 2^-18 of it, infinite, NaN) is added there on its own.  Before, every
 // particle's value was a global FP64 atomic, one launch pair per statistic:
 // 22 launches of 220 us for all statistics of 1e6 particles in 200 slices,
 // now two.  The integer work and the shared-memory atomics bound it (52
@@ -108,11 +108,11 @@ moments_kernel(const __grid_constant__ phk_slicer sl, const __grid_constant__ Mo
         return s;
     };
 
-    // ---- the unit of every value: of the largest magnitude of each warp in
-    // the first tile, the smallest
-    int64_t i = (int64_t)blockIdx.x * kMomThreads + tid;
+    // ---- the window of every value: of the largest magnitude of each warp's
+    // sample, the smallest.  Particles outside the cuts count as zeros.
     double v[NV];
-    int s = values(i, v);
+    int64_t i = own_sample<kMomThreads, kMomThreads>(tid, a.n);
+    int s = values(i < 0 ? a.n : i, v);
 #pragma unroll
     for (int p = 0; p < NV; ++p) {
         const unsigned b = (unsigned)__double2hiint(v[p]) & 0x7fffffffu;
@@ -120,51 +120,46 @@ moments_kernel(const __grid_constant__ phk_slicer sl, const __grid_constant__ Mo
         if ((tid & 31) == 0 && m) atomicMin(&s_typ[p], m);
     }
     __syncthreads();
-    int k[NV];
+    int base[NV];
 #pragma unroll
-    for (int p = 0; p < NV; ++p) k[p] = fix64_k(s_typ[p]);
-
-    // this CTA's totals to the caller's sums
-    auto flush = [&]() {
-        __syncthreads();
-        for (int j = tid; j < S * NV; j += kMomThreads) {
-            const int p = j / S, sj = j - p * S;
-            unsigned* d = reinterpret_cast<unsigned*>(words) + sj * W + D0 + 4 * p;
-            const long long L1 = (long long)d[0] + ((long long)d[1] << 16);
-            const long long d2 = d[2], d3 = (int)d[3];
-            if (L1 | d2 | d3) {
-                atomicAdd(a.sums + j, fix64_value(L1, d2, d3, fix64_k(s_typ[p])));
-                d[0] = d[1] = d[2] = d[3] = 0u;
-            }
-        }
-        if (PASS == 0)
-            for (int sj = tid; sj < S; sj += kMomThreads)
-                if (words[sj * W]) {
-                    atomicAdd(a.counts + sj, words[sj * W]);
-                    words[sj * W] = 0;
-                }
-        __syncthreads();
-    };
+    for (int p = 0; p < NV; ++p) base[p] = fix80_base(s_typ[p]);
 
     const int64_t step = (int64_t)gridDim.x * kMomThreads;
     const int64_t rounds = (a.n + step - 1) / step;
-    for (int64_t it = 0; it < rounds; ++it) {
-        if (it) s = values(i, v);
+    i = (int64_t)blockIdx.x * kMomThreads + tid;
+    for (int64_t it = 0; it < rounds; ++it, i += step) {
+        s = values(i, v);
         if (s >= 0) {
             int* w = words + s * W;
             if (PASS == 0) atomicAdd(a.in_smem ? w : a.counts + s, 1);
 #pragma unroll
             for (int p = 0; p < NV; ++p) {
                 if (PASS == 0 ? p < a.n_q : PAIRS::b(p) < a.n_q)
-                    if (!a.in_smem || !fix64_add(w + D0 + 4 * p, k[p], v[p]))
+                    if (!a.in_smem || !fix80_add(w + D0 + 4 * p, base[p], v[p]))
                         atomicAdd(a.sums + p * S + s, v[p]);
             }
         }
-        i += step;
-        // 2^16 values per counter at most
-        if (a.in_smem && (it + 1) % ((1 << 16) / kMomThreads) == 0) flush();
+        if (a.in_smem && (it + 1) % (kFix80Values / kMomThreads) == 0) {
+            __syncthreads();
+            for (int j = tid; j < S * NV; j += kMomThreads) {
+                const int p = j / S, sj = j - p * S;
+                const int top = fix80_carry(words + sj * W + D0 + 4 * p);
+                if (top) atomicAdd(a.sums + j, fix80_top(top, fix80_base(s_typ[p])));
+            }
+            __syncthreads();
+        }
     }
-    if (a.in_smem) flush();
+    if (!a.in_smem) return;
+    // ---- this CTA's totals to the caller's sums
+    __syncthreads();
+    for (int j = tid; j < S * NV; j += kMomThreads) {
+        const int p = j / S, sj = j - p * S;
+        const double t = fix80_value(words + sj * W + D0 + 4 * p, fix80_base(s_typ[p]));
+        if (t != 0.0) atomicAdd(a.sums + j, t);
+    }
+    if (PASS == 0)
+        for (int sj = tid; sj < S; sj += kMomThreads)
+            if (words[sj * W]) atomicAdd(a.counts + sj, words[sj * W]);
 }
 
 template <typename T, class PAIRS, int PASS>
