@@ -235,13 +235,14 @@ typedef struct phk_kick_set {
  * per-slice count / sum x / sum y to the partial column
  * partials[q * n_slices * grid + s * grid + column] (q = 0,1,2).  Use
  * phk_track_grid() for `grid`; size partials >= 3 * n_slices * grid.
- * Reproducibility: values are summed as integers in a power-of-two unit per
- * cluster (FP32: each value rounds by at most 2^-27 of the largest |value|
- * of the cluster's first tiles; FP64: by at most 2^-56 of a typical one),
- * so the columns are bit-identical on every launch and for every launch
- * plan.  FP64 slices that hold a value beyond 2^5 times the typical one, an
- * infinity or NaN are summed in FP64 through atomics; their last bits may
- * differ between launches.
+ * Accuracy and reproducibility: FP64 values are summed exactly by every CTA,
+ * as integers in a window around a typical |value| of its particles (2^-18 to
+ * 8 times it); values outside the window, infinities and NaN are added to the
+ * column in FP64 through atomics.  FP32 values are summed as integers at a
+ * power-of-two scale per cluster (each rounds by at most 2^-27 of the largest
+ * |value| of the cluster's first tiles).  The columns are the same bits on
+ * every launch with the same `grid`, but for slices with three or more values
+ * outside the FP64 window in one column: their last bits may differ.
  * idx_out (optional, int32[n]) receives the reference's slice index of
  * every particle (outside particles included; NaN -> INT32_MIN).        */
 typedef struct phk_accum {

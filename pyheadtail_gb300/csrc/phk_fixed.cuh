@@ -85,181 +85,160 @@ __device__ __forceinline__ Factor mul_factor(const Factor& a, const Factor& b) {
 }
 
 // -------------------------------------------------------------------
-// FixHist64: per-slice sums of FP64 coordinates as 64-bit fixed-point
-// integers, the FP64 counterpart of FixHist (phk_track.cuh).
+// Exact sums of doubles as fixed-point integers.
 //
-// Every thread-block cluster agrees on one unit per coordinate: of the
-// largest finite |u| of every warp's first values, the smallest (a single
-// stray value cannot coarsen the unit) maps to [2^56, 2^57).  A value
-// becomes the integer v = u / unit truncated toward zero (exact for |u|
-// down to 2^-3 of that typical value, off by at most 2^-56 of it otherwise:
-// below the rounding of the FP64 additions it replaces) and is split into
-// three unsigned 16-bit digits and the signed rest, added to 32-bit
-// shared-memory counters; 2^16 values per counter stay in range (a CTA
-// carries its counters into the cluster's column at least that often).
-// NaN, +-inf and |v| >= 2^62 (32 times the typical value) mark the slice
-// instead; the cluster then sums that slice's values again in FP64 at the
-// end of the pass, so any input gets the sum a floating-point loop would
-// give it.  Unmarked slices are integer sums, converted once: they are the
-// same bits on every launch.
+// A value u = w 2^(e - 1075) (w: its signed 53-bit significand, e: its biased
+// exponent) is the integer w 2^(e - base) of at most 74 bits and a sign, where
+// base <= e <= base + 21; it is split into three unsigned 19-bit digits and the
+// signed rest, added to 32-bit counters.  Nothing is rounded, so the sum of such
+// values is exact and does not depend on their order.  Every other value (far
+// from the typical value that sets the base, subnormal, infinite, NaN) is left
+// to the caller, who adds it in FP64: a sum is never less accurate than a
+// floating-point loop's.  (A 64-bit number that truncates what lies below its
+// unit took 5 cycles less of a warp's 41 per particle, but lost slices whose
+// values are all small.  Digits with the sign, by multiplication, are 2 cycles
+// shorter but hold half as many values, and the pass's multiply pipe is busier
+// than its logic pipe.)
+// -------------------------------------------------------------------
+constexpr int kDigitBits = 19;
+constexpr unsigned kDigitMask = (1u << kDigitBits) - 1u;
+constexpr int kWindow = 21;
+constexpr int kDigitValues = 8190;      // at most, between two carries
+constexpr int kNoBase = 1 << 16;        // no value is representable
+
+// base for a typical magnitude, given as the high word of the double (sign
+// cleared; 0: none seen): down to 2^-low of it
+__device__ __forceinline__ int digit_base(unsigned mhi, int low) {
+    if (mhi == 0u) return kNoBase;
+    const int e = (int)(mhi >> 20);
+    return (e < 100 ? 100 : (e > 2000 ? 2000 : e)) - low;
+}
+
+// adds u to the four digits at d (shared memory); false if it is not
+// representable
+__device__ __forceinline__ bool add_digits(int* d, int base, double u) {
+    const int hi = __double2hiint(u);
+    const unsigned wl = (unsigned)__double2loint(u);
+    const int s = biased_exp(hi) - base;
+    if ((unsigned)s > (unsigned)kWindow) return false;
+    const int sign = hi >> 31;
+    const long long w = ((((long long)((hi & 0xfffff) | 0x100000)) << 32 | wl) ^ sign) - sign;
+    const unsigned w0 = (unsigned)w;
+    const int w1 = (int)(w >> 32);
+    const unsigned v0 = w0 << s, v1 = __funnelshift_l(w0, (unsigned)w1, s);
+    const int v2 = (w1 >> (32 - kWindow)) >> (kWindow - s);
+    atomicAdd(d, (int)(v0 & kDigitMask));
+    atomicAdd(d + 1, (int)(__funnelshift_r(v0, v1, 19) & kDigitMask));
+    atomicAdd(d + 2, (int)((v1 >> 6) & kDigitMask));
+    atomicAdd(d + 3, (int)__funnelshift_r(v1, (unsigned)v2, 25));
+    return true;
+}
+
+// carries the digits at d upwards, at least every kDigitValues values; a top
+// digit that might overflow before the next carry is taken out and returned
+// (in units of 2^57)
+__device__ __forceinline__ int carry_digits(int* d) {
+    u64 c = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        c += (unsigned)d[i];
+        d[i] = (int)((unsigned)c & kDigitMask);
+        c >>= kDigitBits;
+    }
+    const int top = d[3] + (int)c;
+    const int out = top >= (1 << 29) || top <= -(1 << 29) ? top : 0;
+    d[3] = top - out;
+    return out;
+}
+
+// the FP64 value of the digits at d and of a top digit that was taken out
+__device__ __forceinline__ double digit_unit(int base) {
+    return __hiloint2double(((base == kNoBase ? 1023 : base) - 52) << 20, 0);
+}
+__device__ __forceinline__ double digits_value(const int* d, int base) {
+    const long long h = (long long)d[3] * (1 << kDigitBits) + (unsigned)d[2];
+    const long long l = ((long long)(unsigned)d[1] << kDigitBits) + (unsigned)d[0];
+    return fma((double)h, 0x1p38, (double)l) * digit_unit(base);
+}
+__device__ __forceinline__ double top_value(int top, int base) {
+    return (double)top * 0x1p57 * digit_unit(base);
+}
+
+// -------------------------------------------------------------------
+// FixHist64: per-slice counts and sums of x and y of one CTA in shared memory,
+// as the digits above; values outside the window go to the CTA's (cluster's)
+// partial column in global memory, FP64 atomics.
 //
 // What it replaces: warp-private FP64 histograms, whose lanes were
 // serialised by bids in shared memory, two FP64 additions for each round
 // whatever the number of lanes left (19 cycles of the FP64 pipe each, 2 to
 // 5 rounds at 500 to 50 slices).
 // -------------------------------------------------------------------
-
-// adds u to the four digits at d (shared memory; k: the unit, fix64_k); false
-// if it is out of the fixed point's range
-__device__ __forceinline__ bool fix64_add(int* d, int k, double u) {
-    const int hi = __double2hiint(u), lo = __double2loint(u);
-    const int r = k - biased_exp(hi);
-    if (r < 2) return false;
-    u64 v = shr_clamp(mant64(hi, lo), r);
-    if (hi < 0) v = 0ull - v;
-    const unsigned vl = (unsigned)v;
-    const int vh = (int)(v >> 32);
-    atomicAdd(d, (int)(vl & 0xffffu));
-    atomicAdd(d + 1, (int)(vl >> 16));
-    atomicAdd(d + 2, vh & 0xffff);
-    atomicAdd(d + 3, vh >> 16);
-    return true;
-}
-
 constexpr int kFix64Words = 9;   // per slice: count, 4 digits of x, 4 of y
+
+struct Spill64 {
+    double* sum[2];       // of x and y in the partial column
+    int64_t stride;       // between slices
+};
+static __device__ __noinline__ void spill64(const Spill64* sp, int q, int s, double u) {
+    if (u != 0.0) atomicAdd(sp->sum[q] + s * sp->stride, u);
+}
 
 struct FixHist64 {
     int* w;               // [S][kFix64Words]
-    unsigned* flag;       // [(S + 3) / 4]: one byte per slice, bit q: marked
-    int* any;             // a slice of this CTA is marked
-    int k[2];             // v = mant64 >> (k[q] - e)
+    const Spill64* sp;    // in shared memory
+    int base[2];          // windows of x and y (digit_base)
 
     __device__ __forceinline__ void add_q(int q, int s, double u) const {
-        if (!fix64_add(w + s * kFix64Words + 1 + 4 * q, k[q], u)) {
-            atomicOr(flag + (s >> 2), 1u << (8 * (s & 3) + q));
-            *any = 1;
-        }
+        if (!add_digits(w + s * kFix64Words + 1 + 4 * q, base[q], u)) spill64(sp, q, s, u);
     }
     __device__ __forceinline__ void add(int s, double x, double y) const {
         atomicAdd(w + s * kFix64Words, 1);
         add_q(0, s, x);
         add_q(1, s, y);
     }
-    __device__ __forceinline__ bool marked(int s, int q) const {
-        return (flag[s >> 2] >> (8 * (s & 3) + q)) & 1u;
-    }
 };
 
-// k of a coordinate from its typical magnitude (the high word of the
-// double, sign cleared; ~0 when every first value is zero: values below 4
-// are then in range).  Clamped so that add_q marks NaN and infinity
-// (exponent 2047) and shifts zeros and subnormals (exponent 0) out.
-__device__ __forceinline__ int fix64_k(unsigned mhi) {
-    int e = mhi != ~0u ? (int)(mhi >> 20) : 1019;
-    e = e < 100 ? 100 : (e > 2000 ? 2000 : e);
-    return e + 7;
-}
-
-// the FP64 value of a slice's integer sum: L1 = sum of d0 + d1 2^16,
-// d2 and d3 the sums of the third and fourth digits (d3 with the carries)
-__device__ __forceinline__ double fix64_value(long long L1, long long d2,
-                                              long long d3, int k) {
-    const double v = fma((double)(d3 * 65536 + d2), 4294967296.0, (double)L1);
-    // unit 2^(k - 1086) (see FixHist64::k)
-    return scalbn(v, k - 1086);
-}
-
 // -------------------------------------------------------------------
-// Exact sums of doubles as fixed-point integers.
-//
-// A value u = w 2^(e - 1075) (w: its 53-bit significand, e: its biased
-// exponent) is the integer w 2^(e - base) of at most 78 bits and a sign, where
-// base <= e <= base + 25; it is split into three unsigned 20-bit digits and
-// the signed rest, added to 32-bit counters.  Nothing is rounded, so the sum
-// of such values is exact and does not depend on their order.  Every other
-// value (smaller than 2^-18 or more than 2^7 times the typical value that
-// sets the base, subnormal, infinite, NaN) is left to the caller, who adds it
-// in FP64: a sum is never less accurate than a floating-point loop's.
-// A window of 64 bits that truncates what lies below it is a digit's work
-// cheaper but loses the slices whose values are all small.
+// The typical magnitude that sets a CTA's window.
 // -------------------------------------------------------------------
-constexpr int kFix80Values = 4095;      // at most, between two carries
-constexpr int kFix80None = 1 << 16;     // base: no value is representable
 
-// base for a typical magnitude, given as the high word of the double (sign
-// cleared; 0 or ~0: none seen)
-__device__ __forceinline__ int fix80_base(unsigned mhi) {
-    if (mhi == 0u || mhi == ~0u) return kFix80None;
-    const int e = (int)(mhi >> 20);
-    return (e < 100 ? 100 : (e > 2000 ? 2000 : e)) - 18;
-}
-
-// adds u to the four digits at d (shared memory); false if it is not
-// representable (zeros add nothing)
-__device__ __forceinline__ bool fix80_add(int* d, int base, double u) {
-    const int hi = __double2hiint(u);
-    const unsigned wl = (unsigned)__double2loint(u);
-    if ((((unsigned)hi << 1) | wl) == 0u) return true;
-    const int s = biased_exp(hi) - base;
-    if ((unsigned)s > 25u) return false;
-    const unsigned wh = ((unsigned)hi & 0xfffffu) | 0x100000u;
-    unsigned v0 = wl << s, v1 = __funnelshift_l(wl, wh, s), v2 = (wh >> 7) >> (25 - s);
-    if (hi < 0) {
-        v2 = ~v2 + ((v0 | v1) == 0u ? 1u : 0u);
-        v1 = ~v1 + (v0 == 0u ? 1u : 0u);
-        v0 = 0u - v0;
-    }
-    atomicAdd(d, (int)(v0 & 0xfffffu));
-    atomicAdd(d + 1, (int)(__funnelshift_r(v0, v1, 20) & 0xfffffu));
-    atomicAdd(d + 2, (int)((v1 >> 8) & 0xfffffu));
-    atomicAdd(d + 3, (int)__funnelshift_r(v1, v2, 28));
-    return true;
-}
-
-// carries the digits at d upwards, at least every kFix80Values values; a top
-// digit that might overflow before the next carry is taken out and returned
-// (in units of 2^60)
-__device__ __forceinline__ int fix80_carry(int* d) {
-    u64 c = 0;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        c += (unsigned)d[i];
-        d[i] = (int)((unsigned)c & 0xfffffu);
-        c >>= 20;
-    }
-    const int top = d[3] + (int)c;
-    const int out = top >= (1 << 30) || top <= -(1 << 30) ? top : 0;
-    d[3] = top - out;
-    return out;
-}
-
-// the FP64 value of the digits at d and of a carried-out top digit
-__device__ __forceinline__ double fix80_scale(int base) {
-    return __hiloint2double(((base == kFix80None ? 1023 : base) - 52) << 20, 0);
-}
-__device__ __forceinline__ double fix80_value(const int* d, int base) {
-    const long long h = (long long)d[3] * (1 << 20) + (unsigned)d[2];
-    const long long l = ((long long)(unsigned)d[1] << 20) + (unsigned)d[0];
-    return fma((double)h, 0x1p40, (double)l) * fix80_scale(base);
-}
-__device__ __forceinline__ double fix80_top(int top, int base) {
-    return (double)top * 0x1p60 * fix80_scale(base);
-}
-
-// Particle t (0 .. THREADS - 1) of a sample of those that this CTA works on,
-// the tiles blockIdx.x, blockIdx.x + gridDim.x, ... of TILE particles; -1 if
-// it has none.  A warp's 32 are spread over all of them: in a bunch that is
-// ordered by a coordinate, a tile is no sample.
+// Particle of this thread in a sample of those that the CTA works on, the
+// tiles blockIdx.x, blockIdx.x + gridDim.x, ... of TILE particles; -1 if it has
+// none.  Every warp looks into another tile, spread over all of them: in a
+// bunch that is ordered by a coordinate, the first tile is no sample.  (A warp's
+// 32 from as many tiles cost 6 us of a pass over 1e7 particles.)
 template <int THREADS, int TILE>
-__device__ __forceinline__ int64_t own_sample(int t, int64_t n) {
+__device__ __forceinline__ int64_t own_sample(int tid, int64_t n) {
     const int64_t tiles = (n + TILE - 1) / TILE;
     if ((int64_t)blockIdx.x >= tiles) return -1;
     const int64_t own = (tiles - 1 - blockIdx.x) / gridDim.x + 1;
-    const int64_t last = blockIdx.x + (own - 1) * gridDim.x;
-    const int64_t live = n - last * TILE;
-    const int64_t count = (own - 1) * TILE + (live < TILE ? live : TILE);
-    const int64_t j = ((t & 31) * (THREADS / 32) + (t >> 5)) * count / THREADS;
-    return ((int64_t)blockIdx.x + j / TILE * gridDim.x) * TILE + j % TILE;
+    const int64_t it = (tid >> 5) * own / (THREADS / 32);
+    const int64_t i = (blockIdx.x + it * gridDim.x) * TILE + tid;
+    return i < n ? i : -1;
+}
+
+// the high word of |u|; 0 for zero, infinity and NaN
+__device__ __forceinline__ unsigned finite_high(double u) {
+    const unsigned b = (unsigned)__double2hiint(u) & 0x7fffffffu;
+    return b < 0x7ff00000u ? b : 0u;
+}
+
+// The median of what the warps saw at most, of those that saw something: a few
+// stray values, or warps that hold none, do not set it.  most: WARPS entries in
+// shared memory; all lanes of a warp call it.
+template <int WARPS>
+__device__ __forceinline__ unsigned typical_of(const unsigned* most) {
+    const int lane = threadIdx.x & 31;
+    const unsigned v = lane < WARPS ? most[lane] : 0u;
+    int rank = 0;
+    for (int j = 0; j < WARPS; ++j) {
+        const unsigned o = __shfl_sync(0xffffffffu, v, j);
+        rank += o > v || (o == v && j < lane);
+    }
+    const int seen = __popc(__ballot_sync(0xffffffffu, v != 0u));
+    const unsigned at = __ballot_sync(0xffffffffu, lane < WARPS && rank == (seen - 1) / 2);
+    return seen ? __shfl_sync(0xffffffffu, v, __ffs(at) - 1) : 0u;
 }
 
 // -------------------------------------------------------------------

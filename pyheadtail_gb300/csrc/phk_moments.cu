@@ -3,10 +3,10 @@
 // passes over the particles (sums and counts, then centred products).
 //
 // The values are summed per CTA as exact fixed-point digits in shared memory
-// (fix80_add; the window of each value from a sample of the CTA's particles)
+// (add_digits; the window of each value from a sample of the CTA's particles)
 // and the CTA adds its totals to the caller's FP64 arrays, one global atomic
-// per slice and value; a value outside the window (2^7 times the typical one,
-// 2^-18 of it, infinite, NaN) is added there on its own.  Before, every
+// per slice and value; a value outside the window (32 times the typical one,
+// 2^-17 of it, infinite, NaN) is added there on its own.  Before, every
 // particle's value was a global FP64 atomic, one launch pair per statistic:
 // 22 launches of 220 us for all statistics of 1e6 particles in 200 slices,
 // now two.  The integer work and the shared-memory atomics bound it (52
@@ -75,7 +75,9 @@ moments_kernel(const __grid_constant__ phk_slicer sl, const __grid_constant__ Mo
     constexpr int NQ = PAIRS::NQ, NV = PASS == 0 ? NQ : PAIRS::NP;
     constexpr int W = moment_words<PAIRS, PASS>(), D0 = PASS == 0 ? 1 : 0;
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ unsigned s_typ[NV];
+    constexpr int WARPS = kMomThreads / 32;
+    __shared__ unsigned s_most[NV][WARPS];
+    __shared__ int s_base[NV];
     const int S = sl.n_slices, tid = threadIdx.x;
     T* edges = reinterpret_cast<T*>(smem);
     int* words = reinterpret_cast<int*>(smem + align16(sizeof(T) * (S + 1)));
@@ -83,7 +85,6 @@ moments_kernel(const __grid_constant__ phk_slicer sl, const __grid_constant__ Mo
         stage_edge<T>(edges, i, reinterpret_cast<const T*>(sl.edges)[i]);
     if (a.in_smem)
         for (int i = tid; i < W * S; i += kMomThreads) words[i] = 0;
-    if (tid < NV) s_typ[tid] = ~0u;
     __syncthreads();
     Bins<T> bins;
     bins.init(edges, S, sl.negate);
@@ -108,21 +109,25 @@ moments_kernel(const __grid_constant__ phk_slicer sl, const __grid_constant__ Mo
         return s;
     };
 
-    // ---- the window of every value: of the largest magnitude of each warp's
-    // sample, the smallest.  Particles outside the cuts count as zeros.
+    // ---- the window of every value, from a sample; particles outside the
+    // cuts count as zeros
     double v[NV];
     int64_t i = own_sample<kMomThreads, kMomThreads>(tid, a.n);
     int s = values(i < 0 ? a.n : i, v);
 #pragma unroll
     for (int p = 0; p < NV; ++p) {
-        const unsigned b = (unsigned)__double2hiint(v[p]) & 0x7fffffffu;
-        const unsigned m = __reduce_max_sync(0xffffffffu, b < 0x7ff00000u ? b : 0u);
-        if ((tid & 31) == 0 && m) atomicMin(&s_typ[p], m);
+        const unsigned m = __reduce_max_sync(0xffffffffu, finite_high(v[p]));
+        if ((tid & 31) == 0) s_most[p][tid >> 5] = m;
+    }
+    __syncthreads();
+    for (int p = tid >> 5; p < NV; p += WARPS) {
+        const int base = digit_base(typical_of<WARPS>(s_most[p]), 17);
+        if ((tid & 31) == 0) s_base[p] = base;
     }
     __syncthreads();
     int base[NV];
 #pragma unroll
-    for (int p = 0; p < NV; ++p) base[p] = fix80_base(s_typ[p]);
+    for (int p = 0; p < NV; ++p) base[p] = s_base[p];
 
     const int64_t step = (int64_t)gridDim.x * kMomThreads;
     const int64_t rounds = (a.n + step - 1) / step;
@@ -135,16 +140,17 @@ moments_kernel(const __grid_constant__ phk_slicer sl, const __grid_constant__ Mo
 #pragma unroll
             for (int p = 0; p < NV; ++p) {
                 if (PASS == 0 ? p < a.n_q : PAIRS::b(p) < a.n_q)
-                    if (!a.in_smem || !fix80_add(w + D0 + 4 * p, base[p], v[p]))
+                    if (!a.in_smem ||
+                        (!add_digits(w + D0 + 4 * p, base[p], v[p]) && v[p] != 0.0))
                         atomicAdd(a.sums + p * S + s, v[p]);
             }
         }
-        if (a.in_smem && (it + 1) % (kFix80Values / kMomThreads) == 0) {
+        if (a.in_smem && (it + 1) % (kDigitValues / kMomThreads) == 0) {
             __syncthreads();
             for (int j = tid; j < S * NV; j += kMomThreads) {
                 const int p = j / S, sj = j - p * S;
-                const int top = fix80_carry(words + sj * W + D0 + 4 * p);
-                if (top) atomicAdd(a.sums + j, fix80_top(top, fix80_base(s_typ[p])));
+                const int top = carry_digits(words + sj * W + D0 + 4 * p);
+                if (top) atomicAdd(a.sums + j, top_value(top, s_base[p]));
             }
             __syncthreads();
         }
@@ -154,7 +160,7 @@ moments_kernel(const __grid_constant__ phk_slicer sl, const __grid_constant__ Mo
     __syncthreads();
     for (int j = tid; j < S * NV; j += kMomThreads) {
         const int p = j / S, sj = j - p * S;
-        const double t = fix80_value(words + sj * W + D0 + 4 * p, fix80_base(s_typ[p]));
+        const double t = digits_value(words + sj * W + D0 + 4 * p, s_base[p]);
         if (t != 0.0) atomicAdd(a.sums + j, t);
     }
     if (PASS == 0)

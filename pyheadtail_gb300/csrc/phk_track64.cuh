@@ -20,18 +20,17 @@ struct Track64Args {
 };
 
 // shared memory, every region 16-byte aligned: FixHist64 words [Sa][9] int,
-// flag bytes [Sa], accumulation edges [Sa + 1] (keys), pending-kick edges
-// [Sp + 1] (keys; the same table with `share`), kick tables [n_tables][Sp],
-// the quarter wave (`sine`)
+// accumulation edges [Sa + 1] (keys), pending-kick edges [Sp + 1] (keys; the
+// same table with `share`), kick tables [n_tables][Sp], the quarter wave
+// (`sine`)
 struct Track64Smem {
-    size_t words, flags, eacc, epk, ktab, sine, bytes;
+    size_t words, eacc, epk, ktab, sine, bytes;
 };
 __host__ __device__ inline Track64Smem track64_smem(int Sa, int Sp, int n_tables,
                                                     bool share, bool sine) {
     Track64Smem m;
     size_t b = 0;
     m.words = b; b = align16(b + (size_t)4 * kFix64Words * Sa);
-    m.flags = b; b = align16(b + (size_t)4 * ((Sa + 3) / 4));
     m.eacc = b; b = align16(b + (size_t)8 * (Sa > 0 ? Sa + 1 : 0));
     m.epk = share ? m.eacc : b;
     if (!share) b = align16(b + (size_t)8 * (Sp > 0 ? Sp + 1 : 0));
@@ -41,32 +40,54 @@ __host__ __device__ inline Track64Smem track64_smem(int Sa, int Sp, int n_tables
     return m;
 }
 
-// FixHist64: carries the digits of this CTA into the column's 64-bit words
-// (counts of 2^48 units), leaving 16 bits in the lower three (all threads,
-// between two barriers).
-__device__ __forceinline__ void fix64_carry(const FixHist64& f, int S,
-                                            long long* column, int64_t G,
-                                            int tid, int nthreads) {
-    for (int s = tid; s < S; s += nthreads) {
-#pragma unroll
+// The parts of the tile loop that seldom run are out of line: the loop fills
+// the instruction cache as it is (inlined, they cost 5 % of a pass).
+
+// What the warps of a CTA saw at most of x and y (high words): of a sample of
+// the inputs, and of the outputs of a tile
+struct Seen64 {
+    unsigned in[2][kTrackThreads / 32], out[2][kTrackThreads / 32];
+};
+__device__ __forceinline__ void note_seen(unsigned (*to)[kTrackThreads / 32],
+                                          unsigned mx, unsigned my) {
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    my = __reduce_max_sync(0xffffffffu, my);
+    if ((threadIdx.x & 31) == 0) {
+        to[0][threadIdx.x >> 5] = mx;
+        to[1][threadIdx.x >> 5] = my;
+    }
+}
+
+// The windows: the larger of the typical input, of a sample spread over the
+// bunch, and the typical output of this tile (a bunch that starts on the axis,
+// a large beta at the end of the turn); where both are zero, they stay as they
+// are and the next tile is looked at.  mx, my: largest of this thread's.  All
+// threads of the CTA call it; true if a window is still open.
+static __device__ __noinline__ bool set_windows(Seen64* seen, int* base, unsigned mx,
+                                                unsigned my) {
+    constexpr int WARPS = kTrackThreads / 32;
+    note_seen(seen->out, mx, my);
+    __syncthreads();
+    const int q = (threadIdx.x >> 5) & 1;
+    const unsigned typ = max(typical_of<WARPS>(seen->in[q]), typical_of<WARPS>(seen->out[q]));
+    if ((threadIdx.x & ~32u) == 0 && base[q] == kNoBase) base[q] = digit_base(typ, 18);
+    __syncthreads();
+    return base[0] == kNoBase || base[1] == kNoBase;
+}
+
+// Carries the digits of the slices with more than `most` values (all threads)
+static __device__ __noinline__ void carry_slices(int* words, int S, int most,
+                                                 const Spill64* sp, const int* base) {
+    __syncthreads();
+    for (int s = threadIdx.x; s < S; s += kTrackThreads) {
+        int* w = words + s * kFix64Words;
+        if (w[0] <= most) continue;
         for (int q = 0; q < 2; ++q) {
-            unsigned* d = reinterpret_cast<unsigned*>(f.w) + s * kFix64Words +
-                          1 + 4 * q;
-            long long c = 0;
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                c += d[i];
-                d[i] = (unsigned)c & 0xffffu;
-                c >>= 16;
-            }
-            c += (int)d[3];
-            d[3] = 0u;
-            if (c != 0)
-                atomicAdd(reinterpret_cast<unsigned long long*>(
-                              column + ((int64_t)(q + 1) * S + s) * G),
-                          (unsigned long long)c);
+            const int top = carry_digits(w + 1 + 4 * q);
+            if (top) spill64(sp, q, s, top_value(top, base[q]));
         }
     }
+    __syncthreads();
 }
 
 // Three CTAs per SM (80 registers): the FP64 pipe and the integer pipes are
@@ -81,17 +102,15 @@ track64_kernel(const __grid_constant__ phk_program prog,
                const __grid_constant__ Track64Args ka) {
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char smem[];
-    // the sums' unit: smallest over the warps of their largest |x|, |y|
-    // (high words)
-    __shared__ unsigned s_typ[2];
-    __shared__ int s_marked;        // FixHist64::any
+    __shared__ Seen64 s_seen;
+    __shared__ int s_base[2];       // windows of x and y
+    __shared__ Spill64 s_spill;
     constexpr int TILE = kTrackThreads * VEC;
     const TrackArgs& a = ka.t;
     const int Sa = a.has_acc ? acc.slicer.n_slices : 0;
     const int Sp = a.has_pk ? pk.slicer.n_slices : 0;
     const Track64Smem lay = track64_smem(Sa, Sp, a.n_tables, ka.share_edges, ka.sine);
     int* words = reinterpret_cast<int*>(smem + lay.words);
-    unsigned* flags = reinterpret_cast<unsigned*>(smem + lay.flags);
     double* eacc = reinterpret_cast<double*>(smem + lay.eacc);
     double* epk = reinterpret_cast<double*>(smem + lay.epk);
     double* ktab = reinterpret_cast<double*>(smem + lay.ktab);
@@ -106,19 +125,26 @@ track64_kernel(const __grid_constant__ phk_program prog,
     Tile<double, VEC> t;
     load_tile_plain<double, VEC>(a, cx, t, i0, i0 + VEC <= a.n);
 
-    if (tid == 0) {
-        s_typ[0] = s_typ[1] = ~0u;
-        s_marked = 0;
+    // so is a sample of its x and y
+    unsigned m_in[2] = {0u, 0u};
+    if (a.has_acc) {
+        const int64_t i = own_sample<kTrackThreads, TILE>(tid, a.n);
+        if (i >= 0) {
+            m_in[0] = finite_high(cx.cp[PHK_X][i]);
+            m_in[1] = finite_high(cx.cp[PHK_Y][i]);
+        }
     }
+
     if (a.has_acc) {
         const double* e = reinterpret_cast<const double*>(acc.slicer.edges);
         for (int i = tid; i <= Sa; i += kTrackThreads) stage_edge<double>(eacc, i, e[i]);
         for (int i = tid; i < kFix64Words * Sa; i += kTrackThreads) words[i] = 0;
-        for (int i = tid; i < (Sa + 3) / 4; i += kTrackThreads) flags[i] = 0u;
     }
     if (a.has_pk)
         stage_pending<double>(pk, a, epk, ktab, tid, kTrackThreads, ka.share_edges);
     if (ka.sine) stage_sine(sine, tid, kTrackThreads);
+    if (a.has_acc) note_seen(s_seen.in, m_in[0], m_in[1]);
+    if (tid < 2) s_base[tid] = kNoBase;
     __syncthreads();
     if (a.has_pk) cx.bpk.init(epk, Sp, pk.slicer.negate);
     if (a.has_acc) cx.bac.init(eacc, Sa, acc.slicer.negate);
@@ -131,136 +157,91 @@ track64_kernel(const __grid_constant__ phk_program prog,
     const int column = clustered ? (int)(blockIdx.x / a.cluster) : (int)blockIdx.x;
     const int64_t G = acc.grid;
     double* P = acc.partials + column;
-    long long* PL = reinterpret_cast<long long*>(P);
 
     if (a.has_acc) {
-        // ---- the cluster's unit, from the finite |x|, |y| of the inputs of
-        // every member's first tile (the maps change them by factors of
-        // order one; much larger values mark their slice)
-        unsigned m[2] = {0u, 0u};
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) {
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {      // zeros past the end
-                const unsigned b =
-                    (unsigned)__double2hiint(t.c[q ? PHK_Y : PHK_X][j]) & 0x7fffffffu;
-                if (b < 0x7ff00000u && b > m[q]) m[q] = b;
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            m[q] = __reduce_max_sync(0xffffffffu, m[q]);
-            if ((tid & 31) == 0 && m[q]) atomicMin(&s_typ[q], m[q]);
-        }
-        // rank 0 clears its column's 64-bit words before any member adds
+        // rank 0 clears its column's sums before any member adds
         if (crank == 0)
-            for (int s = tid; s < 2 * Sa; s += kTrackThreads) PL[(Sa + s) * G] = 0;
-        unsigned M[2];
-        if (clustered) {
-            cg::cluster_group cl = cg::this_cluster();
-            cl.sync();                   // orders the clears, see kCluster
-            M[0] = M[1] = ~0u;
-            for (unsigned r = 0; r < cl.num_blocks(); ++r) {
-                const unsigned* sm = cl.map_shared_rank(s_typ, r);
-                M[0] = min(M[0], sm[0]);
-                M[1] = min(M[1], sm[1]);
-            }
-        } else {
-            __syncthreads();
-            M[0] = s_typ[0];
-            M[1] = s_typ[1];
+            for (int s = tid; s < 2 * Sa; s += kTrackThreads) P[(Sa + s) * G] = 0.0;
+        if (tid == 0) {
+            s_spill.sum[0] = P + Sa * G;
+            s_spill.sum[1] = P + 2 * Sa * G;
+            s_spill.stride = G;
         }
+        if (clustered) cg::this_cluster().sync();   // orders the clears, see kCluster
+        else __syncthreads();
         cx.fix.w = words;
-        cx.fix.flag = flags;
-        cx.fix.any = &s_marked;
-        cx.fix.k[0] = fix64_k(M[0]);
-        cx.fix.k[1] = fix64_k(M[1]);
+        cx.fix.sp = &s_spill;
+        cx.fix.base[0] = cx.fix.base[1] = kNoBase;
     }
 
     // ---- the tiles: every warp runs whole ones (lanes past the end carry
     // dead particles)
+    constexpr int kTiles = kDigitValues / TILE;
+    int until_carry = kTiles;
+    bool open = a.has_acc;          // a window is still to be set
     const int64_t step = (int64_t)gridDim.x * TILE;
     const int64_t rounds = (a.n_tiles + gridDim.x - 1) / gridDim.x;
     for (int64_t it = 0; it < rounds; ++it, i0 += step) {
-        run_tile<double, VEC, SHAPE, false, true>(prog, pk, acc, a, cx, t, i0,
-                                                  i0 + VEC <= a.n);
+        tile_advance<double, VEC, SHAPE, false>(prog, pk, a, cx, t, i0);
+        if (open) {
+            unsigned m[2] = {0u, 0u};
+#pragma unroll
+            for (int j = 0; j < VEC; ++j)
+                if (i0 + j < a.n) {
+                    m[0] = max(m[0], finite_high(t.c[PHK_X][j]));
+                    m[1] = max(m[1], finite_high(t.c[PHK_Y][j]));
+                }
+            open = set_windows(&s_seen, s_base, m[0], m[1]);
+            cx.fix.base[0] = s_base[0];
+            cx.fix.base[1] = s_base[1];
+        }
+        tile_finish<double, VEC, false, true>(acc, a, cx, t, i0, i0 + VEC <= a.n);
         load_tile_plain<double, VEC>(a, cx, t, i0 + step, i0 + step + VEC <= a.n);
-        if (a.has_acc && (it + 1) % fix_flush_tiles<TILE>() == 0) {
-            __syncthreads();
-            fix64_carry(cx.fix, Sa, PL, G, tid, kTrackThreads);
-            __syncthreads();
+        if (a.has_acc && --until_carry == 0) {
+            // before a counter can overflow in the next kTiles tiles
+            until_carry = kTiles;
+            carry_slices(words, Sa, kDigitValues - kTiles * TILE, &s_spill, s_base);
         }
     }
     if (!a.has_acc) return;
 
-    // ---- rank 0 adds its cluster's counters and 64-bit words as integers
-    // and writes the partial column in FP64
+    // ---- rank 0 writes the partial column: every CTA's exact sums, and what
+    // lay outside their windows
     unsigned nb = 1;
-    int any = 0;
     if (clustered) {
         // adds to the column before the barrier (see kCluster)
         cg::cluster_group cl = cg::this_cluster();
         cl.sync();
         nb = cl.num_blocks();
-        for (unsigned r = 0; r < nb; ++r) any |= *cl.map_shared_rank(&s_marked, r);
-        if (crank == 0 && any) {
-            // this CTA's flags become the cluster's
-            for (int i = tid; i < (Sa + 3) / 4; i += kTrackThreads)
-                for (unsigned r = 1; r < nb; ++r)
-                    flags[i] |= cl.map_shared_rank(flags, r)[i];
-            __syncthreads();
-        }
     } else {
         __syncthreads();
-        any = s_marked;
     }
     if (crank == 0) {
         for (int s = tid; s < Sa; s += kTrackThreads) {
-            long long c = 0, L1[2] = {0, 0}, d2[2] = {0, 0}, d3[2];
-            d3[0] = __ldcg(PL + (Sa + s) * G);
-            d3[1] = __ldcg(PL + (2 * Sa + s) * G);
+            long long c = 0;
+            double v[2];
+            v[0] = __ldcg(P + (Sa + s) * G);
+            v[1] = __ldcg(P + (2 * Sa + s) * G);
             // unrolled over the cluster's members, so that the loads of
             // every member are in flight together
 #pragma unroll
             for (int r = 0; r < kCluster; ++r) {
                 if (r >= (int)nb) break;
                 const int* w = words;
-                if (clustered) w = cg::this_cluster().map_shared_rank(words, r);
+                const int* base = s_base;
+                if (clustered) {
+                    w = cg::this_cluster().map_shared_rank(words, r);
+                    base = cg::this_cluster().map_shared_rank(s_base, r);
+                }
                 w += s * kFix64Words;
                 c += w[0];
 #pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const unsigned* d = reinterpret_cast<const unsigned*>(w) + 1 + 4 * q;
-                    L1[q] += (long long)d[0] + ((long long)d[1] << 16);
-                    d2[q] += d[2];
-                    d3[q] += (int)d[3];
-                }
+                for (int q = 0; q < 2; ++q)
+                    v[q] = add(v[q], digits_value(w + 1 + 4 * q, base[q]));
             }
             P[s * G] = (double)c;
-#pragma unroll
-            for (int q = 0; q < 2; ++q)
-                P[((q + 1) * Sa + s) * G] =
-                    any && cx.fix.marked(s, q)
-                        ? 0.0 : fix64_value(L1[q], d2[q], d3[q], cx.fix.k[q]);
-        }
-    }
-    if (any) {
-        // ---- marked slices: the cluster's CTAs add their particles'
-        // updated values in FP64 (each thread reads what it stored)
-        __threadfence();
-        if (clustered) cg::this_cluster().sync(); else __syncthreads();
-        const unsigned* fl = clustered ? cg::this_cluster().map_shared_rank(flags, 0)
-                                       : flags;
-        i0 = (int64_t)blockIdx.x * TILE + tid * VEC;
-        for (int64_t it = 0; it < rounds; ++it, i0 += step) {
-            for (int j = 0; j < VEC; ++j) {
-                if (i0 + j >= a.n) continue;
-                const int s = cx.bac.index(cx.cp[PHK_Z][i0 + j]);
-                if (s < 0) continue;
-                const unsigned f = fl[s >> 2] >> (8 * (s & 3));
-                if (f & 1u) atomicAdd(P + (Sa + s) * G, cx.cp[PHK_X][i0 + j]);
-                if (f & 2u) atomicAdd(P + (2 * Sa + s) * G, cx.cp[PHK_Y][i0 + j]);
-            }
+            P[(Sa + s) * G] = v[0];
+            P[(2 * Sa + s) * G] = v[1];
         }
     }
     if (clustered) cg::this_cluster().sync();  // members keep their counters until read
