@@ -566,7 +566,10 @@ int phk_slice_moments_all(const phk_slicer *slicer, const phk_coords *coords,
  * bunch (tables batch->kicks; `pending` gives n_kicks, quad, target and the
  * slicer, its kick[] pointers are ignored), the bunch's program, binning
  * and per-slice sums into acc->partials[3][S][batch->n_columns]
- * (acc->grid must equal n_columns).  acc may be NULL (no slicing). */
+ * (acc->grid must equal n_columns).  acc may be NULL (no slicing).  FP32 values
+ * are summed exactly in a window of 2^-19 to 2^11 times a typical |value| of
+ * the CTA's particles of the bunch, others in FP64 (see phk_accum); FP64 values
+ * in FP64, in a fixed order while every warp's histogram fits. */
 int phk_track_batch(const phk_batch *batch, const phk_coords *coords,
                     const phk_kick_set *pending, const phk_accum *acc,
                     void *stream);

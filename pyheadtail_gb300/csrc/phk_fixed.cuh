@@ -200,6 +200,117 @@ struct FixHist64 {
 };
 
 // -------------------------------------------------------------------
+// FixHist32: the same for the FP32 coordinates of a batch's bunch (one CTA, in
+// the bunch's partial column).  A float is split by adding and subtracting
+// 1.5 2^23 units: the low bits of the sum are the value in these units, so the
+// sum itself, as an integer, goes to the counter, and the constant is taken off
+// at the end, once per value.  Three digits, units 2^36, 2^18 and 1, of at most
+// 2^17; the last unit is 2^-42 of the typical value, so that floats from 2^-19
+// to 2^11 times it leave no remainder.  Others are added to the column in FP64.
+// -------------------------------------------------------------------
+// a value outside the window (its digits are the constants)
+static __device__ __noinline__ void outside32(int* d, int S, float top, const Spill64* sp,
+                                              int q, int s, float u) {
+    atomicAdd(d, __float_as_int(top));
+    atomicAdd(d + S, __float_as_int(top * 0x1p-18f));
+    atomicAdd(d + 2 * S, __float_as_int(top * 0x1p-36f));
+    if (u != 0.0f) atomicAdd(sp->sum[q] + s * sp->stride, (double)u);
+}
+
+struct FixHist32 {
+    int* cnt;             // [S]
+    int* dig;             // [6][S]: x top, middle, low, y
+    const Spill64* sp;    // in shared memory
+    int S;
+    float top[2];         // 1.5 2^23 units of the top digit (digit_top)
+
+    __device__ __forceinline__ void add_q(int q, int s, float u) const {
+        const float H = top[q], M = H * 0x1p-18f, L = H * 0x1p-36f;
+        const float h = __fadd_rn(u, H), r = __fsub_rn(u, __fsub_rn(h, H));
+        const float m = __fadd_rn(r, M), e = __fsub_rn(r, __fsub_rn(m, M));
+        const float l = __fadd_rn(e, L);
+        int* d = dig + 3 * q * S + s;
+        if (fabsf(u) < H * (1.0f / 128.0f) && __fsub_rn(l, L) == e) {
+            atomicAdd(d, __float_as_int(h));
+            atomicAdd(d + S, __float_as_int(m));
+            atomicAdd(d + 2 * S, __float_as_int(l));
+        } else {
+            outside32(d, S, H, sp, q, s, u);
+        }
+    }
+    __device__ __forceinline__ void add(int s, float x, float y) const {
+        atomicAdd(cnt + s, 1);
+        add_q(0, s, x);
+        add_q(1, s, y);
+    }
+};
+
+// FixHist32::top for a typical magnitude (float bits; 0: none seen, nothing is
+// within the window)
+__device__ __forceinline__ float digit_top(unsigned bits) {
+    if (bits == 0u) return 0.0f;
+    const int e = (int)(bits >> 23) - 127;
+    return ldexpf(1.5f, (e < -106 ? -106 : (e > 100 ? 100 : e)) + 17);
+}
+// the last digit's unit
+__device__ __forceinline__ double digit_unit32(float top) {
+    const int k = (__float_as_int(top) >> 23) - 127;         // top = 1.5 2^k
+    return top == 0.0f ? 0.0 : __hiloint2double((k - 59 + 1023) << 20, 0);
+}
+// the digits of a slice with n values, without the constants
+__device__ __forceinline__ void digits32(const int* d, int S, float top, int n, int (&v)[3]) {
+    v[0] = (int)((unsigned)d[0] - (unsigned)n * __float_as_uint(top));
+    v[1] = (int)((unsigned)d[S] - (unsigned)n * __float_as_uint(top * 0x1p-18f));
+    v[2] = (int)((unsigned)d[2 * S] - (unsigned)n * __float_as_uint(top * 0x1p-36f));
+}
+__device__ __forceinline__ double digits32_value(const int* d, int S, float top, int n) {
+    int v[3];
+    digits32(d, S, top, n, v);
+    const long long h = ((long long)v[0] << 18) + v[1];
+    return fma((double)h, 0x1p18, (double)v[2]) * digit_unit32(top);
+}
+
+// Carries the digits of the slices with more than `most` values, at least every
+// kDigitValues values; a top digit that might overflow before the next carry
+// goes to the column (all threads)
+static __device__ __noinline__ void carry_slices32(const int* cnt, int* dig, int S, int most,
+                                                   const Spill64* sp, const unsigned* typ) {
+    __syncthreads();
+    for (int s = threadIdx.x; s < S; s += blockDim.x) {
+        const int n = cnt[s];
+        if (n <= most) continue;
+        for (int q = 0; q < 2; ++q) {
+            const float top = digit_top(typ[q]);
+            int* d = dig + 3 * q * S + s;
+            int v[3];
+            digits32(d, S, top, n, v);
+            const int c2 = v[2] >> 18, c1 = (v[1] + c2) >> 18;
+            int c0 = c1;
+            if (v[0] + c1 >= (1 << 29) || v[0] + c1 <= -(1 << 29)) {
+                c0 = -v[0];
+                atomicAdd(sp->sum[q] + s * sp->stride,
+                          (double)(v[0] + c1) * 0x1p36 * digit_unit32(top));
+            }
+            d[0] = (int)((unsigned)d[0] + (unsigned)c0);
+            d[S] = (int)((unsigned)d[S] + (unsigned)(c2 - c1 * (1 << 18)));
+            d[2 * S] = (int)((unsigned)d[2 * S] - (unsigned)(c2 * (1 << 18)));
+        }
+    }
+    __syncthreads();
+}
+
+// A window that is set after the bunch's first tiles: their values (zeros, or
+// in the column already) count as the constants (all threads)
+static __device__ __noinline__ void open_digits32(const int* cnt, int* dig, int S, float top) {
+    for (int s = threadIdx.x; s < S; s += blockDim.x) {
+        const unsigned n = (unsigned)cnt[s];
+        dig[s] = (int)(n * __float_as_uint(top));
+        dig[S + s] = (int)(n * __float_as_uint(top * 0x1p-18f));
+        dig[2 * S + s] = (int)(n * __float_as_uint(top * 0x1p-36f));
+    }
+}
+
+// -------------------------------------------------------------------
 // The typical magnitude that sets a CTA's window.
 // -------------------------------------------------------------------
 
@@ -224,6 +335,12 @@ __device__ __forceinline__ unsigned finite_high(double u) {
     return b < 0x7ff00000u ? b : 0u;
 }
 
+// the bits of |u|; 0 for infinity and NaN
+__device__ __forceinline__ unsigned finite_high(float u) {
+    const unsigned b = __float_as_uint(u) & 0x7fffffffu;
+    return b < 0x7f800000u ? b : 0u;
+}
+
 // The median of what the warps saw at most, of those that saw something: a few
 // stray values, or warps that hold none, do not set it.  most: WARPS entries in
 // shared memory; all lanes of a warp call it.
@@ -239,6 +356,41 @@ __device__ __forceinline__ unsigned typical_of(const unsigned* most) {
     const int seen = __popc(__ballot_sync(0xffffffffu, v != 0u));
     const unsigned at = __ballot_sync(0xffffffffu, lane < WARPS && rank == (seen - 1) / 2);
     return seen ? __shfl_sync(0xffffffffu, v, __ffs(at) - 1) : 0u;
+}
+
+// What the warps of a CTA saw at most of x and y: of a sample of the inputs,
+// and of the outputs of a tile
+template <int WARPS>
+struct Seen {
+    unsigned in[2][WARPS], out[2][WARPS];
+};
+template <int WARPS>
+__device__ __forceinline__ void note_seen(unsigned (*to)[WARPS], unsigned mx, unsigned my) {
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    my = __reduce_max_sync(0xffffffffu, my);
+    if ((threadIdx.x & 31) == 0) {
+        to[0][threadIdx.x >> 5] = mx;
+        to[1][threadIdx.x >> 5] = my;
+    }
+}
+
+// The typical magnitudes (0: none yet) from the sample of the inputs and the
+// outputs of this tile, the larger (a bunch that starts on the axis, a large
+// beta at the end of the turn); where both are zero they stay open and the next
+// tile is looked at.  mx, my: the largest of this thread's outputs.  All threads
+// of the CTA call it; true if one is still open.  Out of line, as everything in
+// the tile loop that seldom runs: the loop fills the instruction cache as it is
+// (inlined, these parts cost 5 % of a pass).
+template <int WARPS>
+__device__ __noinline__ bool find_typical(Seen<WARPS>* seen, unsigned* typ, unsigned mx,
+                                          unsigned my) {
+    note_seen<WARPS>(seen->out, mx, my);
+    __syncthreads();
+    const int q = (threadIdx.x >> 5) & 1;
+    const unsigned t = max(typical_of<WARPS>(seen->in[q]), typical_of<WARPS>(seen->out[q]));
+    if ((threadIdx.x & ~32u) == 0 && typ[q] == 0u) typ[q] = t;
+    __syncthreads();
+    return typ[0] == 0u || typ[1] == 0u;
 }
 
 // -------------------------------------------------------------------

@@ -1014,9 +1014,10 @@ __device__ __forceinline__ void run_program_shape(const phk_program& prog,
 // ===================================================================
 // per-slice accumulation in shared memory
 //
-// Fixed-point sums (FixHist below, FixHist64), one histogram per CTA updated
-//   with 32-bit integer atomics: integer addition is associative, so the
-//   sums are bit-identical whatever the order.
+// Fixed-point sums (FixHist below; FixHist64 and FixHist32, the FP32 batch's, in
+//   phk_fixed.cuh), one histogram per CTA updated with 32-bit integer atomics:
+//   integer addition is associative, so the sums are bit-identical whatever the
+//   order.
 //
 // FP64 batch: each warp owns a private histogram (count, sum x, sum y per
 //   slice) of plain double sums; lanes of a warp holding the same slice are
@@ -1027,7 +1028,7 @@ __device__ __forceinline__ void run_program_shape(const phk_program& prog,
 //   differ in their last bits between launches.  (In the FP32 batch, bids
 //   with compensated float sums took 40 % of the shared-memory pipe and a
 //   fifth of the instructions: 207 us a pass at 64 bunches and 1.03e7
-//   particles against 181 us as fixed-point sums.)
+//   particles against 188 us as exact fixed-point sums.)
 // ===================================================================
 
 // All 32 lanes of the warp must call this together; s < 0 means "no bin".
@@ -1069,10 +1070,9 @@ __device__ __forceinline__ void warp_accumulate(int s, double vx, double vy,
 // -------------------------------------------------------------------
 // FixHist: exact, order-independent per-slice sums of FP32 coordinates.
 //
-// Every thread-block cluster (batch: every CTA, for each bunch it works on)
-// agrees on one power-of-two scale per coordinate, 2^k with k chosen from the
-// largest finite |u| of its first tiles so that it maps to [2^26, 2^27).  A value
-// u becomes the integer v = rint(u 2^k) (u 2^k is exact; the rounding is
+// Every thread-block cluster agrees on one power-of-two scale per
+// coordinate, 2^k with k chosen from the largest finite |u| of its first
+// tiles so that it maps to [2^26, 2^27).  A value u becomes the integer v = rint(u 2^k) (u 2^k is exact; the rounding is
 // the only approximation, at most 2^-27 of that largest value, the order
 // of the FP32 rounding of u itself).  Level A, |u 2^k| < 2^30: v is split into two
 // 15-bit digits d0 = v & 0x7fff in [0, 2^15) and d1 = v >> 15 (arithmetic)
@@ -1084,8 +1084,8 @@ __device__ __forceinline__ void warp_accumulate(int s, double vx, double vy,
 // scale on the cluster's partial column in global memory, zeroed by the
 // cluster's rank 0 before the first add.  Level C: NaN, +-inf and
 // |u 2^k| >= 2^40 set flag bits of the slice; the slice's sum then becomes
-// NaN (NaN, both infinities, or out of range) or +-inf, as a floating-point
-// sum would.  At the end rank 0 adds the digits of its cluster's CTAs and
+// NaN (NaN, both infinities, or a finite value out of range) or +-inf, but for
+// the finite ones as a floating-point sum would.  At the end rank 0 adds the digits of its cluster's CTAs and
 // the level-B sums as 64-bit integers, converts once to FP64 (x 2^-k) and
 // writes the partial column.  Every step is integer arithmetic or a fixed
 // sequence of FP64 operations: the result is bit-identical on every launch.
@@ -1253,11 +1253,14 @@ __device__ __forceinline__ double tmul<double>(double a, double b) { return mul(
 template <>
 __device__ __forceinline__ float tmul<float>(float a, float b) { return a * b; }
 
+// FP32 histograms of track_smem_layout: FixHist, FixHist32
+constexpr int kFixSingle = 1, kFixBatch = 2;
+
 // shared memory layout, in this order (every region 16-byte aligned):
 //   histogram: bid-serialised words [3][n_hist][Sa] (sum x, sum y as double;
 //              count as int in the third region), or with `fix` (FP32) the
-//              FixHist counters: count [Sa], digits [4][Sa], flag bytes [Sa]
-//              (ints)
+//              integer counters: count [Sa], digits [4][Sa] and flag bytes [Sa]
+//              of FixHist, digits [6][Sa] of FixHist32
 //   accumulation edges [Sa + 1] T, pending-kick edges [Sp + 1] T,
 //   kick tables [n_tables][Sp] T (when staged), bid tags [n_hist][Sa] int
 //   (none with `fix`), TMA ring [stages][6][tile] T, one mbarrier per stage
@@ -1267,12 +1270,13 @@ template <typename T>
 __host__ __device__ inline size_t track_smem_layout(int Sa, int Sp, int n_hist,
                                                     int n_tables, int kicks_smem,
                                                     int stages, int tile,
-                                                    size_t* off, bool fix = false) {
+                                                    size_t* off, int fix = 0) {
     size_t b = 0;
     if (fix) {
-        off[0] = b; b = align16(b + (size_t)4 * Sa);              // count
-        off[1] = b; b = align16(b + (size_t)4 * 4 * Sa);          // digits
-        off[2] = b; b = align16(b + (size_t)4 * ((Sa + 3) / 4));  // flags
+        off[0] = b; b = align16(b + (size_t)4 * Sa);                            // count
+        off[1] = b; b = align16(b + (size_t)4 * (fix == kFixBatch ? 6 : 4) * Sa); // digits
+        off[2] = b;                                                             // flags
+        if (fix == kFixSingle) b = align16(b + (size_t)4 * ((Sa + 3) / 4));
     } else {
         off[0] = b; b = align16(b + (size_t)8 * n_hist * Sa);   // sum x words
         off[1] = b; b = align16(b + (size_t)8 * n_hist * Sa);   // sum y words
@@ -1540,8 +1544,9 @@ __device__ __forceinline__ void apply_pending(const phk_kick_set& pk,
     }
 }
 
-// Per-CTA state shared by the tile loops of the track kernel.
-template <typename T, int VEC>
+// Per-CTA state shared by the tile loops of the track kernels.  H: the
+// accumulation's histogram
+template <typename T, int VEC, class H = typename FixOf<T>::type>
 struct TrackCtx {
     T* cp[6];
     Bins<T> bpk, bac;
@@ -1552,7 +1557,7 @@ struct TrackCtx {
     int* tag;
     unsigned epoch;
     bool shared_hist;
-    typename FixOf<T>::type fix;   // single bunch, FP32 batch
+    H fix;                // single bunch, FP32 batch
     Aux64 aux;            // FP64 form
 };
 
@@ -1562,21 +1567,21 @@ struct TrackCtx {
 
 // 1. wake kicks of the previous WakeField.track, in kick order;
 // 2. element program
-template <typename T, int VEC, int SHAPE, bool FULL>
+template <typename T, int VEC, int SHAPE, bool FULL, class H>
 __device__ __forceinline__ void tile_advance(const phk_program& prog,
                                              const phk_kick_set& pk,
                                              const TrackArgs& a,
-                                             TrackCtx<T, VEC>& cx,
+                                             TrackCtx<T, VEC, H>& cx,
                                              Tile<T, VEC>& t, int64_t i0) {
     if (a.has_pk) apply_pending<T, VEC, FULL>(pk, a, cx.bpk, cx.ktab, t, i0);
     run_program_shape<T, VEC, SHAPE>(prog, cx.aux, t);
 }
 
 // 3. slice accumulation; 4. stores
-template <typename T, int VEC, bool FULL, bool FIX>
+template <typename T, int VEC, bool FULL, bool FIX, class H>
 __device__ __forceinline__ void tile_finish(const phk_accum& acc,
                                             const TrackArgs& a,
-                                            TrackCtx<T, VEC>& cx,
+                                            TrackCtx<T, VEC, H>& cx,
                                             Tile<T, VEC>& t, int64_t i0,
                                             bool full) {
     if (a.has_acc) {
@@ -1624,9 +1629,9 @@ __device__ __forceinline__ void run_tile(const phk_program& prog,
     tile_finish<T, VEC, FULL, FIX>(acc, a, cx, t, i0, full);
 }
 
-template <typename T, int VEC>
+template <typename T, int VEC, class H>
 __device__ __forceinline__ void load_tile_plain(const TrackArgs& a,
-                                                const TrackCtx<T, VEC>& cx,
+                                                const TrackCtx<T, VEC, H>& cx,
                                                 Tile<T, VEC>& t, int64_t i0,
                                                 bool full) {
 #pragma unroll
@@ -1706,7 +1711,7 @@ track_kernel(const __grid_constant__ phk_program prog,
     const int Sp = a.has_pk ? pk.slicer.n_slices : 0;
     size_t off[9];
     track_smem_layout<T>(Sa, Sp, a.n_hist, a.n_tables, a.kicks_smem, a.stages,
-                         TILE, off, true);
+                         TILE, off, kFixSingle);
     int* hcnt = reinterpret_cast<int*>(smem + off[0]);
     int* fdig = reinterpret_cast<int*>(smem + off[1]);
     unsigned* fflag = reinterpret_cast<unsigned*>(smem + off[2]);
@@ -2022,7 +2027,7 @@ static inline size_t smem_for(int Sa, int Sp, int n_tables, bool tma,
     auto bytes = [&](int st) {
         size_t off[9];
         return track_smem_layout<float>(Sa, Sp, 1, n_tables, *kicks_smem, st, tile,
-                                        off, true);
+                                        off, kFixSingle);
     };
     if (tma) {
         const size_t budget = budget_in ? budget_in : kF32SmemBudget;
@@ -2300,15 +2305,16 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
     __shared__ DetFix s_det[F64 ? PHK_MAX_DETUNERS : 1];
     unsigned char* rest = smem + batch_head<T>();
     size_t off[9];
-    track_smem_layout<T>(Sa, Sp, a.n_hist, nk, 1, 0, TILE, off, FIX);
-    // FIX: one set of counters per CTA, level B in the partial column
+    track_smem_layout<T>(Sa, Sp, a.n_hist, nk, 1, 0, TILE, off, FIX ? kFixBatch : 0);
+    // FIX: one set of counters per CTA
     double* hsx = reinterpret_cast<double*>(rest + off[0]);
     double* hsy = reinterpret_cast<double*>(rest + off[1]);
     int* hcnt = reinterpret_cast<int*>(rest + (FIX ? off[0] : off[2]));
     int* fdig = reinterpret_cast<int*>(rest + off[1]);
-    unsigned* fflag = reinterpret_cast<unsigned*>(rest + off[2]);
-    __shared__ FixSpill s_spill;
-    __shared__ unsigned s_max[2];
+    constexpr int WARPS = THREADS / 32;
+    __shared__ Spill64 s_spill;
+    __shared__ Seen<WARPS> s_seen;
+    __shared__ unsigned s_typ[2];
     T* eacc = reinterpret_cast<T*>(rest + off[3]);
     T* epk = reinterpret_cast<T*>(rest + off[4]);
     T* ktab = reinterpret_cast<T*>(rest + off[5]);
@@ -2322,8 +2328,7 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
     auto clear = [&]() {
         if constexpr (FIX) {
             for (int i = tid; i < Sa; i += THREADS) hcnt[i] = 0;
-            for (int i = tid; i < 4 * Sa; i += THREADS) fdig[i] = 0;
-            for (int i = tid; i < (Sa + 3) / 4; i += THREADS) fflag[i] = 0u;
+            for (int i = tid; i < 6 * Sa; i += THREADS) fdig[i] = 0;
         } else {
             for (int i = tid; i < a.n_hist * Sa; i += THREADS) {
                 hsx[i] = 0.0; hsy[i] = 0.0;
@@ -2338,7 +2343,8 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
     }
     if (F64) stage_sine(sine, tid, THREADS);
 
-    TrackCtx<T, VEC> cx;
+    using H = typename std::conditional<FIX, FixHist32, FixHist64>::type;
+    TrackCtx<T, VEC, H> cx;
     cx.aux = Aux64{sine, s_op, s_det};
 #pragma unroll
     for (int q = 0; q < 6; ++q) cx.cp[q] = reinterpret_cast<T*>(a.c[q]);
@@ -2346,10 +2352,9 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
     if constexpr (FIX) {
         cx.fix.cnt = hcnt;
         cx.fix.dig = fdig;
-        cx.fix.flag = fflag;
         cx.fix.sp = &s_spill;
         cx.fix.S = Sa;
-        cx.fix.scale[0] = cx.fix.scale[1] = 1.f;
+        if (tid < 2 * WARPS) s_seen.in[tid / WARPS][tid % WARPS] = 0u;   // no sample
     } else {
         const int h = (a.n_hist > 1) ? (tid >> 5) % a.n_hist : 0;
         cx.hx = hsx + h * Sa;
@@ -2371,7 +2376,9 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
         u0 = u1 = 0;
     }
     int cur = -1, col = -1;
-    int tiles = -1;              // FIX: since the last carry; -1: a new run
+    constexpr int kTiles = kDigitValues / TILE;
+    int until_carry = kTiles;    // FIX
+    bool open = false;           // FIX: a window is still to be set
     // write the CTA's sums of the current bunch to its column, then zero
     auto flush = [&]() {
         __syncthreads();
@@ -2381,13 +2388,10 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
             int c = hcnt[s];
             double v[2];
             if constexpr (FIX) {
-                const unsigned fl = (fflag[s >> 2] >> (8 * (s & 3))) & 0xffu;
 #pragma unroll
                 for (int q = 0; q < 2; ++q)
-                    v[q] = fix_value(
-                        __ldcg(s_spill.spill[q] + (int64_t)s * G) +
-                            FixHist::total(fdig + 2 * q * Sa + s, Sa),
-                        q ? fl >> 4 : fl & 15u, cx.fix.scale[q]);
+                    v[q] = __ldcg(s_spill.sum[q] + (int64_t)s * G) +
+                           digits32_value(fdig + 3 * q * Sa + s, Sa, cx.fix.top[q], c);
             } else {
                 v[0] = hsx[s];
                 v[1] = hsy[s];
@@ -2447,18 +2451,19 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
             }
             cur = U.bunch;
             col = U.column;
-            if (FIX && a.has_acc) {
-                const int G = b.n_columns;
-                long long* P = reinterpret_cast<long long*>(acc.partials);
+            if constexpr (FIX) if (a.has_acc) {
+                const int64_t G = b.n_columns;
+                double* P = acc.partials + col;
                 if (tid == 0) {
-                    s_spill.spill[0] = P + (int64_t)Sa * G + col;
-                    s_spill.spill[1] = P + (int64_t)2 * Sa * G + col;
+                    s_spill.sum[0] = P + Sa * G;
+                    s_spill.sum[1] = P + 2 * Sa * G;
                     s_spill.stride = G;
-                    s_max[0] = s_max[1] = 0u;
+                    s_typ[0] = s_typ[1] = 0u;
                 }
-                for (int s = tid; s < 2 * Sa; s += THREADS)
-                    P[(int64_t)(Sa + s) * G + col] = 0;
-                tiles = -1;
+                for (int s = tid; s < 2 * Sa; s += THREADS) P[(Sa + s) * G] = 0.0;
+                cx.fix.top[0] = cx.fix.top[1] = 0.f;
+                until_carry = kTiles;
+                open = true;
             }
             __syncthreads();
         }
@@ -2471,34 +2476,33 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
             load_tile_plain<T, VEC>(ua, cx, t, i0, full);
             tile_advance<T, VEC, SHAPE, false>(*sprog, pk, ua, cx, t, i0);
             if constexpr (FIX) {
-                if (a.has_acc && tiles < 0) {
-                    // the scale of the run, from its first tile
+                if (open) {
                     unsigned m[2] = {0u, 0u};
 #pragma unroll
-                    for (int j = 0; j < VEC; ++j) {
-                        const unsigned x = __float_as_uint(fabsf(t.c[PHK_X][j]));
-                        const unsigned y = __float_as_uint(fabsf(t.c[PHK_Y][j]));
-                        if (i0 + j < ua.n && x < 0x7f800000u) m[0] = max(m[0], x);
-                        if (i0 + j < ua.n && y < 0x7f800000u) m[1] = max(m[1], y);
-                    }
+                    for (int j = 0; j < VEC; ++j)
+                        if (i0 + j < ua.n) {
+                            m[0] = max(m[0], finite_high(t.c[PHK_X][j]));
+                            m[1] = max(m[1], finite_high(t.c[PHK_Y][j]));
+                        }
+                    open = find_typical<WARPS>(&s_seen, s_typ, m[0], m[1]);
 #pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        m[q] = __reduce_max_sync(~0u, m[q]);
-                        if ((tid & 31) == 0) atomicMax(s_max + q, m[q]);
-                    }
+                    for (int q = 0; q < 2; ++q)
+                        if (cx.fix.top[q] == 0.f && s_typ[q]) {
+                            cx.fix.top[q] = digit_top(s_typ[q]);
+                            open_digits32(hcnt, fdig + 3 * q * Sa, Sa, cx.fix.top[q]);
+                        }
                     __syncthreads();
-                    cx.fix.scale[0] = fix_scale(s_max[0]);
-                    cx.fix.scale[1] = fix_scale(s_max[1]);
-                    tiles = 0;
-                } else if (a.has_acc && tiles == fix_flush_tiles<TILE>()) {
-                    __syncthreads();
-                    fix_flush(cx.fix, tid, THREADS);
-                    __syncthreads();
-                    tiles = 0;
                 }
-                ++tiles;
             }
             tile_finish<T, VEC, false, FIX>(acc, ua, cx, t, i0, full);
+            if constexpr (FIX) {
+                if (a.has_acc && --until_carry == 0) {
+                    // before a counter can overflow in the next kTiles tiles
+                    until_carry = kTiles;
+                    carry_slices32(hcnt, fdig, Sa, kDigitValues - kTiles * TILE, &s_spill,
+                                   s_typ);
+                }
+            }
         }
     }
     if (cur >= 0 && a.has_acc) flush();
@@ -2513,7 +2517,7 @@ static size_t batch_smem(int Sa, int Sp, int nk, int threads, int* n_hist) {
     const int warps = threads / 32;
     // FP32: one set of fixed-point counters; FP64: one private histogram copy
     // per warp when it stays within 48 KB
-    constexpr bool fix = sizeof(T) == 4;
+    constexpr int fix = sizeof(T) == 4 ? kFixBatch : 0;
     int nh = Sa > 0 && !fix ? warps : 1;
     size_t bytes = track_smem_layout<T>(Sa, Sp, nh, nk, 1, 0, tile, off, fix);
     if (bytes > 48 * 1024 && Sa > 0 && !fix) {

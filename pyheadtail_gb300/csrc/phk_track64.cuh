@@ -40,51 +40,16 @@ __host__ __device__ inline Track64Smem track64_smem(int Sa, int Sp, int n_tables
     return m;
 }
 
-// The parts of the tile loop that seldom run are out of line: the loop fills
-// the instruction cache as it is (inlined, they cost 5 % of a pass).
-
-// What the warps of a CTA saw at most of x and y (high words): of a sample of
-// the inputs, and of the outputs of a tile
-struct Seen64 {
-    unsigned in[2][kTrackThreads / 32], out[2][kTrackThreads / 32];
-};
-__device__ __forceinline__ void note_seen(unsigned (*to)[kTrackThreads / 32],
-                                          unsigned mx, unsigned my) {
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    my = __reduce_max_sync(0xffffffffu, my);
-    if ((threadIdx.x & 31) == 0) {
-        to[0][threadIdx.x >> 5] = mx;
-        to[1][threadIdx.x >> 5] = my;
-    }
-}
-
-// The windows: the larger of the typical input, of a sample spread over the
-// bunch, and the typical output of this tile (a bunch that starts on the axis,
-// a large beta at the end of the turn); where both are zero, they stay as they
-// are and the next tile is looked at.  mx, my: largest of this thread's.  All
-// threads of the CTA call it; true if a window is still open.
-static __device__ __noinline__ bool set_windows(Seen64* seen, int* base, unsigned mx,
-                                                unsigned my) {
-    constexpr int WARPS = kTrackThreads / 32;
-    note_seen(seen->out, mx, my);
-    __syncthreads();
-    const int q = (threadIdx.x >> 5) & 1;
-    const unsigned typ = max(typical_of<WARPS>(seen->in[q]), typical_of<WARPS>(seen->out[q]));
-    if ((threadIdx.x & ~32u) == 0 && base[q] == kNoBase) base[q] = digit_base(typ, 18);
-    __syncthreads();
-    return base[0] == kNoBase || base[1] == kNoBase;
-}
-
 // Carries the digits of the slices with more than `most` values (all threads)
 static __device__ __noinline__ void carry_slices(int* words, int S, int most,
-                                                 const Spill64* sp, const int* base) {
+                                                 const Spill64* sp, const unsigned* typ) {
     __syncthreads();
     for (int s = threadIdx.x; s < S; s += kTrackThreads) {
         int* w = words + s * kFix64Words;
         if (w[0] <= most) continue;
         for (int q = 0; q < 2; ++q) {
             const int top = carry_digits(w + 1 + 4 * q);
-            if (top) spill64(sp, q, s, top_value(top, base[q]));
+            if (top) spill64(sp, q, s, top_value(top, digit_base(typ[q], 18)));
         }
     }
     __syncthreads();
@@ -102,8 +67,9 @@ track64_kernel(const __grid_constant__ phk_program prog,
                const __grid_constant__ Track64Args ka) {
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ Seen64 s_seen;
-    __shared__ int s_base[2];       // windows of x and y
+    constexpr int WARPS = kTrackThreads / 32;
+    __shared__ Seen<WARPS> s_seen;
+    __shared__ unsigned s_typ[2];   // typical |x|, |y|
     __shared__ Spill64 s_spill;
     constexpr int TILE = kTrackThreads * VEC;
     const TrackArgs& a = ka.t;
@@ -143,8 +109,8 @@ track64_kernel(const __grid_constant__ phk_program prog,
     if (a.has_pk)
         stage_pending<double>(pk, a, epk, ktab, tid, kTrackThreads, ka.share_edges);
     if (ka.sine) stage_sine(sine, tid, kTrackThreads);
-    if (a.has_acc) note_seen(s_seen.in, m_in[0], m_in[1]);
-    if (tid < 2) s_base[tid] = kNoBase;
+    if (a.has_acc) note_seen<WARPS>(s_seen.in, m_in[0], m_in[1]);
+    if (tid < 2) s_typ[tid] = 0u;
     __syncthreads();
     if (a.has_pk) cx.bpk.init(epk, Sp, pk.slicer.negate);
     if (a.has_acc) cx.bac.init(eacc, Sa, acc.slicer.negate);
@@ -191,16 +157,16 @@ track64_kernel(const __grid_constant__ phk_program prog,
                     m[0] = max(m[0], finite_high(t.c[PHK_X][j]));
                     m[1] = max(m[1], finite_high(t.c[PHK_Y][j]));
                 }
-            open = set_windows(&s_seen, s_base, m[0], m[1]);
-            cx.fix.base[0] = s_base[0];
-            cx.fix.base[1] = s_base[1];
+            open = find_typical<WARPS>(&s_seen, s_typ, m[0], m[1]);
+            cx.fix.base[0] = digit_base(s_typ[0], 18);
+            cx.fix.base[1] = digit_base(s_typ[1], 18);
         }
         tile_finish<double, VEC, false, true>(acc, a, cx, t, i0, i0 + VEC <= a.n);
         load_tile_plain<double, VEC>(a, cx, t, i0 + step, i0 + step + VEC <= a.n);
         if (a.has_acc && --until_carry == 0) {
             // before a counter can overflow in the next kTiles tiles
             until_carry = kTiles;
-            carry_slices(words, Sa, kDigitValues - kTiles * TILE, &s_spill, s_base);
+            carry_slices(words, Sa, kDigitValues - kTiles * TILE, &s_spill, s_typ);
         }
     }
     if (!a.has_acc) return;
@@ -228,16 +194,17 @@ track64_kernel(const __grid_constant__ phk_program prog,
             for (int r = 0; r < kCluster; ++r) {
                 if (r >= (int)nb) break;
                 const int* w = words;
-                const int* base = s_base;
+                const unsigned* typ = s_typ;
                 if (clustered) {
                     w = cg::this_cluster().map_shared_rank(words, r);
-                    base = cg::this_cluster().map_shared_rank(s_base, r);
+                    typ = cg::this_cluster().map_shared_rank(s_typ, r);
                 }
                 w += s * kFix64Words;
                 c += w[0];
 #pragma unroll
                 for (int q = 0; q < 2; ++q)
-                    v[q] = add(v[q], digits_value(w + 1 + 4 * q, base[q]));
+                    v[q] = add(v[q], digits_value(w + 1 + 4 * q,
+                                                  digit_base(typ[q], 18)));
             }
             P[s * G] = (double)c;
             P[(Sa + s) * G] = v[0];
