@@ -578,6 +578,10 @@ int launch_track_batch(const phk_batch* bt, const phk_coords* c,
 }
 
 int batch_max_grid(int32_t dtype, int32_t threads, int32_t S, int32_t nk) {
+    // phk_track_batch refuses kick tables beyond 48 KB: they do not narrow the
+    // grid of the turns without kicks
+    const int most = 48 * 1024 / (S * (dtype == PHK_F64 ? 8 : 4));
+    if (nk > most) nk = most;
     int nh = 0;
     int per_sm = 0;
     if (dtype == PHK_F64)
