@@ -283,23 +283,15 @@ int launch_slice_merge(const double* sums, int n_shards, int S,
 // wake convolution
 // ===================================================================
 
-struct WakeArgs {
-    phk_wake_set w;
-};
-
-// numpy path: one warp per (kick, target slice); lanes split the sources.
-// Each lane keeps its partial sums over every stored turn and the warp
-// reduces once at the end (the reference sums each turn's convolution,
-// then the turns: the same terms, regrouped; GB300's FP64 pipe makes the
-// per-turn reductions the larger part of the cost otherwise).
-__device__ __forceinline__ void wake_conv_one(const phk_wake_set& w, int gw,
+// numpy path: one warp for target slice i of kick k; lanes split the sources.
+// Each lane keeps its partial sums over every stored turn and the warp reduces
+// once at the end (the reference sums each turn's convolution, then the turns:
+// the same terms, regrouped; GB300's FP64 pipe makes the per-turn reductions the
+// larger part of the cost otherwise).
+__device__ __forceinline__ void wake_conv_one(const phk_wake_set& w, int k, int i,
                                               int lane) {
     const int S = w.n_slices;
-    const int k = gw / S;
-    const int i = gw - k * S;
-    if (k >= w.n_kicks) return;
     const phk_wake_kick& kk = w.kick[k];
-    if (kk.dense) return;
     const int L2 = 2 * S - 1;
     double p0 = 0.0, p1 = 0.0, p2 = 0.0, p3 = 0.0;
     int slot = (w.head % w.ring_len + w.ring_len) % w.ring_len;
@@ -643,14 +635,49 @@ int launch_batch_finalize(const phk_accum* acc, int nb, const int32_t* bcols,
     return PHK_OK;
 }
 
+// The sum of one lane's target over the sources [j0, j1) of every stored turn, in
+// SETS x 4 chains.  The sample of source j: v[j dj], of the next turn `row` on.
+template <int SETS>
+__device__ __forceinline__ double target_sum(const phk_wake_set& w, const phk_wake_kick& kk,
+                                             const double* v, int64_t row, int64_t dj,
+                                             int j0, int j1) {
+    double p[SETS][4] = {};
+    int slot = (w.head % w.ring_len + w.ring_len) % w.ring_len;
+    for (int a = 0; a < kk.n_lags; ++a, v += row) {
+        const double* m = w.moments + ((int64_t)slot * 3 + kk.source) * w.n_slices;
+        int j = j0;
+        auto four = [&](double (&q)[4]) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                q[u] = fma(__ldg(m + j + u), __ldg(v + (j + u) * dj), q[u]);
+            j += 4;
+        };
+        while (j + 4 * SETS - 1 < j1)
+#pragma unroll
+            for (int t = 0; t < SETS; ++t) four(p[t]);
+#pragma unroll
+        for (int t = 1; t < SETS; ++t)
+            if (j + 3 < j1) four(p[t]);
+        for (; j < j1; ++j) p[0][0] = fma(__ldg(m + j), __ldg(v + j * dj), p[0][0]);
+        slot = slot == 0 ? w.ring_len - 1 : slot - 1;
+    }
+    double sum = 0.0;
+#pragma unroll
+    for (int t = 0; t < SETS; ++t) {
+        const double q = (p[t][0] + p[t][1]) + (p[t][2] + p[t][3]);
+        sum = t ? sum + q : q;
+    }
+    return sum;
+}
+
 // One CTA per (bunch, kick, 32 target slices): lanes are targets, the warps
-// split the sources of every stored turn, four sums in flight each; fixed
-// order.  Bound by FP64: a warp per target spent 9 of its 13 additions on
-// adding its lanes up (64 bunches, 2 kicks, 100 slices: 19 us, now 9.2).  Above
-// kBatchTerms terms per target that share is small, and the lane-split sums
-// (wake_conv_one) have the shorter chains: those targets go one to a warp.
+// split the sources of every stored turn, four sums in flight each (16 above 512
+// terms per target, so that the chains stay short); fixed order.  Bound by FP64:
+// a warp per target spent 9 of its 13 additions on adding its lanes up (64
+// bunches, 2 kicks, 100 slices: 15.5 us, now 7.1; 500 slices 145 / 63; 100 slices
+// of six turns 40 / 27).
 constexpr int kBatchWarps = 8;
-constexpr int kBatchTerms = 512;
+constexpr int kFewTerms = 128;
 
 __global__ void __launch_bounds__(kBatchWarps * 32)
 batch_wake_kernel(const phk_wake_set* __restrict__ sets, int nb, int S, int nk) {
@@ -666,30 +693,23 @@ batch_wake_kernel(const phk_wake_set* __restrict__ sets, int nb, int S, int nk) 
     if (k >= w.n_kicks) return;
     const phk_wake_kick& kk = w.kick[k];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (!kk.dense && (int64_t)kk.n_lags * S > kBatchTerms) {
-        for (int i = i0 + warp; i < i0 + 32 && i < S; i += kBatchWarps)
-            wake_conv_one(w, k * S + i, lane);
-        return;
+    const int64_t n_terms = (int64_t)kk.n_lags * S;
+    if (gridDim.y > 1) {        // few bunches, see launch_wake_batch
+        if (!kk.dense && n_terms > kFewTerms) {
+            const int i = i0 + blockIdx.y * kBatchWarps + warp;
+            if (i < S) wake_conv_one(w, k, i, lane);
+            return;
+        }
+        if (blockIdx.y) return;
     }
     const int i = i0 + lane < S ? i0 + lane : S - 1;
     const int j0 = S * warp / kBatchWarps, j1 = S * (warp + 1) / kBatchWarps;
-    // the sample of source j: numpy path table[i + S - 1 - j], dot path [j][i]
+    // numpy path: table[i + S - 1 - j], dot path [j][i]
     const int64_t row = kk.dense ? (int64_t)S * S : 2 * S - 1;
     const int64_t dj = kk.dense ? S : -1;
     const double* v = kk.table + i + (kk.dense ? 0 : S - 1);
-    double p[4] = {0.0, 0.0, 0.0, 0.0};
-    int slot = (w.head % w.ring_len + w.ring_len) % w.ring_len;
-    for (int a = 0; a < kk.n_lags; ++a, v += row) {
-        const double* m = w.moments + ((int64_t)slot * 3 + kk.source) * S;
-        int j = j0;
-        for (; j + 3 < j1; j += 4)
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                p[u] = fma(__ldg(m + j + u), __ldg(v + (j + u) * dj), p[u]);
-        for (; j < j1; ++j) p[0] = fma(__ldg(m + j), __ldg(v + j * dj), p[0]);
-        slot = slot == 0 ? w.ring_len - 1 : slot - 1;
-    }
-    part[warp][lane] = (p[0] + p[1]) + (p[2] + p[3]);
+    part[warp][lane] = n_terms <= 512 ? target_sum<1>(w, kk, v, row, dj, j0, j1)
+                                      : target_sum<4>(w, kk, v, row, dj, j0, j1);
     __syncthreads();
     if (warp != 0 || i0 + lane >= S) return;
     double t[kBatchWarps];
@@ -709,7 +729,13 @@ batch_wake_kernel(const phk_wake_set* __restrict__ sets, int nb, int S, int nk) 
 int launch_wake_batch(const phk_wake_set* sets, int nb, int S, int nk,
                       cudaStream_t st) {
     const int64_t blocks = (int64_t)nb * nk * ((S + 31) / 32);
-    batch_wake_kernel<<<(unsigned)blocks, kBatchWarps * 32, 0, st>>>(sets, nb, S, nk);
+    // Where the blocks leave half of the SMs idle, four CTAs share a block's
+    // targets, one to a warp, from kFewTerms terms on (2 bunches, 200 slices of 50 turns:
+    // 147 us on one CTA, now 47; 1 bunch, 500 slices of one turn 7.3 / 4.9; 100
+    // slices are better left together, 3.3 / 3.5).
+    const bool few = 2 * blocks <= device_info().sm_count;
+    batch_wake_kernel<<<dim3((unsigned)blocks, few ? 32 / kBatchWarps : 1), kBatchWarps * 32,
+                        0, st>>>(sets, nb, S, nk);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return set_error(PHK_ECUDA, "phk_wake_batch launch: %s",
