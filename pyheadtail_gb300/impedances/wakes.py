@@ -396,7 +396,7 @@ class ResistiveWall(WakeSource):
                       np.pi / self.pipe_radius**3)
             num = -mu_r / np.pi / self.conductivity
             dt_min = abs(self.dt_min)
-            if (self.pipe_radius.size != 1 or before.shape != (3,) or
+            if (np.size(self.pipe_radius) != 1 or before.shape != (3,) or
                     np.ndim(num) or np.ndim(dt_min) or
                     not np.all(np.isfinite(before)) or
                     not -np.inf < num < 0 or not 0 < dt_min < np.inf):
