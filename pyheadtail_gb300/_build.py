@@ -44,6 +44,7 @@ def _stale():
     t = os.path.getmtime(LIB)
     deps = (sources() + glob.glob(os.path.join(CSRC, '*.h')) +
             glob.glob(os.path.join(CSRC, '*.cuh')) +
+            glob.glob(os.path.join(CSRC, '*.inc')) +
             glob.glob(os.path.join(INCLUDE, '*.h')) + [__file__])
     return any(os.path.getmtime(d) > t for d in deps)
 
