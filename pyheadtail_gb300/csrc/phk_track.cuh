@@ -94,9 +94,11 @@ __host__ __device__ inline void op_fix(const phk_op& op, OpFix* r) {
         double off = 0.0;
         if (f & PHK_FLAG_PHI_OFFSET) off += p[3];
         if (f & PHK_FLAG_PHI_LOCK) off += p[4];
-        // no usable factor: every particle takes the library's sine
-        if (!turn_factor(p[0], p[2], &r->k)) r->k.exp = -(1 << 20);
-        r->off = angle_fraction(off);
+        // no usable factor, an offset that is not finite or far beyond a turn:
+        // every particle takes the library's sine
+        const bool far = !turn_factor(p[0], p[2], &r->k) || !(fabs(off) < 0x1p31);
+        if (far) r->k.exp = -(1 << 20);
+        r->off = far ? 0 : angle_fraction(off);
         r->c[0] = p[5] * p[12] * 0x1p-62;
         r->c[1] = p[6] == p[8] ? 1.0 : p[6] * p[12];
         r->c[2] = (f & PHK_FLAG_P_INC) ? p[7] * p[12] : 0.0;
