@@ -512,7 +512,7 @@ __device__ __forceinline__ u64 turn_fraction(double t) {
 struct TurnFactor {
     u64 mant;
     int32_t exp;
-    int32_t reserved;
+    int32_t span;       // RF kick: exponents of z that the fixed-point sine takes
 };
 
 // num / den as 64 significant bits: the quotient and, from its exact
@@ -526,7 +526,7 @@ __host__ __device__ inline bool turn_factor(double num, double den, TurnFactor* 
     k->mant = ((u64)(m * 9007199254740992.0) << 11) +
               (u64)(long long)rint(ldexp(lo, 64 - e));
     k->exp = 64 - e;
-    k->reserved = 0;
+    k->span = 0;
     return true;
 }
 

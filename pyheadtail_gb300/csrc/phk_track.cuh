@@ -98,6 +98,7 @@ __host__ __device__ inline void op_fix(const phk_op& op, OpFix* r) {
         // every particle takes the library's sine
         const bool far = !turn_factor(p[0], p[2], &r->k) || !(fabs(off) < 0x1p31);
         if (far) r->k.exp = -(1 << 20);
+        r->k.span = fabs(off) < 0x1p-8 ? 21 : 4096;
         r->off = far ? 0 : angle_fraction(off);
         r->c[0] = p[5] * p[12] * 0x1p-62;
         r->c[1] = p[6] == p[8] ? 1.0 : p[6] * p[12];
@@ -432,10 +433,30 @@ __device__ __forceinline__ void op_drift_rf(const OpFix& f, Tile<double, VEC>& t
         t.c[PHK_Z][j] = fma(-f.c[0], t.c[PHK_DP][j], t.c[PHK_Z][j]);
 }
 
-// phase of 2^9 turns and more, NaN and infinities (and factors without a
-// fixed-point form): the sine times 2^62
-static __device__ __noinline__ double rf_sine_far(double z, double hk, double off) {
-    return sin(fma(hk, z, off)) * 0x1p62;
+// The sine, times 2^62, of what the fixed point does not hold to 53 bits.  Phases
+// below about 2^-10 without an offset (sine_turn's error is at most 2^-61,
+// whatever the sine): the significand of the phase keeps its 62 bits, times 1 -
+// theta^2/6 + theta^4/120 (next term 2^-66).  Phases of 2^9 turns and more, NaN,
+// infinities, small phases beside a small offset: the library's sine.  One warp
+// in forty comes here at a bunch length of a radian (1 % of a pass; without, the
+// kick of a particle at a phase of 1e-10 was off by 4e-9 of itself).
+static __device__ __noinline__ double rf_sine_cold(double z, u64 kmant, int kexp, double hk,
+                                                   double off) {
+    const int hi = __double2hiint(z), lo = __double2loint(z);
+    const int be = biased_exp(hi);
+    if (z == 0.0 && off == 0.0) return 0.0;
+    if (off != 0.0 || be > 968 + kexp || be < 200) return sin(fma(hk, z, off)) * 0x1p62;
+    const u64 m = __umul64hi(mant64(hi, lo), kmant);
+    const int r = 958 + kexp - be;                        // phase: m 2^(-64 - r) turns
+    const u64 th = __umul64hi(m, 0xc90fdaa22168c235ull);  // theta, units of 2^(-61 - r)
+    const u64 x = shr_clamp(th, r - 5);                   // 2^-66
+    const u64 q = __umul64hi(x, x);                       // theta^2, 2^-68
+    const unsigned q4 = __umulhi((unsigned)(q >> 20), (unsigned)(q >> 20));   // 2^-64
+    const u64 c = __umul64hi(q, 0x2aaaaaaaaaaaaaabull) -
+                  ((u64)__umulhi(q4, 0x02222222u) << 4);
+    const double s = (double)(th - (__umul64hi(th, c) >> 4));
+    return __hiloint2double((__double2hiint(s) + ((1 - r) << 20)) | (hi & 0x80000000),
+                            __double2loint(s));
 }
 
 // RF kick, plain form.  The per-particle sine makes the step inexact whatever
@@ -459,14 +480,14 @@ __device__ __forceinline__ void op_rfkick(const phk_op& op, const OpFix& f,
         }
         const double z = t.c[PHK_Z][j];
         double s;      // sine, times 2^62
-        if (biased_exp(__double2hiint(z)) <= 968 + f.k.exp) {
+        if ((unsigned)(968 + f.k.exp - biased_exp(__double2hiint(z))) <= (unsigned)f.k.span) {
             unsigned sign;
             const u64 m = sine_turn(sine, turn_product(z, f.k.mant, f.k.exp) + f.off, &sign);
             s = (double)(long long)m;
             s = __hiloint2double((int)((unsigned)__double2hiint(s) | sign),
                                  __double2loint(s));
         } else {
-            s = rf_sine_far(z, f.c[3], f.c[4]);
+            s = rf_sine_cold(z, f.k.mant, f.k.exp, f.c[3], f.c[4]);
         }
         if (PLAIN) dp = fma(f.c[0], s, dp);
         else dp = fma(dp, f.c[1], fma(f.c[0], s, -f.c[2]));
