@@ -391,7 +391,10 @@ wake_direct_kernel(const __grid_constant__ phk_wake_set w) {
 // accuracy: each factor is off by at most 2^-54 of the largest in the window),
 // converts them into its part of shared memory and accumulates one target
 // per lane.  Warps, then CTAs, are added in a fixed order.  A unit with a
-// non-finite, subnormal or extreme factor runs in FP64 (conv_unit_fp64).
+// non-finite, subnormal or extreme factor runs in FP64 (conv_unit_fp64), one
+// whose moments or samples are all zero (empty slices, targets ahead of the
+// source) adds nothing: as FP64 units those took 25 of 47 us at 500 slices, 50
+// turns, a bunch within a tenth of the cuts.
 constexpr int kConvWarps = 16;
 constexpr int kConvCluster = 4;
 constexpr int kConvTargets = 32;    // per cluster, one per lane
@@ -459,15 +462,20 @@ wake_conv_kernel(const __grid_constant__ phk_wake_set w) {
             const int j = lane + 32 * q;
             mv[q] = j < len ? __ldg(m + j) : 0.0;
         }
+        // the low word counts for subnormals alone
         unsigned bt = 0u, bm = 0u;
 #pragma unroll
         for (int q = 0; q < NT; ++q)
-            bt = max(bt, (unsigned)__double2hiint(tv[q]) & 0x7fffffffu);
+            bt = max(bt, ((unsigned)__double2hiint(tv[q]) & 0x7fffffffu) |
+                             (__double2loint(tv[q]) != 0 ? 1u : 0u));
 #pragma unroll
         for (int q = 0; q < NM; ++q)
-            bm = max(bm, (unsigned)__double2hiint(mv[q]) & 0x7fffffffu);
-        const int et = (int)(__reduce_max_sync(0xffffffffu, bt) >> 20);
-        const int em = (int)(__reduce_max_sync(0xffffffffu, bm) >> 20);
+            bm = max(bm, ((unsigned)__double2hiint(mv[q]) & 0x7fffffffu) |
+                             (__double2loint(mv[q]) != 0 ? 1u : 0u));
+        bt = __reduce_max_sync(0xffffffffu, bt);
+        bm = __reduce_max_sync(0xffffffffu, bm);
+        if ((bt == 0u || bm == 0u) && max(bt, bm) < 0x7ff00000u) continue;   // zeros
+        const int et = (int)(bt >> 20), em = (int)(bm >> 20);
         const bool normal = et >= 100 && et < 2000 && em >= 100 && em < 2000 &&
                             et + em > 1100 && et + em < 3100;
         if (!normal) {
