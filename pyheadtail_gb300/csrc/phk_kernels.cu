@@ -387,14 +387,18 @@ wake_direct_kernel(const __grid_constant__ phk_wake_set w) {
 // One cluster of kConvCluster CTAs per (kick, block of 32 target slices); its
 // warps share the (stored turn, chunk of source slices) units.  A warp loads
 // a unit's sources and its window of the table, finds the largest magnitude
-// of each (the unit's own scales, so a decaying wake keeps its relative
-// accuracy: each factor is off by at most 2^-54 of the largest in the window),
-// converts them into its part of shared memory and accumulates one target
-// per lane.  Warps, then CTAs, are added in a fixed order.  A unit with a
-// non-finite, subnormal or extreme factor runs in FP64 (conv_unit_fp64), one
-// whose moments or samples are all zero (empty slices, targets ahead of the
-// source) adds nothing: as FP64 units those took 25 of 47 us at 500 slices, 50
-// turns, a bunch within a tenth of the cuts.
+// of each (the unit's own scales: each factor is off by at most 2^-54 of the
+// largest in the window), converts them into its part of shared memory and
+// accumulates one target per lane.  Warps, then CTAs, are added in a fixed
+// order.  A unit with a non-finite, subnormal or extreme factor runs in FP64
+// (conv_unit_fp64), one whose moments or samples are all zero adds nothing.
+//
+// A target whose terms are all far below its windows' largest (the head of a
+// bunch in a causal wake) would lose relative accuracy.  So every unit also notes
+// its error (rms, sqrt(sources) / 2 of the unit that its sum is rounded to) and
+// the magnitudes of every eighth source's terms.  An FP64 sum of n terms is off
+// by n 2^-53 of their magnitudes at most; a target whose noted errors exceed a
+// sixteenth of that is summed again in FP64.  The notes cost 2.5 us of 27.
 constexpr int kConvWarps = 16;
 constexpr int kConvCluster = 4;
 constexpr int kConvTargets = 32;    // per cluster, one per lane
@@ -416,6 +420,34 @@ __device__ __forceinline__ void conv_unit_fp64(const double* m, const double* ta
     for (int j = 0; j < len; ++j) acc = fma(m[j], tab[i - j], acc);
 }
 
+// Errors (squared, they are independent) and terms of integer units, in units of
+// 2^e
+struct ConvBound {
+    int e;
+    float error;
+    float terms[kConvTargets];
+};
+__device__ __forceinline__ float exp2_int(int d) {       // 2^d, d <= 0; 0 below 2^-126
+    return d < -126 ? 0.0f : __int_as_float((d + 127) << 23);
+}
+
+// The sum of n bounds for target t (32 threads of a warp)
+__device__ __forceinline__ void add_bounds(const ConvBound* b, int n, int t, ConvBound* sum) {
+    int e = b[0].e;
+    for (int q = 1; q < n; ++q) e = max(e, b[q].e);
+    float error = 0.0f, terms = 0.0f;
+    for (int q = 0; q < n; ++q) {
+        const float down = exp2_int(max(b[q].e - e, -1000));
+        error += b[q].error * down * down;
+        terms += b[q].terms[t] * down;
+    }
+    sum->terms[t] = terms;
+    if (t == 0) {
+        sum->e = e;
+        sum->error = error;
+    }
+}
+
 __global__ void __cluster_dims__(kConvCluster, 1, 1) __launch_bounds__(kConvWarps * 32)
 wake_conv_kernel(const __grid_constant__ phk_wake_set w) {
     namespace cg = cooperative_groups;
@@ -423,6 +455,9 @@ wake_conv_kernel(const __grid_constant__ phk_wake_set w) {
     __shared__ int2 s_mom[kConvWarps][kConvSources];
     __shared__ double s_acc[kConvWarps][kConvTargets];
     __shared__ double s_sum[kConvTargets];
+    __shared__ ConvBound s_bound[kConvWarps];
+    __shared__ ConvBound s_all;
+    __shared__ unsigned s_again;        // targets to sum in FP64
     cg::cluster_group cl = cg::this_cluster();
     const unsigned rank = cl.block_rank();
     const int S = w.n_slices;
@@ -439,6 +474,8 @@ wake_conv_kernel(const __grid_constant__ phk_wake_set w) {
     const int chunks = (S + per - 1) / per;
     const int units = work ? kk.n_lags * chunks : 0;
     double acc = 0.0;
+    int be = -(1 << 20);                 // this warp's ConvBound
+    float error = 0.0f, terms = 0.0f;
     for (int u = warp * kConvCluster + rank; u < units; u += kConvWarps * kConvCluster) {
         const int a = u / chunks, j0 = (u - a * chunks) * per;
         const int len = min(per, S - j0);
@@ -490,7 +527,7 @@ wake_conv_kernel(const __grid_constant__ phk_wake_set w) {
 #pragma unroll
         for (int q = 0; q < NM; ++q) s_mom[warp][lane + 32 * q] = conv_limbs(mv[q], em);
         __syncwarp();
-        long long hh = 0, mid = 0, mil = 0, ll = 0;
+        long long hh = 0, mid = 0, mil = 0, ll = 0, mag = 0;
         const int2* tp = &s_tab[warp][lane + len - 1];
         const int2* mp = s_mom[warp];
 #pragma unroll 8
@@ -500,27 +537,97 @@ wake_conv_kernel(const __grid_constant__ phk_wake_set w) {
             mid += (long long)f.y * t.x;
             mil += (long long)f.x * t.y;
             ll += (long long)f.x * t.x;
+            if (j % 8 == 0) mag += (long long)abs(f.y) * abs(t.y);
         }
+        // unit: 2^(et + em - 2099), a product of high limbs is twice that
+        if (et + em > be) {
+            const float down = exp2_int(be - (et + em));
+            error *= down * down;
+            terms *= down;
+            be = et + em;
+        }
+        const float here = exp2_int(et + em - be);
+        error += here * here * 0.25f * (float)len;
+        terms += here * 2.0f * (float)mag;
         // sum = hh 2^54 + mid 2^27 + ll in units of 2^(et + em - 2152); in
         // units of 2^53 of these it fits 63 bits: one rounding
         const double unit = __hiloint2double((et + em - 1076) << 20, 0);
         acc = fma((double)((hh << 1) + ((mid + mil + (ll >> 27)) >> 26)), unit, acc);
     }
     s_acc[warp][lane] = acc;
+    s_bound[warp].terms[lane] = terms;
+    if (lane == 0) {
+        s_bound[warp].e = be;
+        s_bound[warp].error = error;
+    }
     __syncthreads();
     if (threadIdx.x < kConvTargets) {
         double sum = s_acc[0][threadIdx.x];
         for (int q = 1; q < kConvWarps; ++q) sum += s_acc[q][threadIdx.x];
         s_sum[threadIdx.x] = sum;
+        add_bounds(s_bound, kConvWarps, threadIdx.x, &s_all);
     }
     cl.sync();
-    if (rank == 0 && threadIdx.x < kConvTargets && work) {
-        const int i = i0 + threadIdx.x;
-        double sum = s_sum[threadIdx.x];
-        for (int r = 1; r < kConvCluster; ++r)
-            sum += cl.map_shared_rank(s_sum, r)[threadIdx.x];
-        if (i < S) {
+    // ---- every CTA finds the targets to sum again, rank 0 stores the others
+    if (work && threadIdx.x < kConvTargets) {
+        __shared__ ConvBound s_each[kConvCluster], s_total;
+        for (int r = 0; r < kConvCluster; ++r) {
+            const ConvBound* o = cl.map_shared_rank(&s_all, r);
+            s_each[r].terms[lane] = o->terms[lane];
+            if (lane == 0) {
+                s_each[r].e = o->e;
+                s_each[r].error = o->error;
+            }
+        }
+        __syncwarp();
+        add_bounds(s_each, kConvCluster, lane, &s_total);
+        __syncwarp();
+        const int i = i0 + lane;
+        const bool again = sqrtf(s_total.error) >
+                               s_total.terms[lane] * 0x1p-57f * (float)(kk.n_lags * S) &&
+                           i < S;
+        const unsigned mask = __ballot_sync(0xffffffffu, again);
+        if (lane == 0) s_again = mask;
+        if (rank == 0 && i < S && !again) {
+            double sum = s_sum[lane];
+            for (int r = 1; r < kConvCluster; ++r) sum += cl.map_shared_rank(s_sum, r)[lane];
             const double r = mul(kk.factor, sum);
+            if (w.out_dtype == PHK_F64)
+                reinterpret_cast<double*>(kk.out)[i] = r;
+            else
+                reinterpret_cast<float*>(kk.out)[i] = (float)r;
+        }
+    }
+    __syncthreads();
+    // ---- in FP64: this CTA's share of these targets, side by side, the warps
+    // divided among them
+    unsigned mine = work ? s_again & (0x11111111u << rank) : 0u;
+    if (mine) {
+        const int count = __popc(mine);
+        const int per_target = kConvWarps >> (count > 4 ? 3 : count > 2 ? 2 : count - 1);
+        const int which = warp / per_target, part = warp % per_target;
+        for (int n = 0; n < which; ++n) mine &= mine - 1u;
+        const int i = i0 + __ffs(mine) - 1;
+        double p[4] = {0.0, 0.0, 0.0, 0.0};
+        const int n_terms = which < count ? kk.n_lags * S : 0, step = 32 * per_target;
+        for (int n0 = 32 * part + lane; n0 < n_terms; n0 += 4 * step)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {          // four loads in flight
+                const int n = n0 + u * step;
+                const int a = n / S, j = n - a * S;
+                const int slot = ((w.head - a) % w.ring_len + w.ring_len) % w.ring_len;
+                if (n < n_terms)
+                    p[u] = fma(__ldg(w.moments + ((int64_t)slot * 3 + kk.source) * S + j),
+                               __ldg(kk.table + (int64_t)a * L2 + i + S - 1 - j), p[u]);
+            }
+        double t = (p[0] + p[1]) + (p[2] + p[3]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) s_acc[warp][0] = t;
+        __syncthreads();
+        if (lane == 0 && part == 0 && which < count) {
+            for (int q = 1; q < per_target; ++q) t += s_acc[warp + q][0];
+            const double r = mul(kk.factor, t);
             if (w.out_dtype == PHK_F64)
                 reinterpret_cast<double*>(kk.out)[i] = r;
             else
