@@ -55,10 +55,10 @@ static __device__ __noinline__ void carry_slices(int* words, int S, int most,
     __syncthreads();
 }
 
-// Three CTAs per SM (80 registers): the FP64 pipe and the integer pipes are
-// each about half busy, and the more warps, the better their phases overlap
-// (two / three / four CTAs at 1e7 macroparticles with RF and a 50-turn wake:
-// 406 / 371 / 358 us a turn; with detuning at 1e6: 107 / 92 / 96 us).
+// Three CTAs per SM (80 registers): the FP64 pipe is three quarters busy, the
+// integer pipes half, and the more warps, the better their phases overlap; at
+// four the exact sums spill (three / four CTAs: RF and a 50-turn wake, 3e6
+// macroparticles 157 / 161 us a turn; 1e6 detuned 94 / 101; 1e6 linear 60 / 64).
 template <int VEC, int SHAPE>
 __global__ void __launch_bounds__(kTrackThreads, 3)
 track64_kernel(const __grid_constant__ phk_program prog,

@@ -4,11 +4,10 @@
 namespace phk {
 
 // One particle per thread: the 64-bit chains are long, and 24 warps of them
-// hide each other better than 16 with two (three CTAs per SM at 80 registers
-// against two at 128; 1e6 macroparticles with detuning 92 / 105 us, linear
-// maps 1e6 62 / 72 us).  Two where little is computed for what is loaded:
-// slicing alone, and the undetuned turn with RF from about 4e6 macroparticles
-// on (3e6: 130 / 131 us a turn, 1e7 with a 50-turn wake: 384 / 371 us).
+// hide each other better than 16 with two (three CTAs per SM at 80 registers;
+// with RF and a 50-turn wake, one and two particles per thread: 1e6
+// macroparticles 88 / 95 us a turn, 3e6 157 / 158, 4e6 191 / 196, 1e7 373 / 375).
+// Two where nothing is computed, slicing alone.
 int launch_track_f64(const phk_program* prog, const phk_coords* c,
                      const phk_kick_set* pk, const phk_accum* acc, int ld,
                      int stm, bool vec_ok, cudaStream_t st) {
@@ -19,8 +18,6 @@ int launch_track_f64(const phk_program* prog, const phk_coords* c,
         case SHAPE_T:
             return launch_track64_t<1, SHAPE_T>(prog, c, pk, acc, ld, stm, st);
         case SHAPE_T_RF:
-            if (vec_ok && c->n >= 4000000)
-                return launch_track64_t<2, SHAPE_T_RF>(prog, c, pk, acc, ld, stm, st);
             return launch_track64_t<1, SHAPE_T_RF>(prog, c, pk, acc, ld, stm, st);
         case SHAPE_T_LIN:
             return launch_track64_t<1, SHAPE_T_LIN>(prog, c, pk, acc, ld, stm, st);
