@@ -134,6 +134,24 @@ __device__ __forceinline__ bool add_digits(int* d, int base, double u) {
     return true;
 }
 
+// What add_digits leaves: of a value below the window, the bits above the unit go
+// to the digits and the rest is returned, too small to cost the sum that it is
+// added to a rounding of its own; other values are returned whole.
+static __device__ __noinline__ double add_outside(int* d, int base, double u) {
+    const int hi = __double2hiint(u);
+    const int drop = base - biased_exp(hi);          // bits below the unit
+    if (drop < 1 || drop > 52 || base == kNoBase) return u;
+    const u64 w = ((u64)((hi & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(u);
+    const long long v = hi < 0 ? -(long long)(w >> drop) : (long long)(w >> drop);
+    atomicAdd(d, (int)((unsigned)v & kDigitMask));
+    atomicAdd(d + 1, (int)((unsigned)(v >> 19) & kDigitMask));
+    atomicAdd(d + 2, (int)((unsigned)(v >> 38) & kDigitMask));
+    atomicAdd(d + 3, (int)(v >> 57));
+    // u without the bits that were added
+    const u64 bits = (u64)__double_as_longlong(u) & (~0ull << drop);
+    return u - __longlong_as_double((long long)bits);
+}
+
 // carries the digits at d upwards, at least every kDigitValues values; a top
 // digit that might overflow before the next carry is taken out and returned
 // (in units of 2^57)
@@ -180,8 +198,12 @@ struct Spill64 {
     double* sum[2];       // of x and y in the partial column
     int64_t stride;       // between slices
 };
-static __device__ __noinline__ void spill64(const Spill64* sp, int q, int s, double u) {
+__device__ __forceinline__ void spill64(const Spill64* sp, int q, int s, double u) {
     if (u != 0.0) atomicAdd(sp->sum[q] + s * sp->stride, u);
+}
+static __device__ __noinline__ void outside64(const Spill64* sp, int q, int s, int* d,
+                                              int base, double u) {
+    spill64(sp, q, s, add_outside(d, base, u));
 }
 
 struct FixHist64 {
@@ -190,7 +212,8 @@ struct FixHist64 {
     int base[2];          // windows of x and y (digit_base)
 
     __device__ __forceinline__ void add_q(int q, int s, double u) const {
-        if (!add_digits(w + s * kFix64Words + 1 + 4 * q, base[q], u)) spill64(sp, q, s, u);
+        int* d = w + s * kFix64Words + 1 + 4 * q;
+        if (!add_digits(d, base[q], u)) outside64(sp, q, s, d, base[q], u);
     }
     __device__ __forceinline__ void add(int s, double x, double y) const {
         atomicAdd(w + s * kFix64Words, 1);

@@ -5,8 +5,8 @@
 // The values are summed per CTA as exact fixed-point digits in shared memory
 // (add_digits; the window of each value from a sample of the CTA's particles)
 // and the CTA adds its totals to the caller's FP64 arrays, one global atomic
-// per slice and value; a value outside the window (32 times the typical one,
-// 2^-17 of it, infinite, NaN) is added there on its own.  Before, every
+// per slice and value; what the digits do not hold of a value (32 times the
+// typical one, bits below 2^-69 of it, infinite, NaN) is added there on its own.  Before, every
 // particle's value was a global FP64 atomic, one launch pair per statistic:
 // 22 launches of 220 us for all statistics of 1e6 particles in 200 slices,
 // now two.  The integer work and the shared-memory atomics bound it (52
@@ -139,10 +139,14 @@ moments_kernel(const __grid_constant__ phk_slicer sl, const __grid_constant__ Mo
             if (PASS == 0) atomicAdd(a.in_smem ? w : a.counts + s, 1);
 #pragma unroll
             for (int p = 0; p < NV; ++p) {
-                if (PASS == 0 ? p < a.n_q : PAIRS::b(p) < a.n_q)
-                    if (!a.in_smem ||
-                        (!add_digits(w + D0 + 4 * p, base[p], v[p]) && v[p] != 0.0))
-                        atomicAdd(a.sums + p * S + s, v[p]);
+                if (PASS == 0 ? p < a.n_q : PAIRS::b(p) < a.n_q) {
+                    double r = v[p];            // what the digits do not hold
+                    if (a.in_smem) {
+                        int* d = w + D0 + 4 * p;
+                        r = add_digits(d, base[p], r) ? 0.0 : add_outside(d, base[p], r);
+                    }
+                    if (r != 0.0) atomicAdd(a.sums + p * S + s, r);
+                }
             }
         }
         if (a.in_smem && (it + 1) % (kDigitValues / kMomThreads) == 0) {
@@ -181,14 +185,10 @@ static int launch_moments_t(const phk_slicer* sl, MomentArgs a, cudaStream_t st)
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)limit) != cudaSuccess)
         cudaGetLastError();
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kMomThreads, smem) !=
-            cudaSuccess || per_sm < 1) {
-        cudaGetLastError();
-        per_sm = 1;
-    }
+    // one CTA per SM: every CTA's total is a rounding of the caller's sum, and two
+    // per SM are hardly faster
     int64_t blocks = (a.n + kMomThreads - 1) / kMomThreads;
-    if (blocks > (int64_t)d.sm_count * per_sm) blocks = (int64_t)d.sm_count * per_sm;
+    if (blocks > d.sm_count) blocks = d.sm_count;
     kern<<<(unsigned)(blocks < 1 ? 1 : blocks), kMomThreads, smem, st>>>(*sl, a);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
