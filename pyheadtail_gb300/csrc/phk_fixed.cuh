@@ -240,6 +240,8 @@ static __device__ __noinline__ void outside32(int* d, int S, float top, const Sp
     if (u != 0.0f) atomicAdd(sp->sum[q] + s * sp->stride, (double)u);
 }
 
+constexpr int kDigitValues32 = 16380;   // at most, between two carries
+
 struct FixHist32 {
     int* cnt;             // [S]
     int* dig;             // [6][S]: x top, middle, low, y
@@ -294,7 +296,7 @@ __device__ __forceinline__ double digits32_value(const int* d, int S, float top,
 }
 
 // Carries the digits of the slices with more than `most` values, at least every
-// kDigitValues values; a top digit that might overflow before the next carry
+// kDigitValues32 values; a top digit that might overflow before the next carry
 // goes to the column (all threads)
 static __device__ __noinline__ void carry_slices32(const int* cnt, int* dig, int S, int most,
                                                    const Spill64* sp, const unsigned* typ) {
@@ -364,14 +366,15 @@ __device__ __forceinline__ unsigned finite_high(float u) {
     return b < 0x7f800000u ? b : 0u;
 }
 
-// The median of what the warps saw at most, of those that saw something: a few
-// stray values, or warps that hold none, do not set it.  most: WARPS entries in
-// shared memory; all lanes of a warp call it.
+// The median of what the warps saw at most (v: lane w holds warp w's), of those
+// that saw something: a few stray values, or warps that hold none, do not set it.
+// All lanes of a warp call it.
 template <int WARPS>
-__device__ __forceinline__ unsigned typical_of(const unsigned* most) {
+__device__ __forceinline__ unsigned typical_of(unsigned v) {
     const int lane = threadIdx.x & 31;
-    const unsigned v = lane < WARPS ? most[lane] : 0u;
+    if (lane >= WARPS) v = 0u;
     int rank = 0;
+#pragma unroll
     for (int j = 0; j < WARPS; ++j) {
         const unsigned o = __shfl_sync(0xffffffffu, v, j);
         rank += o > v || (o == v && j < lane);
@@ -398,19 +401,19 @@ __device__ __forceinline__ void note_seen(unsigned (*to)[WARPS], unsigned mx, un
 }
 
 // The typical magnitudes (0: none yet) from the sample of the inputs and the
-// outputs of this tile, the larger (a bunch that starts on the axis, a large
-// beta at the end of the turn); where both are zero they stay open and the next
-// tile is looked at.  mx, my: the largest of this thread's outputs.  All threads
-// of the CTA call it; true if one is still open.  Out of line, as everything in
-// the tile loop that seldom runs: the loop fills the instruction cache as it is
-// (inlined, these parts cost 5 % of a pass).
+// outputs of this tile, of every warp the larger (a bunch that starts on the
+// axis, a large beta at the end of the turn); where all are zero they stay open
+// and the next tile is looked at.  mx, my: the largest of this thread's outputs.
+// All threads of the CTA call it; true if one is still open.  Out of line, as
+// everything in the tile loop that seldom runs: the loop fills the instruction
+// cache as it is (inlined, these parts cost 5 % of a pass).
 template <int WARPS>
 __device__ __noinline__ bool find_typical(Seen<WARPS>* seen, unsigned* typ, unsigned mx,
                                           unsigned my) {
     note_seen<WARPS>(seen->out, mx, my);
     __syncthreads();
-    const int q = (threadIdx.x >> 5) & 1;
-    const unsigned t = max(typical_of<WARPS>(seen->in[q]), typical_of<WARPS>(seen->out[q]));
+    const int q = (threadIdx.x >> 5) & 1, w = threadIdx.x & (WARPS - 1);
+    const unsigned t = typical_of<WARPS>(max(seen->in[q][w], seen->out[q][w]));
     if ((threadIdx.x & ~32u) == 0 && typ[q] == 0u) typ[q] = t;
     __syncthreads();
     return typ[0] == 0u || typ[1] == 0u;

@@ -129,7 +129,7 @@ __device__ __forceinline__ void merge_slice(const double* __restrict__ P,
     }
 }
 
-// One warp, one CTA per slice.  Bound by FP64, 64 instructions of 20 cycles
+// One warp, one CTA per slice.  Bound by FP64, 64 instructions of 19 cycles
 // for a slice, so the slices are spread over the SMs: eight to a CTA kept 7 of
 // them busy at 50 slices and 63 at 500 (50 slices: 9.4 us, now 6.9 from cold
 // caches; 16 or 8 lanes per slice have fewer instructions but longer chains: 200
@@ -700,7 +700,7 @@ int batch_max_grid(int32_t dtype, int32_t threads, int32_t S, int32_t nk) {
     return per_sm * device_info().sm_count;
 }
 
-// LANES lanes per (bunch, slice).  Bound by FP64 (about 20 cycles per warp
+// LANES lanes per (bunch, slice).  Bound by FP64 (about 19 cycles per warp
 // instruction and SM): with a warp per slice, its 15 shuffled additions, two
 // divisions and conversions were 256000 warp instructions at 64 bunches of
 // 100 slices; four lanes share them among eight slices (25 to 9.4 us).

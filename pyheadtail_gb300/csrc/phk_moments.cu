@@ -121,7 +121,7 @@ moments_kernel(const __grid_constant__ phk_slicer sl, const __grid_constant__ Mo
     }
     __syncthreads();
     for (int p = tid >> 5; p < NV; p += WARPS) {
-        const int base = digit_base(typical_of<WARPS>(s_most[p]), 17);
+        const int base = digit_base(typical_of<WARPS>(s_most[p][tid & (WARPS - 1)]), 17);
         if ((tid & 31) == 0) s_base[p] = base;
     }
     __syncthreads();

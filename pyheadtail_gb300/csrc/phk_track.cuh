@@ -1,7 +1,8 @@
 // The FP32 fused track kernel, the batched track kernel and the element
-// arithmetic of both forms as templates, with their launch helpers.  Included by the per-precision translation units
-// (phk_track_f32.cu, phk_track_f64.cu), which instantiate and launch them,
-// and by phk_kernels.cu for the host-side planning helpers.
+// arithmetic of both forms as templates, with their launch helpers.  Included
+// by the per-precision translation units (phk_track_f32.cu, phk_track_f64.cu),
+// which instantiate and launch them, and by phk_kernels.cu for the host-side
+// planning helpers.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -34,7 +35,7 @@ struct Tile {
 // element arithmetic, plain FP64 form (reference evaluation order)
 // ===================================================================
 
-// An FP64 instruction takes its 16 cycles of the pipe even when a short
+// An FP64 instruction takes its 19 cycles of the pipe even when a short
 // branch around it is compiled to predication and it is predicated off (16
 // of the 34 FP64 instructions a particle of the undetuned turn with RF were
 // such dispersion terms).  The element functions of the plain form are
@@ -1679,8 +1680,8 @@ __device__ __forceinline__ void load_tile_plain(const TrackArgs& a,
 // barrier releases and acquires at cluster scope (its default), global memory
 // included, and only the cluster touches its partial column until the kernel
 // ends: no fence of the whole device is needed beside it.  Two of those waited
-// for the particles' stores: 1.8 us of a pass (1e6 particles, the turn 39.1 to
-// 37.3 us).
+// for the particles' stores: 0.9 us of a pass (1e6 particles, the turn 40.6 to
+// 39.7 us).
 constexpr int kCluster = 4;
 
 // FP32 single-bunch kernel: particles per thread, resident CTAs per SM it
@@ -2399,7 +2400,7 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
         u0 = u1 = 0;
     }
     int cur = -1, col = -1;
-    constexpr int kTiles = kDigitValues / TILE;
+    constexpr int kTiles = kDigitValues32 / TILE;
     int until_carry = kTiles;    // FIX
     bool open = false;           // FIX: a window is still to be set
     // write the CTA's sums of the current bunch to its column, then zero
@@ -2522,7 +2523,7 @@ batch_track_kernel(const __grid_constant__ phk_kick_set pk,
                 if (a.has_acc && --until_carry == 0) {
                     // before a counter can overflow in the next kTiles tiles
                     until_carry = kTiles;
-                    carry_slices32(hcnt, fdig, Sa, kDigitValues - kTiles * TILE, &s_spill,
+                    carry_slices32(hcnt, fdig, Sa, kDigitValues32 - kTiles * TILE, &s_spill,
                                    s_typ);
                 }
             }

@@ -1,7 +1,7 @@
 // The plain form's fused pass: pending kicks, element program, slicing, one
 // read and one write of the coordinates.  Included by phk_track_f64.cu.
 //
-// GB300 starts an FP64 instruction of a warp every 16 cycles per SM, so this
+// GB300 starts an FP64 instruction of a warp every 19 cycles per SM, so this
 // kernel is built around having few of them: the slice sums (FixHist64) and
 // the RF sine (sine_turn) are integer arithmetic, the slice lookup compares
 // integer keys.
@@ -302,8 +302,8 @@ static int launch_track64_t(const phk_program* prog, const phk_coords* c,
         // One partial column per CTA: folding four CTAs into a column costs two
         // cluster barriers, and only 440 of 456 CTAs found room (a turn with
         // linear maps of 1e5 macroparticles at 50 / 500 / 1000 slices 24.8 / 63 /
-        // 97 us, now 22.8 / 37 / 53; 1e7 with RF and a 50-turn wake 371 us, now
-        // 354).  A caller with fewer columns than SMs and tiles (the
+        // 97 us against 22.8 / 37 / 53; 1e7 with RF and a 50-turn wake 371 against
+        // 354, when this was chosen).  A caller with fewer columns than SMs and tiles (the
         // workspace-free pass) gets clusters of kCluster CTAs per column.
         // Launched as clusters of one too: their CTAs are spread better than
         // those of a plain launch (1e6 with detuning 90.1 / 92.2 us).

@@ -23,7 +23,7 @@ __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, 
 // shared by all tables of the launch.  Samples ahead of the source
 // (sign +1, half of them) are a zero coefficient times the root at -dt_min,
 // one value.  Bound by FP64: a division and a square root, about 25 operations
-// of 20 cycles per warp (500 slices, four tables: 24 us).  As NumPy on the host,
+// of 19 cycles per warp (500 slices, four tables: 24 us).  As NumPy on the host,
 // with the upload of every table, it was 7 ms a turn.
 __global__ void wall_table_kernel(const __grid_constant__ phk_wall_tables w) {
     const int S = w.n_slices;
