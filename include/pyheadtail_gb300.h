@@ -264,7 +264,10 @@ typedef struct phk_accum {
  *   numpy path  (dense=0): conv_a[i] = sum_m m_a[m] * table_k[a][i + S-1 - m],
  *                          table_k[a] has 2S-1 entries
  *   dot path    (dense=1): conv_a[i] = sum_j m_a[j] * table_k[a][j][i]
- * where m_a = moments[slot(a)][source_k].  out_k has the dtype out_dtype. */
+ * where m_a = moments[slot(a)][source_k].  out_k has the dtype out_dtype.
+ * From 2^20 multiply-adds per call on, the numpy path sums 54-bit fixed-point
+ * factors; the error of out_k[i] stays below a sixteenth of the bound of an FP64
+ * sum of its n terms (n 2^-53 of their magnitudes), in FP64 where it would not. */
 typedef struct phk_wake_kick {
     int32_t source; /* 0 count, 1 count*mean_x, 2 count*mean_y */
     int32_t n_lags;
@@ -557,7 +560,8 @@ int phk_slice_moments(const phk_slicer *slicer, const void *z, int64_t n,
  *   pass 1: sums[pair][s] (double[13][S]), means double[6][S] given, for
  *           (x,x) (y,y) (z,z) (dp,dp) (x,xp) (y,yp) (z,dp) (xp,xp) (yp,yp)
  *           (x,dp) (y,dp) (xp,dp) (yp,dp)
- * all accumulated.                                                        */
+ * all accumulated.  A CTA's sums are exact but for bits below 2^-69 of a typical
+ * value and values 16 times it and more, which are added in FP64.          */
 int phk_slice_moments_all(const phk_slicer *slicer, const phk_coords *coords,
                           int32_t pass, const double *means, double *sums,
                           int32_t *counts, void *stream);
