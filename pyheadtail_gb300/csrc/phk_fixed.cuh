@@ -169,14 +169,33 @@ __device__ __forceinline__ int carry_digits(int* d) {
     return out;
 }
 
-// the FP64 value of the digits at d and of a top digit that was taken out
-__device__ __forceinline__ double digit_unit(int base) {
-    return __hiloint2double(((base == kNoBase ? 1023 : base) - 52) << 20, 0);
-}
+// the FP64 value of the digits at d, rounded once to nearest (integer work: with
+// two conversions and three FP64 instructions, 89 cycles of a warp, the end of a
+// pass over 1e5 particles in 1000 slices took 7 us more)
 __device__ __forceinline__ double digits_value(const int* d, int base) {
     const long long h = (long long)d[3] * (1 << kDigitBits) + (unsigned)d[2];
-    const long long l = ((long long)(unsigned)d[1] << kDigitBits) + (unsigned)d[0];
-    return fma((double)h, 0x1p38, (double)l) * digit_unit(base);
+    const u64 l = ((u64)(unsigned)d[1] << kDigitBits) + (unsigned)d[0];
+    // h 2^38 + l in 128 bits, its magnitude
+    u64 lo = ((u64)h << 38) + l;
+    u64 hi = (u64)(h >> 26) + (lo < l ? 1u : 0u);
+    if ((hi | lo) == 0) return 0.0;
+    const unsigned sign = (unsigned)(hi >> 32) & 0x80000000u;
+    if (sign) {
+        lo = 0 - lo;
+        hi = ~hi + (lo == 0 ? 1u : 0u);
+    }
+    // its top 64 bits, whether anything is below them, and 53 bits of it
+    const int lz = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
+    const u64 top = hi ? (hi << lz) | (lo >> (64 - lz)) : lo << (lz - 64);
+    const unsigned below = hi && (lo << lz) != 0 ? 1u : 0u;
+    u64 r = top >> 11;
+    r += (((unsigned)top & 0x7ffu) << 1 | below) + ((unsigned)r & 1u) > 0x800u ? 1u : 0u;
+    r += (u64)(unsigned)(74 - lz + base) << 52;      // r 2^(75 - lz + base - 1075)
+    return __hiloint2double((int)((unsigned)(r >> 32) | sign), (int)r);
+}
+// the unit of the digits, and the FP64 value of a top digit that was taken out
+__device__ __forceinline__ double digit_unit(int base) {
+    return __hiloint2double((base - 52) << 20, 0);
 }
 __device__ __forceinline__ double top_value(int top, int base) {
     return (double)top * 0x1p57 * digit_unit(base);

@@ -202,9 +202,11 @@ track64_kernel(const __grid_constant__ phk_program prog,
                 w += s * kFix64Words;
                 c += w[0];
 #pragma unroll
-                for (int q = 0; q < 2; ++q)
-                    v[q] = add(v[q], digits_value(w + 1 + 4 * q,
-                                                  digit_base(typ[q], 18)));
+                for (int q = 0; q < 2; ++q) {
+                    const double t = digits_value(w + 1 + 4 * q, digit_base(typ[q], 18));
+                    // mostly the first: no FP64 instruction
+                    v[q] = __double_as_longlong(v[q]) == 0 ? t : add_cold(v[q], t);
+                }
             }
             P[s * G] = (double)c;
             P[(Sa + s) * G] = v[0];

@@ -59,8 +59,48 @@ def test_fp64_counters_stay_in_range():
     # a carried digit, and VALUES more of the largest
     assert M + VALUES * M < 1 << 32
     assert (1 << 29) + VALUES * (1 << 17) + (1 << 13) < 1 << 31
-    # the two halves of a total are exact as doubles
-    assert ((1 << 32) - 1 << 19) + (1 << 32) < 1 << 53
+
+
+def _value(d, base):
+    """digits_value: d as 32-bit counters (the last signed)."""
+    U = (1 << 64) - 1
+    h, l = (d[3] << 19) + d[2], (d[1] << 19) + d[0]
+    lo = ((h << 38) & U) + l & U
+    hi = (h >> 26) + (lo < l) & U
+    if not hi | lo:
+        return 0.
+    neg = hi >> 63
+    if neg:
+        lo = -lo & U
+        hi = (~hi & U) + (lo == 0) & U
+    lz = 128 - ((hi << 64) | lo).bit_length()
+    top = (hi << lz & U) | lo >> (64 - lz) if hi else lo << (lz - 64)
+    below = int(bool(hi) and (lo << lz & U) != 0)
+    r = top >> 11
+    r += ((top & 0x7ff) << 1 | below) + (r & 1) > 0x800
+    r += 74 - lz + base << 52
+    return float(np.uint64(r | neg << 63).view(np.float64))
+
+
+@pytest.mark.parametrize('base', [82, 1005, 1900])
+def test_fp64_value_is_rounded_once(base):
+    rs = np.random.RandomState(3)
+    unit = Fraction(2) ** (base - 1075)
+    for n in range(6000):
+        k = rs.randint(1, 33)
+        d = [int(rs.randint(0, 1 << k, dtype=np.int64)) for _ in range(3)]
+        d.append(int(rs.randint(-(1 << k - 1), 1 << k - 1, dtype=np.int64))
+                 if n % 3 else -(n % 2))
+        if n % 5 == 0:       # ties: 53 bits and a half
+            d = [1 << 19 + n % 4, 0, 0, 0] if n % 2 else \
+                [0, 0, 1 << 15, 1 << 12 + n % 3]
+            d[0] += n % 3
+        if n == 0:
+            d = [0, 0, 0, 0]
+        total = d[0] + (d[1] << 19) + (d[2] << 38) + (d[3] << 57)
+        # Python rounds the quotient of two integers once
+        q = Fraction(total) * unit
+        assert _value(d, base) == q.numerator / q.denominator, d
 
 
 @pytest.mark.parametrize('e', [-106, -10, 0, 100])
