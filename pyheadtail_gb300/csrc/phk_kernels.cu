@@ -609,16 +609,18 @@ wake_conv_kernel(const __grid_constant__ phk_wake_set w) {
         for (int n = 0; n < which; ++n) mine &= mine - 1u;
         const int i = i0 + __ffs(mine) - 1;
         double p[4] = {0.0, 0.0, 0.0, 0.0};
-        const int n_terms = which < count ? kk.n_lags * S : 0, step = 32 * per_target;
-        for (int n0 = 32 * part + lane; n0 < n_terms; n0 += 4 * step)
+        // terms (turn a, source j) in the order of the tables, four loads in flight
+        int a = 0, j = 32 * part + lane, slot = w.head % w.ring_len;
+        const int turns = which < count ? kk.n_lags : 0, step = 32 * per_target;
+        while (a < turns)
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {          // four loads in flight
-                const int n = n0 + u * step;
-                const int a = n / S, j = n - a * S;
-                const int slot = ((w.head - a) % w.ring_len + w.ring_len) % w.ring_len;
-                if (n < n_terms)
+            for (int u = 0; u < 4; ++u) {
+                for (; j >= S && a < turns; j -= S, ++a)
+                    slot = slot == 0 ? w.ring_len - 1 : slot - 1;
+                if (a < turns)
                     p[u] = fma(__ldg(w.moments + ((int64_t)slot * 3 + kk.source) * S + j),
                                __ldg(kk.table + (int64_t)a * L2 + i + S - 1 - j), p[u]);
+                j += step;
             }
         double t = (p[0] + p[1]) + (p[2] + p[3]);
 #pragma unroll
