@@ -216,18 +216,22 @@ constexpr int kFix64Words = 9;   // per slice: count, 4 digits of x, 4 of y
 struct Spill64 {
     double* sum[2];       // of x and y in the partial column
     int64_t stride;       // between slices
+    int any;              // a value was added
 };
-__device__ __forceinline__ void spill64(const Spill64* sp, int q, int s, double u) {
-    if (u != 0.0) atomicAdd(sp->sum[q] + s * sp->stride, u);
+__device__ __forceinline__ void spill64(Spill64* sp, int q, int s, double u) {
+    if (u != 0.0) {
+        sp->any = 1;
+        atomicAdd(sp->sum[q] + s * sp->stride, u);
+    }
 }
-static __device__ __noinline__ void outside64(const Spill64* sp, int q, int s, int* d,
+static __device__ __noinline__ void outside64(Spill64* sp, int q, int s, int* d,
                                               int base, double u) {
     spill64(sp, q, s, add_outside(d, base, u));
 }
 
 struct FixHist64 {
     int* w;               // [S][kFix64Words]
-    const Spill64* sp;    // in shared memory
+    Spill64* sp;          // in shared memory
     int base[2];          // windows of x and y (digit_base)
 
     __device__ __forceinline__ void add_q(int q, int s, double u) const {

@@ -42,7 +42,7 @@ __host__ __device__ inline Track64Smem track64_smem(int Sa, int Sp, int n_tables
 
 // Carries the digits of the slices with more than `most` values (all threads)
 static __device__ __noinline__ void carry_slices(int* words, int S, int most,
-                                                 const Spill64* sp, const unsigned* typ) {
+                                                 Spill64* sp, const unsigned* typ) {
     __syncthreads();
     for (int s = threadIdx.x; s < S; s += kTrackThreads) {
         int* w = words + s * kFix64Words;
@@ -132,6 +132,7 @@ track64_kernel(const __grid_constant__ phk_program prog,
             s_spill.sum[0] = P + Sa * G;
             s_spill.sum[1] = P + 2 * Sa * G;
             s_spill.stride = G;
+            s_spill.any = 0;
         }
         if (clustered) cg::this_cluster().sync();   // orders the clears, see kCluster
         else __syncthreads();
@@ -183,11 +184,15 @@ track64_kernel(const __grid_constant__ phk_program prog,
         __syncthreads();
     }
     if (crank == 0) {
+        // the column is read only if values lay outside
+        const bool outside = clustered || s_spill.any;
         for (int s = tid; s < Sa; s += kTrackThreads) {
             long long c = 0;
-            double v[2];
-            v[0] = __ldcg(P + (Sa + s) * G);
-            v[1] = __ldcg(P + (2 * Sa + s) * G);
+            double v[2] = {0.0, 0.0};
+            if (outside) {
+                v[0] = __ldcg(P + (Sa + s) * G);
+                v[1] = __ldcg(P + (2 * Sa + s) * G);
+            }
             // unrolled over the cluster's members, so that the loads of
             // every member are in flight together
 #pragma unroll
